@@ -9,15 +9,40 @@ namespace aphi_b200 {
 
 namespace {
 
-template <class T>
-T* upload(const std::vector<T>& h, long long& bytes) {
-    T* d = nullptr;
-    const size_t n = std::max<size_t>(h.size(), 1);
-    APHI_CUDA(cudaMalloc(&d, n * sizeof(T)));
-    if (!h.empty()) APHI_CUDA(cudaMemcpy(d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-    bytes += static_cast<long long>(n * sizeof(T));
-    return d;
-}
+// Host arrays gathered for the device: one allocation for all of them, each
+// at a 256-byte boundary (a device allocation costs 0.1 ms and more).
+struct Uploads {
+    struct Part {
+        void** to;
+        const void* from;
+        size_t bytes;
+    };
+    std::vector<Part> parts;
+    template <class T>
+    void add(T*& d, const std::vector<T>& h) {
+        parts.push_back({reinterpret_cast<void**>(&d), h.data(), h.size() * sizeof(T)});
+    }
+    void* run(long long& bytes) {
+        auto padded = [](size_t b) { return (std::max<size_t>(b, 1) + 255) / 256 * 256; };
+        size_t total = 0;
+        for (const Part& p : parts) total += padded(p.bytes);
+        char* base = nullptr;
+        APHI_CUDA(cudaMalloc(&base, total));
+        try {
+            char* at = base;
+            for (const Part& p : parts) {
+                *p.to = at;
+                if (p.bytes) APHI_CUDA(cudaMemcpy(at, p.from, p.bytes, cudaMemcpyHostToDevice));
+                at += padded(p.bytes);
+            }
+        } catch (...) {
+            cudaFree(base);
+            throw;
+        }
+        bytes += static_cast<long long>(total);
+        return base;
+    }
+};
 
 // The factorization plans: per level, extend-add items, then one-CTA fronts,
 // then the blocked steps of the large fronts. A large front is processed in
@@ -377,27 +402,29 @@ void analysis_ensure_device(aphi_analysis* A) {
     const Symbolic& S = A->S;
     long long& b = A->device_bytes;
     DeviceSchedule& d = A->d;
-    d.first = upload(S.sn_first, b);
-    d.rows = upload(S.sn_rows, b);
-    d.loff = upload(S.sn_loff, b);
-    d.cboff = upload(S.sn_cboff, b);
-    d.soff = upload(S.sn_struct_off, b);
-    d.structs = upload(S.structs, b);
-    d.reloff = upload(S.rel_off, b);
-    d.rel = upload(S.rel, b);
-    d.child_ptr = upload(S.child_ptr, b);
-    d.child_list = upload(S.child_list, b);
-    d.uoff = upload(A->h_uoff, b);
-    d.a_dest = upload(S.a_dest, b);
-    d.row_ptr = upload(A->h_row_ptr, b);
-    d.col_idx = upload(A->h_col_idx, b);
-    d.new_of_orig = upload(S.new_of_orig, b);
-    d.orig_of_new = upload(S.orig_of_new, b);
-    d.ref_of_post = upload(S.ref_of_post, b);
-    d.fptr = upload(A->h_fptr, b);
-    d.fcol = upload(A->h_fcol, b);
-    d.fmap = upload(A->h_fmap, b);
-    d.items = upload(A->h_items, b);
+    Uploads up;
+    up.add(d.first, S.sn_first);
+    up.add(d.rows, S.sn_rows);
+    up.add(d.loff, S.sn_loff);
+    up.add(d.cboff, S.sn_cboff);
+    up.add(d.soff, S.sn_struct_off);
+    up.add(d.structs, S.structs);
+    up.add(d.reloff, S.rel_off);
+    up.add(d.rel, S.rel);
+    up.add(d.child_ptr, S.child_ptr);
+    up.add(d.child_list, S.child_list);
+    up.add(d.uoff, A->h_uoff);
+    up.add(d.a_dest, S.a_dest);
+    up.add(d.row_ptr, A->h_row_ptr);
+    up.add(d.col_idx, A->h_col_idx);
+    up.add(d.new_of_orig, S.new_of_orig);
+    up.add(d.orig_of_new, S.orig_of_new);
+    up.add(d.ref_of_post, S.ref_of_post);
+    up.add(d.fptr, A->h_fptr);
+    up.add(d.fcol, A->h_fcol);
+    up.add(d.fmap, A->h_fmap);
+    up.add(d.items, A->h_items);
+    A->device_arrays = up.run(b);
     A->device = dev;
     A->on_device = true;
 }
@@ -423,11 +450,8 @@ void analysis_info(const aphi_analysis* a, double* info) {
 }  // namespace aphi_b200
 
 aphi_analysis::~aphi_analysis() {
+    if (host_factor) host_factor_free(host_factor);
     for (void* w : ws)
         if (w) cudaFree(w);
-    void* ptrs[] = {d.first, d.rows, d.loff, d.cboff, d.soff, d.structs, d.reloff, d.rel, d.child_ptr,
-                    d.child_list, d.uoff, d.a_dest, d.row_ptr, d.col_idx, d.new_of_orig, d.orig_of_new,
-                    d.ref_of_post, d.fptr, d.fcol, d.fmap, d.items};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    if (device_arrays) cudaFree(device_arrays);
 }

@@ -102,6 +102,7 @@ struct aphi_analysis {
     std::vector<int> h_fptr, h_fcol;
     std::vector<long long> h_fmap;
     bool on_device = false;
+    void* device_arrays = nullptr;  // the one allocation behind d
     int device = -1;       // the CUDA device holding the device copy (set with it)
     bool fronts = false;   // built from independent dense fronts (no matrix pattern)
     // Contribution-block workspaces shared by this analysis's factors, one per
@@ -111,6 +112,11 @@ struct aphi_analysis {
     void* ws[2] = {nullptr, nullptr};
     size_t ws_bytes[2] = {0, 0};
     std::mutex ws_mu[2];
+    // An idle FP64 factor kept for aphi_solve_symmetric_host (capi_factor.cpp),
+    // freed with the analysis.
+    void* host_factor = nullptr;
+    void (*host_factor_free)(void*) = nullptr;
+    std::mutex host_factor_mu;
     long long num_items = 0;
     long long upool = 0;   // update-vector pool entries (per rhs)
     int max_parts = 1;

@@ -2,6 +2,7 @@
 // whole solve_symmetric pipeline on host buffers.
 #include <chrono>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "capi_util.hpp"
@@ -244,6 +245,56 @@ int aphi_csr_residuals_host(int n, const int* row_ptr, const int* col_idx, const
     });
 }
 
+}  // extern "C"
+
+namespace {
+
+// The factor that aphi_solve_symmetric_host works in. Making one takes a dozen
+// device allocations and giving it back as many frees, each of which waits for
+// the whole device: on the smallest meshes that was half of the call (6^3:
+// 3.8 ms, of which 2.0 ms on the device), and up to 30 ms of it when the
+// driver returned the memory to the system in between. So the analysis, which
+// its caller keeps between calls, keeps one idle factor of up to
+// kHostFactorKeep bytes until it is destroyed; a larger one's factorization
+// outweighs its allocations, and it is given back at once. A call takes the
+// idle factor out of the analysis, so concurrent calls never share one. A
+// call that ends in an exception destroys its factor.
+constexpr size_t kHostFactorKeep = size_t(256) << 20;
+
+aphi_factor* host_factor_take(aphi_analysis* an) {
+    {
+        std::lock_guard<std::mutex> lock(an->host_factor_mu);
+        if (void* kept = an->host_factor) {
+            int dev = 0;
+            APHI_CUDA(cudaGetDevice(&dev));
+            if (dev == an->device) {
+                an->host_factor = nullptr;
+                return static_cast<aphi_factor*>(kept);
+            }
+        }
+    }
+    return factor_create(an, 64, 1);
+}
+
+void host_factor_give(aphi_analysis* an, aphi_factor* f) {
+    const Symbolic& S = an->S;
+    const size_t bytes = 16 * static_cast<size_t>(S.stored) + static_cast<size_t>(f->dws_stride) +
+                         16 * static_cast<size_t>(an->upool) + 256 * static_cast<size_t>(S.n) + f->hvals_bytes;
+    if (bytes <= kHostFactorKeep) {
+        std::lock_guard<std::mutex> lock(an->host_factor_mu);
+        if (!an->host_factor) {
+            an->host_factor = f;
+            an->host_factor_free = [](void* p) { factor_destroy(static_cast<aphi_factor*>(p)); };
+            return;
+        }
+    }
+    factor_destroy(f);
+}
+
+}  // namespace
+
+extern "C" {
+
 int aphi_solve_symmetric_host(const aphi_analysis* an_c, const double* values, const double* b, int equil_iters,
                               double pivot_floor, double* x, double* report) {
     int rc = APHI_OK;
@@ -254,14 +305,14 @@ int aphi_solve_symmetric_host(const aphi_analysis* an_c, const double* values, c
         const long long nnz = an->S.nnz_a;
         std::memset(report, 0, sizeof(double) * 13);
         report[3] = report[4] = 1.0;
-        aphi_factor* f = factor_create(an, 64, 1);
-        double *dv = nullptr, *db = nullptr, *dx = nullptr;
+        aphi_factor* f = host_factor_take(an);
         try {
-            APHI_CUDA(cudaMalloc(&dv, sizeof(double) * 2 * std::max<long long>(nnz, 1)));
-            APHI_CUDA(cudaMalloc(&db, sizeof(double) * 2 * std::max(n, 1)));
-            APHI_CUDA(cudaMalloc(&dx, sizeof(double) * 2 * std::max(n, 1)));
+            const size_t vec = 2 * static_cast<size_t>(n);
+            double* dv = grow(f->hvals, f->hvals_bytes, sizeof(double) * 2 * static_cast<size_t>(nnz));
+            double* db = grow(f->hvec, f->hvec_bytes, 2 * sizeof(double) * vec);
+            double* dx = db + vec;
             APHI_CUDA(cudaMemcpy(dv, values, sizeof(double) * 2 * nnz, cudaMemcpyHostToDevice));
-            APHI_CUDA(cudaMemcpy(db, b, sizeof(double) * 2 * n, cudaMemcpyHostToDevice));
+            APHI_CUDA(cudaMemcpy(db, b, sizeof(double) * vec, cudaMemcpyHostToDevice));
             aphi_factor_stats st{};
             rc = factorize(f, dv, equil_iters, pivot_floor, &st, nullptr);
             report[3] = st.equilibration_min;
@@ -282,21 +333,15 @@ int aphi_solve_symmetric_host(const aphi_analysis* an_c, const double* values, c
                 report[1] = res[1];
                 report[2] = res[0];
                 report[0] = 1.0;
-                APHI_CUDA(cudaMemcpy(x, dx, sizeof(double) * 2 * n, cudaMemcpyDeviceToHost));
+                APHI_CUDA(cudaMemcpy(x, dx, sizeof(double) * vec, cudaMemcpyDeviceToHost));
             } else {
                 set_last_error("factorize_ldlt: a pivot at or below the floor stopped the factorization");
             }
         } catch (...) {
-            cudaFree(dv);
-            cudaFree(db);
-            cudaFree(dx);
             factor_destroy(f);
             throw;
         }
-        cudaFree(dv);
-        cudaFree(db);
-        cudaFree(dx);
-        factor_destroy(f);
+        host_factor_give(an, f);
     });
     if (g != APHI_OK) return g;
     return rc;

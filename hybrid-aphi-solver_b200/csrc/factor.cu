@@ -247,6 +247,19 @@ T* dalloc(size_t n) {
     return p;
 }
 
+// One device allocation, its parts at 256-byte boundaries.
+void device_parts(void** base, const std::vector<std::pair<void**, size_t>>& parts) {
+    auto padded = [](size_t bytes) { return (std::max<size_t>(bytes, 1) + 255) / 256 * 256; };
+    size_t total = 0;
+    for (const auto& p : parts) total += padded(p.second);
+    APHI_CUDA(cudaMalloc(base, total));
+    char* at = static_cast<char*>(*base);
+    for (const auto& p : parts) {
+        *p.first = at;
+        at += padded(p.second);
+    }
+}
+
 template <class R>
 void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_t st, const SolveArgs* sa,
               cx<R>* y, cx<R>* U, cx<R>* part) {
@@ -475,14 +488,13 @@ void solve_numeric(aphi_factor* f, int nrhs, const double* b, double* x, cudaStr
     const aphi_analysis* A = f->an;
     const int n = A->S.n;
     if (f->nrhs_cap < nrhs) {
-        if (f->y) cudaFree(f->y);
-        if (f->U) cudaFree(f->U);
-        if (f->part) cudaFree(f->part);
-        f->y = f->U = f->part = nullptr;
-        APHI_CUDA(cudaMalloc(&f->y, static_cast<size_t>(n) * nrhs * f->capacity * sizeof(cx<R>) + 16));
-        APHI_CUDA(cudaMalloc(&f->U, static_cast<size_t>(std::max<long long>(A->upool, 1)) * nrhs * f->capacity *
-                                        sizeof(cx<R>)));
-        APHI_CUDA(cudaMalloc(&f->part, static_cast<size_t>(A->max_parts) * kSolveBlock * 8 * f->capacity * sizeof(cx<R>)));
+        if (f->solve_arena) cudaFree(f->solve_arena);
+        f->solve_arena = nullptr;
+        f->nrhs_cap = 0;
+        const size_t vectors = sizeof(cx<R>) * static_cast<size_t>(nrhs) * f->capacity;
+        device_parts(&f->solve_arena, {{&f->y, vectors * n},
+                                       {&f->U, vectors * A->upool},
+                                       {&f->part, sizeof(cx<R>) * A->max_parts * kSolveBlock * 8 * f->capacity}});
         f->nrhs_cap = nrhs;
     }
     set_smem_limits<R>(A->opt.small_front);
@@ -539,26 +551,29 @@ aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
         f->presplit = !(pre && pre[0] == '0');
         const char* pst = std::getenv("APHI_TC_PRESTAGES");
         f->pre_stages = pst && pst[0] == '4' ? 4 : 3;
-        if (precision == 32 && an->tc_ws_units > 0) {
-            f->tcws_stride = an->tc_ws_units * 256;
-            APHI_CUDA(cudaMalloc(&f->tcws, static_cast<size_t>(f->tcws_stride) * batch));
-        }
+        if (precision == 32) f->tcws_stride = an->tc_ws_units * 256;
         const char* psc = std::getenv("APHI_DMMA_PRESCALE");
-        if (precision == 64 && an->dmma_ws_units > 0 && !(psc && psc[0] == '0')) {
-            f->dws_stride = an->dmma_ws_units * 256;
-            APHI_CUDA(cudaMalloc(&f->dws, static_cast<size_t>(f->dws_stride) * batch));
-        }
+        if (precision == 64 && !(psc && psc[0] == '0')) f->dws_stride = an->dmma_ws_units * 256;
+        // One allocation for everything whose size is known here: a device
+        // allocation costs 0.1 ms and more, which a small mesh's first call feels.
         const Symbolic& S = an->S;
-        APHI_CUDA(cudaMalloc(&f->L, static_cast<size_t>(std::max<long long>(S.stored, 1)) * batch * f->elem));
-        f->dscale = dalloc<double>(static_cast<size_t>(S.n) * batch);
-        f->rowmax = dalloc<unsigned long long>(static_cast<size_t>(S.n) * batch);
-        f->stats = dalloc<unsigned long long>(4 * static_cast<size_t>(batch));
-        f->dref = dalloc<double>(2 * static_cast<size_t>(S.n) * batch);
-        f->err = dalloc<int>(4);
-        f->kmax = dalloc<int>(batch);
+        const size_t nb = static_cast<size_t>(S.n) * batch;
+        const size_t counters = sizeof(int) * static_cast<size_t>(std::max(S.ns, 1)) * batch;
+        std::vector<std::pair<void**, size_t>> parts;
+        auto want = [&](auto** p, size_t bytes) { parts.push_back({reinterpret_cast<void**>(p), bytes}); };
+        want(&f->L, static_cast<size_t>(S.stored) * batch * f->elem);
+        want(&f->dscale, nb * sizeof(double));
+        want(&f->rowmax, nb * sizeof(unsigned long long));
+        want(&f->stats, 4 * sizeof(unsigned long long) * batch);
+        want(&f->dref, 2 * nb * sizeof(double));
+        want(&f->kmax, sizeof(int) * batch);
+        want(&f->err, 4 * sizeof(int));
+        want(&f->counters, counters);
+        if (f->tcws_stride > 0) want(&f->tcws, static_cast<size_t>(f->tcws_stride) * batch);
+        if (f->dws_stride > 0) want(&f->dws, static_cast<size_t>(f->dws_stride) * batch);
+        device_parts(&f->arena, parts);
         APHI_CUDA(cudaMemset(f->err, 0, 4 * sizeof(int)));
-        f->counters = dalloc<int>(static_cast<size_t>(std::max(S.ns, 1)) * batch);
-        APHI_CUDA(cudaMemset(f->counters, 0, sizeof(int) * std::max(S.ns, 1) * batch));
+        APHI_CUDA(cudaMemset(f->counters, 0, counters));
         const char* split_solve = std::getenv("APHI_SOLVE_SPLIT");
         f->solve_form = split_solve && split_solve[0] == '1' ? 1 : (split_solve && split_solve[0] == '0' ? 0 : -1);
         f->host_stats.assign(batch, aphi_factor_stats{});
@@ -1421,8 +1436,7 @@ void factor_export(const aphi_factor* f, int k, int* col_ptr, int* row_index, do
 
 aphi_factor::~aphi_factor() {
     for (cudaEvent_t e : prof_events) cudaEventDestroy(e);
-    void* ptrs[] = {L, dscale, rowmax, stats, dref, y, U, part, ir, red, norms, kr, err, kmax, hvals, hvec, tcws,
-                    counters, dws};
+    void* ptrs[] = {arena, solve_arena, ir, red, norms, kr, hvals, hvec};
     for (void* p : ptrs)
         if (p) cudaFree(p);
 }

@@ -15,6 +15,7 @@ struct aphi_factor {
     int batch = 1;             // active entries (<= capacity): what factorize/solve process
     int capacity = 1;          // entries the buffers are sized for
     size_t elem = 16;          // bytes per complex entry
+    void* arena = nullptr;     // the one allocation behind L .. counters and the prepared operands
     void* L = nullptr;         // batch x stored
     void* CB = nullptr;        // batch x cb_pool: the analysis's workspace, set at factorize
     double* dscale = nullptr;  // batch x n, original numbering
@@ -22,6 +23,7 @@ struct aphi_factor {
     unsigned long long* stats = nullptr;   // batch x 4 (max|L| bits, ...)
     double* dref = nullptr;    // batch x n complex128: D in the reference's permuted order
     // Solve scratch, grown on demand: y (batch x nrhs x n), U (batch x nrhs x upool).
+    void* solve_arena = nullptr;  // the one allocation behind y, U and part
     void* y = nullptr;
     void* U = nullptr;
     void* part = nullptr;  // backward partial sums: batch x max_parts x 64 x 8
