@@ -178,11 +178,11 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
                         // the launch's workspace (R = m - pe rounded up to 128):
                         //  tensor-core plan: split into TF32 planes, 10 planes x
                         //    8-column stages x R rows, 32 bytes per row and stage;
-                        //  FP64 plan: W = L D, R x K complex128, column-major.
+                        //  FP64 plan: the byte digits of both operands and the rows' scales.
                         const int K = std::min(cap_group * kTcPanel, w - p0);
                         const long long R = (m - pe + kTcM - 1) / kTcM * kTcM;
                         const long long units = trailing == K_UPDATE_TC ? ((K + kTcK - 1) / kTcK) * kTcPlanes * R / 8
-                                                                        : R * K / 16;
+                                                                        : i8_units(R, K, kI8Digits64);
                         for (long long t = before; t < static_cast<long long>(items.size()); ++t)
                             items[t].d = static_cast<int>(region);
                         split_fronts.push_back({s, p0, pe, static_cast<int>(region)});

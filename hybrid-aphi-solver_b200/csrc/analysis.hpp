@@ -30,7 +30,7 @@ enum Kind : int {
     K_UPDATE_PANEL = 10,  // (s, k0, i0, j0): update tile restricted to the current 128-column panel
     K_UPDATE_TC = 11,     // (s, p0, i0, j0, d): tensor-core trailing update by a whole panel
     K_TC_SPLIT = 12,      // (s, p0, r0, d): a front's trailing operands split into TF32 planes, 128 rows
-    K_DMMA_SCALE = 13,    // (s, p0, r0, d): a front's trailing rows scaled by the group's pivots (W = L D), 128 rows
+    K_DMMA_SCALE = 13,    // (s, p0, r0, d): a front's trailing operands (W = L D and L) as byte digits, 128 rows
 };
 
 struct Launch {
@@ -123,7 +123,7 @@ struct aphi_analysis {
     long long stat_first = 0;  // items of the statistics pass (s, col0)
     int stat_count = 0;     // partial-sum slots of the largest backward update launch
     long long tc_ws_units = 0;    // split-operand workspace of the tensor-core plan, per entry (256-byte units)
-    long long dmma_ws_units = 0;  // scaled-operand (W = L D) workspace of the FP64 plan, per entry (256-byte units)
+    long long dmma_ws_units = 0;  // byte-digit operand workspace of the FP64 plan, per entry (256-byte units)
     long long device_bytes = 0;
     ~aphi_analysis();
 };

@@ -274,11 +274,11 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     const bool presplit = sizeof(R) == 4 && f->tc_split == 2 && f->presplit && f->tcws;
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
     const size_t bwd_smem = (kTriSmem + kRedSmem) * sizeof(cx<R>);  // backward triangles
-    // FP64 trailing updates on pre-scaled operands (W = L D per panel group).
+    // FP64 trailing updates on INT8 digits, prepared once per panel group.
     const bool prescaled = sizeof(R) == 8 && f->dws;
     for (const Launch& l : plan) {
-        // Without pre-split (pre-scaled) operands the tile splits (scales) them
-        // itself: no operand launch.
+        // Without prepared operands the tile splits (FP64: scales) them itself:
+        // no operand launch.
         if (l.kind == K_TC_SPLIT && !presplit) continue;
         if (l.kind == K_DMMA_SCALE && !prescaled) continue;
         dim3 grid(l.count, sa && sa->ny > 0 ? sa->ny : f->batch);
@@ -304,20 +304,23 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                     break;
                 }
                 if constexpr (sizeof(R) == 8) {
-                    if (l.kind == K_UPDATE_WIDE && prescaled)
-                        k_update_wide_dmma<true><<<grid, 256, kDmmaSmem, st>>>(S, l.first, L, CB, ls, cs, l.kcap, 0,
-                                                                              f->dws, f->dws_stride);
-                    else
-                        k_update_wide_dmma<false><<<grid, 256, kDmmaSmem, st>>>(
-                            S, l.first, L, CB, ls, cs, l.kcap, l.kind == K_UPDATE_PANEL ? 1 : 0, nullptr, 0);
+                    if (l.kind == K_UPDATE_WIDE && prescaled) {
+                        const long long tiles = static_cast<long long>(l.count) * (kTcN / I8Fp64::Nc) * grid.y;
+                        k_update_i8<double, I8Fp64>
+                            <<<static_cast<unsigned>(std::min<long long>(tiles, f->sms)), kI8Threads, I8Fp64::smem, st>>>(
+                                S, l.first, l.count, static_cast<int>(grid.y), L, CB, ls, cs, l.kcap, f->dws,
+                                f->dws_stride, f->err);
+                    } else
+                        k_update_wide_dmma<<<grid, 256, kDmmaSmem, st>>>(S, l.first, L, CB, ls, cs, l.kcap,
+                                                                         l.kind == K_UPDATE_PANEL ? 1 : 0);
                 } else
                     k_update_wide<R><<<grid, 256, wide_smem<R>(), st>>>(S, l.first, L, CB, ls, cs, l.kcap,
                                                                       l.kind == K_UPDATE_PANEL ? 1 : 0);
                 break;
             case K_DMMA_SCALE:
                 if constexpr (sizeof(R) == 8)
-                    k_dmma_scale<<<dim3(grid.x, grid.y, (l.kcap + 63) / 64), 128, 0, st>>>(S, l.first, L, ls, f->dws,
-                                                                                         f->dws_stride, l.kcap);
+                    k_i8_split<double, I8Fp64><<<dim3(grid.x, grid.y, kTcM / 32), 256, 0, st>>>(
+                        S, l.first, L, ls, f->dws, f->dws_stride, l.kcap);
                 else
                     throw Error(APHI_ERR_INVALID, "operand scaling planned for an FP32 factor");
                 break;
@@ -408,10 +411,9 @@ void set_smem_limits(int small_front) {
                                    2 * kStep * kTile * static_cast<int>(sizeof(cx<R>))));
     APHI_CUDA(cudaFuncSetAttribute(k_update_wide<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem<R>()));
     if constexpr (sizeof(R) == 8) {
-        APHI_CUDA(cudaFuncSetAttribute(k_update_wide_dmma<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kDmmaSmem));
-        APHI_CUDA(cudaFuncSetAttribute(k_update_wide_dmma<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       kDmmaSmem));
+        APHI_CUDA(cudaFuncSetAttribute(k_update_wide_dmma, cudaFuncAttributeMaxDynamicSharedMemorySize, kDmmaSmem));
+        APHI_CUDA(cudaFuncSetAttribute(k_update_i8<double, I8Fp64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       I8Fp64::smem));
     }
     if constexpr (sizeof(R) == 4)
         APHI_CUDA(cudaFuncSetAttribute(k_update_tc<3, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -538,6 +540,7 @@ aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
         f->precision = precision;
         f->batch = batch;
         f->capacity = batch;
+        APHI_CUDA(cudaDeviceGetAttribute(&f->sms, cudaDevAttrMultiProcessorCount, an->device));
         f->elem = precision == 64 ? 16 : 8;
         const char* no_tc = std::getenv("APHI_NO_TC");
         f->use_tc = !(no_tc && no_tc[0] == '1');

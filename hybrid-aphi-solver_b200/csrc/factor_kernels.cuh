@@ -16,6 +16,7 @@
 
 #include "analysis.hpp"
 #include "common.cuh"
+#include "i8_update.cuh"
 #include "tc_update.cuh"
 
 namespace aphi_b200 {
@@ -462,9 +463,10 @@ __global__ void __launch_bounds__(256) k_update_wide(Sched S, long long item0, c
     }
 }
 
-// FP64 trailing update of complete panels on the FP64 tensor path (DMMA,
-// mma.sync m8n8k4). Same items, tile and K (up to kcap = kWidePair: a group
-// of 128-column panels) as k_update_wide. 8 warps in a 4 x 2
+// FP64 update on the FP64 tensor path (DMMA, mma.sync m8n8k4): the in-panel
+// updates (K = 32, too short for the INT8 tiles below), and the trailing ones
+// too with APHI_DMMA_PRESCALE=0. Same items, tile and K (up to kcap =
+// kWidePair: a group of 128-column panels) as k_update_wide. 8 warps in a 4 x 2
 // grid, each a 32 x 32 complex block of the tile: 4 x 4 blocks of 8 x 8, each
 // four real products (Cr += Ar Br - Ai Bi, Ci += Ar Bi + Ai Br; the minus by
 // a negated copy of Ai's fragment).
@@ -505,59 +507,366 @@ __device__ __forceinline__ void red_sub(double* p, double v) {
 }
 
 // K_DMMA_SCALE item (s, p0, r0, d): rows pe + r0 .. pe + r0 + 127 of front
-// s's trailing part (pe = p0 + K) times the group's pivots, W[r, k] =
-// L[pe + r, p0 + k] D[k] (the product the tile forms for its A operand, in
-// the same order), into region d: column-major, leading dimension R (the
-// trailing rows rounded up to 128); rows past the front are zeros. One thread
-// per row; blockIdx.z picks 64 of the K columns, whose loads are all in
-// flight at once.
-__global__ void __launch_bounds__(128) k_dmma_scale(Sched S, long long item0, const cx<double>* Lb,
-                                                    long long lstride, unsigned char* ws, long long ws_stride,
-                                                    int kcap) {
-    constexpr int kCols = 64;
-    __shared__ cx<double> piv[kCols];
+// s's trailing part (pe = p0 + K) prepared for the group's INT8 tiles
+// (i8_update.cuh): A = L D and B = L, each row scaled to integers and split
+// into byte digits, into region d. Rows past the front and columns past K are
+// zeros. A row with a component that is not finite gets a NaN scale, so that
+// the entries that it reaches become NaN, as in a floating-point update.
+//
+// 32 rows per CTA (blockIdx.z picks them), lane = row, so every global load is
+// a contiguous run of a column; a warp takes 16 columns at a time, which is
+// one 16-byte row of a core matrix per digit. Two passes over the operands,
+// the second served by the caches: the rows' largest components, then the
+// digits. Bound by its writes (48 bytes per entry; 24^3, 8 entries: 15.2 ms
+// per factorization beside 117 ms of tiles) and, on small fronts, by the
+// passes' dependent round trips (11 us a launch).
+template <class R, class C>
+__global__ void __launch_bounds__(256) k_i8_split(Sched S, long long item0, const cx<R>* Lb, long long lstride,
+                                                  unsigned char* ws, long long ws_stride, int kcap) {
+    constexpr int kWarps = 8;
+    __shared__ double dre[kWidePair], dim[kWidePair], up[kWidePair];  // D 2^-h, 2^h
+    __shared__ int top[2][kWarps][32];                                // largest high words of A, B
     const Item it = S.items[item0 + blockIdx.x];
-    const int s = it.s, p0 = it.a, r0 = it.b;
+    const int s = it.s, p0 = it.a;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
     const int K = min(kcap, w - p0), pe = p0 + K;
-    const long long R = (m - pe + kTcM - 1) / kTcM * kTcM;
-    const int k0 = blockIdx.z * kCols;
-    if (k0 >= K) return;  // the whole CTA: no barrier follows for it
-    cx<double>* W = reinterpret_cast<cx<double>*>(ws + ws_stride * blockIdx.y + static_cast<long long>(it.d) * 256);
-    const cx<double>* P = Lb + lstride * blockIdx.y + S.loff[s];
-    if (threadIdx.x < kCols) {
-        const int k = k0 + threadIdx.x;
-        piv[threadIdx.x] = k < K ? P[(p0 + k) + static_cast<long long>(p0 + k) * m] : cx<double>{0, 0};
+    const int Rp = (m - pe + kTcM - 1) / kTcM * kTcM;
+    const int nst = (K + kI8K - 1) / kI8K;
+    unsigned char* region = ws + ws_stride * blockIdx.y + static_cast<long long>(it.d) * 256;
+    const cx<R>* P = Lb + lstride * blockIdx.y + S.loff[s];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int r = it.b + 32 * blockIdx.z + lane;  // row within the trailing part
+    const bool in = pe + r < m;
+    const cx<R>* X = P + (in ? pe + r : pe) + static_cast<long long>(p0) * m;
+    for (int k = threadIdx.x; k < K; k += 256) {
+        const cx<R> d = P[(p0 + k) + static_cast<long long>(p0 + k) * m];
+        const double re = d.re, im = d.im;
+        const int e = __double2hiint(fmax(fabs(re), fabs(im))) >> 20;
+        const int h = e == 0 || e == 0x7ff ? 0 : (e - 1023) >> 1;
+        const double dn = __hiloint2double((1023 - h) << 20, 0);
+        dre[k] = re * dn;
+        dim[k] = im * dn;
+        up[k] = __hiloint2double((1023 + h) << 20, 0);
     }
-    const int r = r0 + threadIdx.x;  // row within the trailing part
-    const int row = pe + r;
-    const bool in = row < m;
     __syncthreads();
-#pragma unroll 2
-    for (int c = 0; c < kCols; c += 32) {
-        cx<double> v[32];
+    auto load = [&](int c, double (&re)[16], double (&im)[16]) {
 #pragma unroll
-        for (int u = 0; u < 32; ++u) {
-            const int k = k0 + c + u;
-            v[u] = in && k < K ? P[row + static_cast<long long>(p0 + k) * m] : cx<double>{0, 0};
+        for (int u = 0; u < 16; ++u) {
+            const int k = 16 * c + u;
+            const cx<R> x = in && k < K ? X[static_cast<long long>(k) * m] : cx<R>{0, 0};
+            re[u] = x.re;
+            im[u] = x.im;
+        }
+    };
+    int ta = 0, tb = 0;
+    for (int c = warp; 16 * c < K; c += kWarps) {
+        double re[16], im[16];
+        load(c, re, im);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int k = min(16 * c + u, K - 1);
+            const double ar = re[u] * dre[k] - im[u] * dim[k], ai = re[u] * dim[k] + im[u] * dre[k];
+            const double br = re[u] * up[k], bi = im[u] * up[k];
+            ta = max(ta, max(__double2hiint(ar) & 0x7fffffff, __double2hiint(ai) & 0x7fffffff));
+            tb = max(tb, max(__double2hiint(br) & 0x7fffffff, __double2hiint(bi) & 0x7fffffff));
+        }
+    }
+    top[0][warp][lane] = ta;
+    top[1][warp][lane] = tb;
+    __syncthreads();
+#pragma unroll
+    for (int v = 0; v < kWarps; ++v) {
+        ta = max(ta, top[0][v][lane]);
+        tb = max(tb, top[1][v][lane]);
+    }
+    // Biased exponents; tiny rows share one that keeps every scale normal.
+    const int ea = max(ta >> 20, 200), eb = max(tb >> 20, 200);
+    constexpr int kBits = 8 * C::S - 2;   // |integer| <= 2^kBits
+    constexpr int kTop = 4 * (2 * C::S - 1 - C::L);  // half of log2 of the last kept level's weight
+    const double fa = __hiloint2double((1023 + kBits + 1022 - ea) << 20, 0);
+    const double fb = __hiloint2double((1023 + kBits + 1022 - eb) << 20, 0);
+    if (warp == 0) {
+        double* scale = reinterpret_cast<double*>(region + i8_scale_off<C>(Rp, nst));
+        const double bad = __longlong_as_double(0x7ff8000000000000LL);
+        scale[r] = ea >= 0x7ff ? bad : __hiloint2double((ea + 1 - kBits + kTop) << 20, 0);
+        scale[Rp + r] = eb >= 0x7ff ? bad : __hiloint2double((eb + 1 - kBits + kTop) << 20, 0);
+    }
+    // 16 values -> digit p of each, 16 bytes, to dst + p * step.
+    auto digits = [&](const double (&v)[16], double f, unsigned char* dst, int step) {
+        constexpr long long kBias = (1LL << (8 * (C::S - 1))) / 255 * 128;  // 128 in every byte but the top digit's
+        unsigned out[C::S][4];
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            unsigned lo[4], hi[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const long long z = (__double2ll_rn(v[4 * g + u] * f) + kBias) ^ kBias;
+                lo[u] = static_cast<unsigned>(z);
+                hi[u] = static_cast<unsigned>(static_cast<unsigned long long>(z) >> 32);
+            }
+            // byte b of the four numbers = digit S - 1 - b
+            unsigned t[8];
+            t[0] = __byte_perm(lo[0], lo[1], 0x5140), t[1] = __byte_perm(lo[2], lo[3], 0x5140);
+            t[2] = __byte_perm(lo[0], lo[1], 0x7362), t[3] = __byte_perm(lo[2], lo[3], 0x7362);
+            t[4] = __byte_perm(hi[0], hi[1], 0x5140), t[5] = __byte_perm(hi[2], hi[3], 0x5140);
+            t[6] = __byte_perm(hi[0], hi[1], 0x7362), t[7] = __byte_perm(hi[2], hi[3], 0x7362);
+#pragma unroll
+            for (int b = 0; b < C::S; ++b)
+                out[C::S - 1 - b][g] = __byte_perm(t[b / 2 * 2], t[b / 2 * 2 + 1], b % 2 ? 0x7632 : 0x5410);
         }
 #pragma unroll
-        for (int u = 0; u < 32; ++u) {
-            const int k = k0 + c + u;
-            if (k < K) W[r + k * R] = v[u] * piv[c + u];
+        for (int p = 0; p < C::S; ++p)
+            *reinterpret_cast<uint4*>(dst + p * step) = make_uint4(out[p][0], out[p][1], out[p][2], out[p][3]);
+    };
+    for (int c = warp; c < 2 * nst; c += kWarps) {
+        double re[16], im[16], v[16];
+        load(c, re, im);
+        unsigned char* A = region + i8_a_off<C>(nst, r, c >> 1) + i8_off(r % kTcM, c & 1);
+        unsigned char* B = region + i8_b_off<C>(Rp, nst, r, c >> 1) + i8_off(r % C::Nc, c & 1);
+        constexpr int kPlaneA = kTcM * kI8K, kDigitB = C::W * kI8K, kHalfB = C::Nc * kI8K;
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int k = min(16 * c + u, K - 1);
+            v[u] = re[u] * dre[k] - im[u] * dim[k];
         }
+        digits(v, fa, A, 2 * kPlaneA);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) {
+            const int k = min(16 * c + u, K - 1);
+            v[u] = re[u] * dim[k] + im[u] * dre[k];
+        }
+        digits(v, fa, A + kPlaneA, 2 * kPlaneA);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) re[u] = re[u] * up[min(16 * c + u, K - 1)];
+        digits(re, fb, B, kDigitB);
+        digits(re, fb, B + C::imageB + kHalfB, kDigitB);
+#pragma unroll
+        for (int u = 0; u < 16; ++u) im[u] = im[u] * up[min(16 * c + u, K - 1)];
+        digits(im, fb, B + kHalfB, kDigitB);
+        digits(im, -fb, B + C::imageB, kDigitB);
     }
 }
 
-// Pre: the A operand comes scaled (W = L D, written by the launch's
-// k_dmma_scale into workspace region it.d), so the tile only moves it; without
-// it the A fragments are scaled by the pivots as they are read.
-template <bool Pre>
+// The trailing update on prepared INT8 operands. Items (s, p0, i0, j0, d) as
+// the other trailing updates': a 128 x 64 tile each, taken here as 64 / Nc
+// tiles of Nc columns. Persistent: one CTA per SM (its accumulators are all
+// of TMEM) walks the launch's tiles -- entries outermost, so that one
+// entry's operands stay in L2 -- in three roles that run side by side:
+//   warp 0, lane 0  copies operand stages (two bulk copies each) into the
+//                   ring of buffers, across tile boundaries;
+//   warp 1, lane 0  issues each stage's MMAs;
+//   warps 2 .. 9    read the destination while the tile is computed, then the
+//                   accumulators, and write the difference.
+// A tile's MMAs wait until the previous tile's accumulators have been read.
+// Every wait is bounded and gives up early once another role has failed.
+//
+// Measured on the 32^3 cylinder, two FP64 entries: the trailing updates of a
+// factorization take 178 ms (75 useful FP64 TFLOP/s, 2.7e15 INT8 operations/s)
+// against 486 ms (27.5) on DMMA with pre-scaled operands; 24^3, eight
+// entries: 117 against 292 ms; 8^3, one entry: 11 against 26 us a launch. It
+// is the faster one from the smallest launches up, so every FP64 trailing
+// update takes it.
+constexpr int kI8Threads = 320;
+
+template <class R, class C>
+__global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long item0, int count, int entries,
+                                                             cx<R>* Lb, cx<R>* CBb, long long lstride,
+                                                             long long cbstride, int kcap, const unsigned char* ws,
+                                                             long long ws_stride, int* err) {
+    extern __shared__ __align__(128) unsigned char smem_raw[];
+    constexpr int kHalves = kTcN / C::Nc, kEpWarps = 8;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + C::Stages * C::stage);
+    uint64_t* empty = full + C::Stages;
+    uint64_t* acc_full = empty + C::Stages;
+    uint64_t* acc_empty = acc_full + 1;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    volatile int* state = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] failed, [1] stages committed, [2] stages loaded
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(C::tmem));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        for (int b = 0; b < C::Stages; ++b) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(full + b)));
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(empty + b)));
+        }
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(acc_full)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(acc_empty)), "r"(kEpWarps));
+        asm volatile("fence.mbarrier_init.release.cluster;");
+        state[0] = 0;
+        state[1] = 0;
+        state[2] = 0;
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = *tmem_slot;
+
+    // This CTA's tiles: g = blockIdx.x, + gridDim.x, ...; the next one with
+    // entries on or below the front's diagonal.
+    struct Tile {
+        long long g;
+        int entry, s, p0, i0, j0, w, m, K, nst, d;
+    };
+    const long long total = static_cast<long long>(count) * kHalves * entries;
+    auto next = [&](Tile& t, long long g) -> bool {
+        for (; g < total; g += gridDim.x) {
+            t.entry = static_cast<int>(g / (count * kHalves));
+            const int q = static_cast<int>(g - static_cast<long long>(t.entry) * count * kHalves);
+            const Item it = S.items[item0 + q / kHalves];
+            t.s = it.s;
+            t.p0 = it.a;
+            t.i0 = it.b;
+            t.j0 = it.c + (q % kHalves) * C::Nc;
+            t.d = it.d;
+            t.m = S.rows[t.s];
+            if (t.j0 >= t.m || t.i0 + kTcM <= t.j0) continue;
+            t.w = S.first[t.s + 1] - S.first[t.s];
+            t.K = min(kcap, t.w - t.p0);
+            t.nst = (t.K + kI8K - 1) / kI8K;
+            t.g = g;
+            return true;
+        }
+        return false;
+    };
+
+    if (tid == 0) {
+        int c = 0;  // stages loaded so far
+        Tile t;
+        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x)) {
+            const int pe = t.p0 + t.K;
+            const int Rp = (t.m - pe + kTcM - 1) / kTcM * kTcM;
+            const unsigned char* region = ws + ws_stride * t.entry + static_cast<long long>(t.d) * 256;
+            const unsigned char* A = region + i8_a_off<C>(t.nst, t.i0 - pe, 0);
+            const unsigned char* B = region + i8_b_off<C>(Rp, t.nst, t.j0 - pe, 0);
+            for (int k = 0; k < t.nst; ++k, ++c) {
+                const int b = c % C::Stages;
+                if (c >= C::Stages && !mbar_wait_live(smem_u32(empty + b), ((c / C::Stages) - 1) & 1, state)) {
+                    state[0] = 1;
+                    break;
+                }
+                const uint32_t dst = smem_u32(smem_raw + b * C::stage), fb = smem_u32(full + b);
+                mbar_expect_tx(fb, C::stage);
+                bulk_g2s(dst, A + static_cast<long long>(k) * C::blockA, C::blockA, fb);
+                bulk_g2s(dst + C::blockA, B + static_cast<long long>(k) * C::blockB, C::blockB, fb);
+                state[2] = c + 1;
+            }
+        }
+    } else if (tid == 32) {
+        int c = 0, n = 0;  // stages, tiles issued so far
+        Tile t;
+        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x), ++n) {
+            if (n > 0 && !mbar_wait_live(smem_u32(acc_empty), (n - 1) & 1, state)) {
+                state[0] = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            for (int k = 0; k < t.nst; ++k, ++c) {
+                const int b = c % C::Stages;
+                if (!mbar_wait_live(smem_u32(full + b), (c / C::Stages) & 1, state)) {
+                    state[0] = 1;
+                    break;
+                }
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                i8_issue<C>(smem_u32(smem_raw + b * C::stage), tmem, k == 0);
+                mma_commit(smem_u32(empty + b));
+                state[1] = c + 1;
+            }
+            if (!state[0]) mma_commit(smem_u32(acc_full));
+        }
+    } else if (warp >= 2) {
+        constexpr int kCols = C::Nc / 2, kChunk = 4;  // columns per warp, and at a time
+        const int quad = warp & 3, half = (warp - 2) >> 2;
+        const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
+        int n = 0;
+        Tile t;
+        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x), ++n) {
+            const int cs = t.m - t.w, pe = t.p0 + t.K;
+            const int Rp = (t.m - pe + kTcM - 1) / kTcM * kTcM;
+            cx<R>* Ls = Lb + lstride * t.entry + S.loff[t.s];
+            cx<R>* CBs = CBb + cbstride * t.entry + (cs > 0 ? S.cboff[t.s] : 0);
+            const double* scale = reinterpret_cast<const double*>(
+                ws + ws_stride * t.entry + static_cast<long long>(t.d) * 256 + i8_scale_off<C>(Rp, t.nst));
+            const int i = t.i0 + quad * 32 + lane, j0 = t.j0 + half * kCols;
+            // The destination, read while the tile is computed.
+            cx<R> old[kCols];
+            auto at = [&](int j) {
+                return j < t.w ? Ls + i + static_cast<long long>(j) * t.m
+                               : CBs + (i - t.w) + static_cast<long long>(j - t.w) * cs;
+            };
+#pragma unroll
+            for (int q = 0; q < kCols; ++q) {
+                const int j = j0 + q;
+                old[q] = j < t.m && i < t.m && i >= j ? *at(j) : cx<R>{0, 0};
+            }
+            const double sa = scale[i - pe];
+            const double* sb = scale + Rp + (j0 - pe);
+            bool mine = mbar_wait_live(smem_u32(acc_full), n & 1, state);
+            mine = __all_sync(0xffffffffu, mine);  // the TMEM loads are warp-wide
+            if (!mine) {
+                state[0] = 1;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll
+            for (int q0 = 0; q0 < kCols; q0 += kChunk) {
+                double re[kChunk], im[kChunk];
+#pragma unroll
+                for (int part = 0; part < 2; ++part) {
+                    int v[C::L][kChunk];
+#pragma unroll
+                    for (int l = 0; l < C::L; ++l)
+                        tmem_ld4(tmem + lanes + l * C::W + part * C::Nc + half * kCols + q0, v[l]);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                    for (int q = 0; q < kChunk; ++q) {
+                        int a[C::L];
+#pragma unroll
+                        for (int l = 0; l < C::L; ++l) a[l] = v[l][q];
+                        (part ? im : re)[q] = i8_combine<C::L>(a);
+                    }
+                }
+                if (q0 + kChunk == kCols) {  // everything this warp reads has been read
+                    asm volatile("tcgen05.fence::before_thread_sync;");
+                    __syncwarp();
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(acc_empty)) : "memory");
+                }
+#pragma unroll
+                for (int q = 0; q < kChunk; ++q) {
+                    const int j = j0 + q0 + q;
+                    if (j < t.m && i < t.m && i >= j) {
+                        const double sc = sa * sb[q0 + q];
+                        *at(j) = cx<R>{static_cast<R>(fma(-re[q], sc, static_cast<double>(old[q0 + q].re))),
+                                       static_cast<R>(fma(-im[q], sc, static_cast<double>(old[q0 + q].im)))};
+                    }
+                }
+            }
+        }
+    }
+    __syncthreads();
+    // What is still in flight after a failure: the last commits, then any
+    // copies that no MMA consumed.
+    const bool failed = state[0] != 0;
+    if (tid == 0 && failed) {
+        const int committed = state[1], loaded = state[2];
+        for (int c = max(0, committed - C::Stages); c < committed; ++c)
+            mbar_wait(smem_u32(empty + c % C::Stages), (c / C::Stages) & 1);
+        for (int c = committed; c < loaded; ++c) mbar_wait(smem_u32(full + c % C::Stages), (c / C::Stages) & 1);
+        atomicExch(err, 1);
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::tmem));
+}
+
 __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long item0, cx<double>* Lb,
                                                           cx<double>* CBb, long long lstride, long long cbstride,
-                                                          int kcap, int panel, const unsigned char* ws,
-                                                          long long ws_stride) {
+                                                          int kcap, int panel) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<double>* Ds = reinterpret_cast<cx<double>*>(smem_raw);  // [kWidePair] pivots of the group's panels
     cx<double>* Ring = Ds + kWidePair;                           // [stage][A: KC x ldA | B: KC x ldB]
@@ -573,13 +882,6 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
     cx<double>* CBs = CB + (cs > 0 ? S.cboff[s] : 0);
     const cx<double>* P = Ls + static_cast<long long>(p0) * m;
     const cx<double>* dg = Ls + p0 + static_cast<long long>(p0) * m;
-    // The A operand: W's rows i0 - pe .. (leading dimension R), or the panel's.
-    const int pe = p0 + K;
-    const long long ldw = Pre ? static_cast<long long>(m - pe + kTcM - 1) / kTcM * kTcM : m;
-    const cx<double>* PA =
-        Pre ? reinterpret_cast<const cx<double>*>(ws + ws_stride * blockIdx.y + static_cast<long long>(it.d) * 256) +
-                  (i0 - pe)
-            : P + i0;
     const int tid = threadIdx.x;
     const uint32_t ring = smem_u32(Ring);
     // Chunk c: panel columns 16c.. of rows i0.. (A, 128 rows) and j0.. (B, 64).
@@ -591,7 +893,7 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
         for (int q = 0; q < kDmmaKC * kWideM / 256; ++q) {
             const int e = tid + 256 * q, k = e / kWideM, r = e % kWideM;
             const bool in = kbase + k < K && i0 + r < m;
-            cp_async16(sa + (k * kDmmaLdA + r) * 16, in ? PA + static_cast<long long>(kbase + k) * ldw + r : P,
+            cp_async16(sa + (k * kDmmaLdA + r) * 16, in ? P + static_cast<long long>(kbase + k) * m + i0 + r : P,
                        in ? 16u : 0u);
         }
 #pragma unroll
@@ -615,8 +917,7 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
     cp_async_commit();
     if (nc > 1) fetch(1);
     cp_async_commit();
-    if constexpr (!Pre)
-        for (int t = tid; t < kWidePair; t += 256) Ds[t] = t < K ? dg[static_cast<long long>(t) * (m + 1)] : cx<double>{0, 0};
+    for (int t = tid; t < kWidePair; t += 256) Ds[t] = t < K ? dg[static_cast<long long>(t) * (m + 1)] : cx<double>{0, 0};
     for (int c = 0; c < nc; ++c) {
         cp_async_wait<1>();  // this thread's copies of chunk c have landed
         __syncthreads();     // everyone's have; everyone is done with chunk c - 1
@@ -627,14 +928,9 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
 #pragma unroll
         for (int ks = 0; ks < kDmmaKC; ks += 4) {
             cx<double> af[4], bf[4];
-            if constexpr (Pre) {
+            const cx<double> d = Ds[c * kDmmaKC + ks + t4];
 #pragma unroll
-                for (int a = 0; a < 4; ++a) af[a] = A[(ks + t4) * kDmmaLdA + 32 * wm + 8 * a + g];
-            } else {
-                const cx<double> d = Ds[c * kDmmaKC + ks + t4];
-#pragma unroll
-                for (int a = 0; a < 4; ++a) af[a] = A[(ks + t4) * kDmmaLdA + 32 * wm + 8 * a + g] * d;
-            }
+            for (int a = 0; a < 4; ++a) af[a] = A[(ks + t4) * kDmmaLdA + 32 * wm + 8 * a + g] * d;
 #pragma unroll
             for (int b = 0; b < 4; ++b) bf[b] = B[(ks + t4) * kDmmaLdB + 32 * wn + 8 * b + g];
             // One real product over all 16 blocks before the next, so that

@@ -1,0 +1,157 @@
+// Trailing updates on the INT8 tensor cores (tcgen05.mma kind::i8, sm_100a):
+// products of byte digits, accumulated exactly in 32-bit integers.
+//
+// The update is F -= W B^T over one panel group's K columns (W = L D, B = L,
+// complex). FP64 runs at 37 TFLOP/s on this device, INT8 at over a hundred times
+// that, so the FP64 operands are written as fixed-point numbers and those as
+// base-256 digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump,
+// "Error-free transformations of matrix multiplication", 2012):
+//
+//   row i of W:  w_ik 2^(62 - e_i), rounded to an integer, |.| <= 2^62, with
+//   2^e_i just above the row's largest component; = sum_p d_p 256^(7 - p),
+//   eight digits in [-128, 127]. Rows of B likewise, with exponents of their own.
+//
+// A product of two digits is at most 2^14, and every product of digits p and q
+// belongs to level l = p + q, of weight 256^(14 - l). Level by level the
+// products of all K columns are summed in a 32-bit accumulator (below 2^28 for
+// K = 512), without any rounding. Levels 0 .. kLevels - 1 are kept; what is
+// dropped is below K 2^-56 of the rows' largest products. So the errors are
+// the operands' rounding (2^-62 of the row's largest component: entries down
+// to 2^-9 of it are exact), the dropped levels and two roundings of the sum.
+// Seven digits (2^-54) are enough for the solutions' accuracy but not for the
+// smallest pivots, which are what is left of sums of much larger terms: on
+// the 32^3 cylinder at 1 MHz the smallest pivot came out 2e-8 off, and 1e-10
+// from the FP64 FMA chains' with eight, nearer to the reference's (2.9e-10)
+// than theirs (4.0e-10).
+// The pivots' magnitudes are shared out between the operands (column k of W is
+// divided and of B multiplied by 2^h, h half of D_k's exponent), so that the
+// columns of both have the scale of a Cholesky factor's and one exponent per
+// row serves them all.
+//
+// Tile: 128 rows x Nc complex columns. B is staged twice per digit, [Br | Bi]
+// and [-Bi | Br], so that [Cr | Ci] += Ar [Br | Bi]^T + Ai [-Bi | Br]^T; the
+// digits q of B lie back to back, and their levels p + q back to back in
+// TMEM, so one MMA takes digit p of A against up to four digits of B
+// (N = 256): the tensor core reads each A digit once per N = 256 rather than
+// once per 64 columns.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include <cstdint>
+
+#include "tc_config.hpp"
+#include "tc_update.cuh"
+
+namespace aphi_b200 {
+
+// S digits per operand, L levels kept, Nc complex columns per tile, Stages
+// operand buffers.
+template <int S_, int L_, int Nc_, int Stages_>
+struct I8Shape {
+    static constexpr int S = S_, L = L_, Nc = Nc_, Stages = Stages_;
+    static constexpr int W = 2 * Nc;                       // accumulator columns per level: Cr, Ci
+    static constexpr int blockA = S * 2 * kTcM * kI8K;     // one stage of 128 A rows: digits x (re, im)
+    static constexpr int imageB = S * W * kI8K;            // one stage of Nc B rows, one image
+    static constexpr int blockB = 2 * imageB;              // [Br | Bi] per digit, then [-Bi | Br] per digit
+    static constexpr int stage = blockA + blockB;
+    static constexpr int smem = Stages * stage + 256;
+    static constexpr int tmem = 512;                       // columns allocated (L W of them used)
+    static_assert(L * W <= tmem && L >= S && L <= 2 * S - 1, "levels must fit TMEM");
+    static_assert(smem <= 227 * 1024, "operand buffers exceed shared memory");
+};
+using I8Fp64 = I8Shape<kI8Digits64, kI8Levels64, kI8Nc64, 2>;
+
+// A front's region (R padded rows, nst stages of 32 columns): the A blocks
+// [R / 128][nst], the B blocks [R / Nc][nst], then a scale per A row and per
+// B row (doubles).
+template <class C>
+__device__ __forceinline__ long long i8_a_off(int nst, int r, int c) {
+    return (static_cast<long long>(r / kTcM) * nst + c) * C::blockA;
+}
+template <class C>
+__device__ __forceinline__ long long i8_b_off(int R, int nst, int r, int c) {
+    return static_cast<long long>(R / kTcM) * nst * C::blockA + (static_cast<long long>(r / C::Nc) * nst + c) * C::blockB;
+}
+template <class C>
+__device__ __forceinline__ long long i8_scale_off(int R, int nst) {
+    return static_cast<long long>(R / kTcM) * nst * C::blockA + static_cast<long long>(R / C::Nc) * nst * C::blockB;
+}
+
+// Row r's 16 bytes of columns 16 h .. of a 32-column stage, in the canonical
+// K-major no-swizzle layout (8-row x 16-byte core matrices; the strides of
+// smem_desc).
+__device__ __forceinline__ uint32_t i8_off(int r, int h) { return (r >> 3) * 256 + h * 128 + (r & 7) * 16; }
+
+// kind::i8 instruction descriptor: S32 accumulators, signed 8-bit A and B,
+// K-major, M = 128, N = n.
+__device__ __forceinline__ constexpr uint32_t i8_idesc(int n) {
+    return (2u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(n >> 3) << 17) |
+           (static_cast<uint32_t>(kTcM >> 4) << 24);
+}
+
+__device__ __forceinline__ void mma_i8(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d_tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc));
+}
+
+// The MMAs of one stage (32 columns of K). first: the tile's first stage,
+// whose products start the accumulators afresh.
+template <class C>
+__device__ __forceinline__ void i8_issue(uint32_t stage, uint32_t tmem, bool first) {
+    const uint32_t B = stage + C::blockA;
+    int top = -1;  // highest level written so far in this stage
+#pragma unroll
+    for (int p = 0; p < C::S; ++p) {
+        const int q = C::L - p < C::S ? C::L - p : C::S;  // digits 0 .. q - 1 of B meet digit p of A
+#pragma unroll
+        for (int im = 0; im < 2; ++im) {
+            const uint64_t a = smem_desc(stage + (2 * p + im) * kTcM * kI8K);
+            const uint32_t b = B + im * C::imageB;
+            // Columns [0, q W) of the stacked B rows, at most 256 at a time;
+            // levels above `top` start afresh in the first stage.
+            const int split = im == 0 && p > 0 && p + q - 1 > top ? (q - 1) * C::W : q * C::W;
+#pragma unroll
+            for (int n0 = 0; n0 < C::S * C::W; n0 += 256) {
+                if (n0 >= q * C::W) break;
+                const int n1 = n0 + 256 < q * C::W ? n0 + 256 : q * C::W;
+                const bool fresh0 = first && im == 0 && p == 0;
+                if (split < n1 && first) {  // [n0, split) accumulates, [split, n1) is new
+                    if (split > n0)
+                        mma_i8(tmem + p * C::W + n0, a, smem_desc(b + n0 * kI8K), i8_idesc(split - n0), 1);
+                    const int s0 = split > n0 ? split : n0;
+                    mma_i8(tmem + p * C::W + s0, a, smem_desc(b + s0 * kI8K), i8_idesc(n1 - s0), 0);
+                } else {
+                    mma_i8(tmem + p * C::W + n0, a, smem_desc(b + n0 * kI8K), i8_idesc(n1 - n0), fresh0 ? 0u : 1u);
+                }
+            }
+        }
+        if (p + q - 1 > top) top = p + q - 1;
+    }
+}
+
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, int (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr));
+}
+
+// sum_l a_l 256^(L - 1 - l) as a double: exact 64-bit sums of up to four
+// levels, then one rounding.
+template <int L>
+__device__ __forceinline__ double i8_combine(const int (&a)[L]) {
+    constexpr int kLo = L > 4 ? L - 4 : 0;  // levels [kLo, L) in the low word
+    long long lo = a[L - 1];
+#pragma unroll
+    for (int l = L - 2; l >= kLo; --l) lo += static_cast<long long>(a[l]) * (1 << (8 * (L - 1 - l)));
+    if constexpr (kLo == 0) return static_cast<double>(lo);
+    long long hi = a[kLo > 0 ? kLo - 1 : 0];
+#pragma unroll
+    for (int l = kLo - 2; l >= 0; --l) hi += static_cast<long long>(a[l]) * (1 << (8 * (kLo - 1 - l)));
+    return fma(static_cast<double>(hi), 4294967296.0, static_cast<double>(lo));
+}
+
+}  // namespace aphi_b200

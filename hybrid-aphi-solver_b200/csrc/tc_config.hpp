@@ -42,4 +42,16 @@ struct TcSmem {
 };
 constexpr int kTcSmem = TcSmem<kTcSplit>::bytes;
 
+// The FP64 trailing update on INT8 digits (i8_update.cuh).
+constexpr int kI8K = 32;         // columns of K per stage (one MMA step)
+constexpr int kI8Digits64 = 8;   // base-256 digits per FP64 operand
+constexpr int kI8Levels64 = 8;   // digit-product levels kept
+constexpr int kI8Nc64 = 32;      // complex columns per tile
+// 256-byte units of a front's prepared operands: R (a multiple of 128) rows,
+// K columns; per row and column 2 S bytes of A digits and 4 S of B digits,
+// and two doubles per row.
+constexpr long long i8_units(long long R, int K, int digits) {
+    return R / kTcM * (((K + kI8K - 1) / kI8K) * (6LL * digits * kI8K * kTcM / 256) + 2 * 8 * kTcM / 256);
+}
+
 }  // namespace aphi_b200
