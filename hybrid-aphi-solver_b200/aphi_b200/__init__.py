@@ -752,7 +752,9 @@ class Factor:
         return panels, cb
 
     def set_tc_split(self, split: int) -> None:
-        """FP32 factors: TF32 pieces per operand in the tensor-core update (3 or 2)."""
+        """FP32 factors: the tensor-core update's form. 3: three TF32 pieces per
+        operand; 2: the faster form (INT8 digits; two TF32 pieces when
+        APHI_TC_PRESPLIT was set as the factor was made)."""
         check(lib().aphi_factor_set_tc_split(self._h, split))
         self.tc_split = split
 
@@ -913,9 +915,8 @@ class SweepSolver:
     most fp64_batch (FP64) or fp32_batch (FP32) entries per factorization, so
     no factorization is spent on padding.
 
-    tc_split: TF32 pieces per FP32 operand in the tensor-core updates of the
-    FP32 factors. 2 (hh + hl + lh, half the tensor-core work of 3) by default:
-    on the 32^3 sweep it needs the same refinement iterations as 3 (4-13).
+    tc_split: the form of the FP32 factors' tensor-core updates
+    (Factor.set_tc_split). 2 by default.
 
     overlap=True: entries predicted to need FP64 are factorized and solved on
     a side stream, from a second host thread, while the FP32 entries are

@@ -181,8 +181,10 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
                         //  FP64 plan: the byte digits of both operands and the rows' scales.
                         const int K = std::min(cap_group * kTcPanel, w - p0);
                         const long long R = (m - pe + kTcM - 1) / kTcM * kTcM;
-                        const long long units = trailing == K_UPDATE_TC ? ((K + kTcK - 1) / kTcK) * kTcPlanes * R / 8
-                                                                        : i8_units(R, K, kI8Digits64);
+                        const long long units =
+                            trailing == K_UPDATE_TC
+                                ? std::max(((K + kTcK - 1) / kTcK) * kTcPlanes * R / 8, i8_units(R, K, kI8Digits32))
+                                : i8_units(R, K, kI8Digits64);
                         for (long long t = before; t < static_cast<long long>(items.size()); ++t)
                             items[t].d = static_cast<int>(region);
                         split_fronts.push_back({s, p0, pe, static_cast<int>(region)});

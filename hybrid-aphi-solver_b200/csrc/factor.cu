@@ -13,6 +13,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "factor.hpp"
@@ -272,6 +273,14 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     aphi_factor* fm = const_cast<aphi_factor*>(f);
     const bool prof = f->profile;
     const bool presplit = sizeof(R) == 4 && f->tc_split == 2 && f->presplit && f->tcws;
+    const bool i8 = presplit && f->tc_i8;  // FP32 trailing updates on INT8 digits
+    auto update_i8 = [&](const Launch& l) {
+        using C = std::conditional_t<sizeof(R) == 8, I8Fp64, I8Fp32>;
+        const long long tiles = static_cast<long long>(l.count) * (kTcN / C::Nc) * f->batch;
+        k_update_i8<R, C><<<static_cast<unsigned>(std::min<long long>(tiles, f->sms)), kI8Threads, C::smem, st>>>(
+            S, l.first, l.count, f->batch, L, CB, ls, cs, l.kcap, sizeof(R) == 8 ? f->dws : f->tcws,
+            sizeof(R) == 8 ? f->dws_stride : f->tcws_stride, f->err);
+    };
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
     const size_t bwd_smem = (kTriSmem + kRedSmem) * sizeof(cx<R>);  // backward triangles
     // FP64 trailing updates on INT8 digits, prepared once per panel group.
@@ -304,13 +313,9 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                     break;
                 }
                 if constexpr (sizeof(R) == 8) {
-                    if (l.kind == K_UPDATE_WIDE && prescaled) {
-                        const long long tiles = static_cast<long long>(l.count) * (kTcN / I8Fp64::Nc) * grid.y;
-                        k_update_i8<double, I8Fp64>
-                            <<<static_cast<unsigned>(std::min<long long>(tiles, f->sms)), kI8Threads, I8Fp64::smem, st>>>(
-                                S, l.first, l.count, static_cast<int>(grid.y), L, CB, ls, cs, l.kcap, f->dws,
-                                f->dws_stride, f->err);
-                    } else
+                    if (l.kind == K_UPDATE_WIDE && prescaled)
+                        update_i8(l);
+                    else
                         k_update_wide_dmma<<<grid, 256, kDmmaSmem, st>>>(S, l.first, L, CB, ls, cs, l.kcap,
                                                                          l.kind == K_UPDATE_PANEL ? 1 : 0);
                 } else
@@ -325,14 +330,23 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                     throw Error(APHI_ERR_INVALID, "operand scaling planned for an FP32 factor");
                 break;
             case K_TC_SPLIT:
-                if constexpr (sizeof(R) == 4)
+                if constexpr (sizeof(R) == 4) {
+                    if (i8) {
+                        k_i8_split<float, I8Fp32><<<dim3(grid.x, grid.y, kTcM / 32), 256, 0, st>>>(
+                            S, l.first, L, ls, f->tcws, f->tcws_stride, l.kcap);
+                        break;
+                    }
                     k_tc_split<<<dim3(grid.x, grid.y, (l.kcap + 8 * kTcK - 1) / (8 * kTcK)), kTcThreads, 0, st>>>(
                         S, l.first, L, ls, f->tcws, f->tcws_stride, l.kcap);
-                else
+                } else
                     throw Error(APHI_ERR_INVALID, "operand split planned for an FP64 factor");
                 break;
             case K_UPDATE_TC:
                 if constexpr (sizeof(R) == 4) {
+                    if (i8) {
+                        update_i8(l);
+                        break;
+                    }
                     if (presplit) {
                         auto go = [&](auto kern, int smem) {
                             kern<<<grid, kTcThreads, smem, st>>>(S, l.first, L, CB, ls, cs, l.kcap, f->tcws,
@@ -415,7 +429,9 @@ void set_smem_limits(int small_front) {
         APHI_CUDA(cudaFuncSetAttribute(k_update_i8<double, I8Fp64>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        I8Fp64::smem));
     }
-    if constexpr (sizeof(R) == 4)
+    if constexpr (sizeof(R) == 4) {
+        APHI_CUDA(cudaFuncSetAttribute(k_update_i8<float, I8Fp32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       I8Fp32::smem));
         APHI_CUDA(cudaFuncSetAttribute(k_update_tc<3, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        TcSmem<3, 2>::bytes));
         APHI_CUDA(cudaFuncSetAttribute(k_update_tc<2, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -432,6 +448,7 @@ void set_smem_limits(int small_front) {
                                        TcPreSmem<4>::bytes));
         APHI_CUDA(cudaFuncSetAttribute(k_update_tc_presplit<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        TcPreSmem<4>::bytes));
+    }
     const int tri = kTriSmem * static_cast<int>(sizeof(cx<R>)), bwd = (kTriSmem + kRedSmem) * static_cast<int>(sizeof(cx<R>));
     APHI_CUDA(cudaFuncSetAttribute(k_fwd_diag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
     APHI_CUDA(cudaFuncSetAttribute(k_fwd_gather<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
@@ -552,6 +569,7 @@ aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
         f->tc_group = group && group[0] == '4' ? 4 : 2;
         const char* pre = std::getenv("APHI_TC_PRESPLIT");
         f->presplit = !(pre && pre[0] == '0');
+        f->tc_i8 = !pre;
         const char* pst = std::getenv("APHI_TC_PRESTAGES");
         f->pre_stages = pst && pst[0] == '4' ? 4 : 3;
         if (precision == 32) f->tcws_stride = an->tc_ws_units * 256;

@@ -38,10 +38,11 @@ struct aphi_factor {
     int kr_cap = 0;
     bool factored = false;
     bool use_tc = true;         // FP32: tensor-core updates (APHI_NO_TC=1 selects the SIMT kernels)
-    int tc_split = 3;           // FP32 tensor-core updates: TF32 pieces per operand (3, or 2: hh + hl + lh)
+    int tc_split = 3;           // FP32 tensor-core updates: 3 TF32 pieces per operand, or 2: INT8 digits (tc_i8), or two pieces
     int tc_stages = 2;          // split 2: split-operand stages in flight (2 or 3; APHI_TC_STAGES)
     int tc_group = 2;           // split 2: stages per fresh main accumulator (2 or 4; APHI_TC_GROUP)
     bool presplit = true;       // split 2: operands split once per panel group (k_tc_split; APHI_TC_PRESPLIT=0: in the tile)
+    bool tc_i8 = true;          // split 2: INT8 digits (i8_update.cuh); APHI_TC_PRESPLIT set, to anything: two TF32 pieces
     int pre_stages = 3;         // plane buffers of the pre-split tile (APHI_TC_PRESTAGES=4: four; always four with tc_group 4)
     unsigned char* dws = nullptr;  // FP64: the trailing updates' prepared operands (byte digits), dws_stride bytes per entry
     long long dws_stride = 0;      // (APHI_DMMA_PRESCALE=0: none, the tiles run on DMMA from the panels)

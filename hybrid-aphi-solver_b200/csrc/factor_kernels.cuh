@@ -14,6 +14,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cfloat>
+
 #include "analysis.hpp"
 #include "common.cuh"
 #include "i8_update.cuh"
@@ -521,11 +523,12 @@ __device__ __forceinline__ void red_sub(double* p, double v) {
 // per factorization beside 117 ms of tiles) and, on small fronts, by the
 // passes' dependent round trips (11 us a launch).
 template <class R, class C>
-__global__ void __launch_bounds__(256) k_i8_split(Sched S, long long item0, const cx<R>* Lb, long long lstride,
-                                                  unsigned char* ws, long long ws_stride, int kcap) {
+__global__ void __launch_bounds__(256, 2) k_i8_split(Sched S, long long item0, const cx<R>* Lb, long long lstride,
+                                                     unsigned char* ws, long long ws_stride, int kcap) {
+    using Real = I8Real<R>;
     constexpr int kWarps = 8;
-    __shared__ double dre[kWidePair], dim[kWidePair], up[kWidePair];  // D 2^-h, 2^h
-    __shared__ int top[2][kWarps][32];                                // largest high words of A, B
+    __shared__ R dre[kWidePair], dim[kWidePair], up[kWidePair];  // D 2^-h, 2^h
+    __shared__ int top[2][kWarps][32];                           // largest sizes of A, B
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, p0 = it.a;
     const int w = S.first[s + 1] - S.first[s];
@@ -539,37 +542,31 @@ __global__ void __launch_bounds__(256) k_i8_split(Sched S, long long item0, cons
     const int r = it.b + 32 * blockIdx.z + lane;  // row within the trailing part
     const bool in = pe + r < m;
     const cx<R>* X = P + (in ? pe + r : pe) + static_cast<long long>(p0) * m;
-    for (int k = threadIdx.x; k < K; k += 256) {
-        const cx<R> d = P[(p0 + k) + static_cast<long long>(p0 + k) * m];
-        const double re = d.re, im = d.im;
-        const int e = __double2hiint(fmax(fabs(re), fabs(im))) >> 20;
-        const int h = e == 0 || e == 0x7ff ? 0 : (e - 1023) >> 1;
-        const double dn = __hiloint2double((1023 - h) << 20, 0);
-        dre[k] = re * dn;
-        dim[k] = im * dn;
-        up[k] = __hiloint2double((1023 + h) << 20, 0);
+    for (int k = threadIdx.x; k < kWidePair; k += 256) {
+        const cx<R> d = k < K ? P[(p0 + k) + static_cast<long long>(p0 + k) * m] : cx<R>{0, 0};
+        const int e = max(Real::exponent(Real::size(d.re)), Real::exponent(Real::size(d.im)));
+        const int h = e == 0 || e == Real::none ? 0 : (e - Real::bias) >> 1;
+        const R dn = Real::pow2(Real::bias - h);
+        dre[k] = d.re * dn;
+        dim[k] = d.im * dn;
+        up[k] = Real::pow2(Real::bias + h);
     }
     __syncthreads();
-    auto load = [&](int c, double (&re)[16], double (&im)[16]) {
+    auto load = [&](int c, cx<R> (&x)[16]) {
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int k = 16 * c + u;
-            const cx<R> x = in && k < K ? X[static_cast<long long>(k) * m] : cx<R>{0, 0};
-            re[u] = x.re;
-            im[u] = x.im;
-        }
+        for (int u = 0; u < 16; ++u)
+            x[u] = in && 16 * c + u < K ? X[static_cast<long long>(16 * c + u) * m] : cx<R>{0, 0};
     };
     int ta = 0, tb = 0;
     for (int c = warp; 16 * c < K; c += kWarps) {
-        double re[16], im[16];
-        load(c, re, im);
+        cx<R> x[16];
+        load(c, x);
 #pragma unroll
         for (int u = 0; u < 16; ++u) {
-            const int k = min(16 * c + u, K - 1);
-            const double ar = re[u] * dre[k] - im[u] * dim[k], ai = re[u] * dim[k] + im[u] * dre[k];
-            const double br = re[u] * up[k], bi = im[u] * up[k];
-            ta = max(ta, max(__double2hiint(ar) & 0x7fffffff, __double2hiint(ai) & 0x7fffffff));
-            tb = max(tb, max(__double2hiint(br) & 0x7fffffff, __double2hiint(bi) & 0x7fffffff));
+            const int k = 16 * c + u;
+            const R ar = x[u].re * dre[k] - x[u].im * dim[k], ai = x[u].re * dim[k] + x[u].im * dre[k];
+            ta = max(ta, max(Real::size(ar), Real::size(ai)));
+            tb = max(tb, max(Real::size(x[u].re * up[k]), Real::size(x[u].im * up[k])));
         }
     }
     top[0][warp][lane] = ta;
@@ -581,70 +578,63 @@ __global__ void __launch_bounds__(256) k_i8_split(Sched S, long long item0, cons
         tb = max(tb, top[1][v][lane]);
     }
     // Biased exponents; tiny rows share one that keeps every scale normal.
-    const int ea = max(ta >> 20, 200), eb = max(tb >> 20, 200);
-    constexpr int kBits = 8 * C::S - 2;   // |integer| <= 2^kBits
-    constexpr int kTop = 4 * (2 * C::S - 1 - C::L);  // half of log2 of the last kept level's weight
-    const double fa = __hiloint2double((1023 + kBits + 1022 - ea) << 20, 0);
-    const double fb = __hiloint2double((1023 + kBits + 1022 - eb) << 20, 0);
+    const int ea = max(Real::exponent(ta), Real::least), eb = max(Real::exponent(tb), Real::least);
+    constexpr int kBits = 8 * C::S - 2;              // |integer| <= 2^kBits
+    constexpr int kTop = 4 * (2 * C::S - 1 - C::L) + Real::shift;  // half of log2 of the last kept level's weight
+    const R fa = Real::pow2(2 * Real::bias - 1 + kBits - ea), fb = Real::pow2(2 * Real::bias - 1 + kBits - eb);
     if (warp == 0) {
-        double* scale = reinterpret_cast<double*>(region + i8_scale_off<C>(Rp, nst));
-        const double bad = __longlong_as_double(0x7ff8000000000000LL);
-        scale[r] = ea >= 0x7ff ? bad : __hiloint2double((ea + 1 - kBits + kTop) << 20, 0);
-        scale[Rp + r] = eb >= 0x7ff ? bad : __hiloint2double((eb + 1 - kBits + kTop) << 20, 0);
+        R* scale = reinterpret_cast<R*>(region + i8_scale_off<C>(Rp, nst));
+        const R bad = Real::pow2(Real::none) - Real::pow2(Real::none);  // NaN
+        scale[r] = ea >= Real::none ? bad : Real::pow2(ea + 1 - kBits + kTop);
+        scale[Rp + r] = eb >= Real::none ? bad : Real::pow2(eb + 1 - kBits + kTop);
     }
     // 16 values -> digit p of each, 16 bytes, to dst + p * step.
-    auto digits = [&](const double (&v)[16], double f, unsigned char* dst, int step) {
-        constexpr long long kBias = (1LL << (8 * (C::S - 1))) / 255 * 128;  // 128 in every byte but the top digit's
+    auto digits = [&](const R (&v)[16], R f, unsigned char* dst, int step) {
+        using Int = decltype(Real::integer(R(0)));
+        constexpr Int kBias = static_cast<Int>((1LL << (8 * (C::S - 1))) / 255 * 128);  // 128 in every byte but the top digit's
+        static_assert(sizeof(Int) == C::S, "one byte per digit");
         unsigned out[C::S][4];
 #pragma unroll
-        for (int g = 0; g < 4; ++g) {
-            unsigned lo[4], hi[4];
+        for (int g = 0; g < 4; ++g)
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-                const long long z = (__double2ll_rn(v[4 * g + u] * f) + kBias) ^ kBias;
-                lo[u] = static_cast<unsigned>(z);
-                hi[u] = static_cast<unsigned>(static_cast<unsigned long long>(z) >> 32);
+            for (int h = 0; h < C::S / 4; ++h) {  // bytes 4 h .. 4 h + 3 of four numbers
+                unsigned z[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    z[u] = static_cast<unsigned>(((Real::integer(v[4 * g + u] * f) + kBias) ^ kBias) >> (h ? 8 * sizeof(Int) - 32 : 0));
+                const unsigned t0 = __byte_perm(z[0], z[1], 0x5140), t1 = __byte_perm(z[2], z[3], 0x5140);
+                const unsigned t2 = __byte_perm(z[0], z[1], 0x7362), t3 = __byte_perm(z[2], z[3], 0x7362);
+                // byte b = digit S - 1 - b
+                out[C::S - 1 - 4 * h][g] = __byte_perm(t0, t1, 0x5410);
+                out[C::S - 2 - 4 * h][g] = __byte_perm(t0, t1, 0x7632);
+                out[C::S - 3 - 4 * h][g] = __byte_perm(t2, t3, 0x5410);
+                out[C::S - 4 - 4 * h][g] = __byte_perm(t2, t3, 0x7632);
             }
-            // byte b of the four numbers = digit S - 1 - b
-            unsigned t[8];
-            t[0] = __byte_perm(lo[0], lo[1], 0x5140), t[1] = __byte_perm(lo[2], lo[3], 0x5140);
-            t[2] = __byte_perm(lo[0], lo[1], 0x7362), t[3] = __byte_perm(lo[2], lo[3], 0x7362);
-            t[4] = __byte_perm(hi[0], hi[1], 0x5140), t[5] = __byte_perm(hi[2], hi[3], 0x5140);
-            t[6] = __byte_perm(hi[0], hi[1], 0x7362), t[7] = __byte_perm(hi[2], hi[3], 0x7362);
-#pragma unroll
-            for (int b = 0; b < C::S; ++b)
-                out[C::S - 1 - b][g] = __byte_perm(t[b / 2 * 2], t[b / 2 * 2 + 1], b % 2 ? 0x7632 : 0x5410);
-        }
 #pragma unroll
         for (int p = 0; p < C::S; ++p)
             *reinterpret_cast<uint4*>(dst + p * step) = make_uint4(out[p][0], out[p][1], out[p][2], out[p][3]);
     };
     for (int c = warp; c < 2 * nst; c += kWarps) {
-        double re[16], im[16], v[16];
-        load(c, re, im);
+        cx<R> x[16];
+        R v[16];
+        load(c, x);
         unsigned char* A = region + i8_a_off<C>(nst, r, c >> 1) + i8_off(r % kTcM, c & 1);
         unsigned char* B = region + i8_b_off<C>(Rp, nst, r, c >> 1) + i8_off(r % C::Nc, c & 1);
         constexpr int kPlaneA = kTcM * kI8K, kDigitB = C::W * kI8K, kHalfB = C::Nc * kI8K;
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int k = min(16 * c + u, K - 1);
-            v[u] = re[u] * dre[k] - im[u] * dim[k];
-        }
+        for (int u = 0; u < 16; ++u) v[u] = x[u].re * dre[16 * c + u] - x[u].im * dim[16 * c + u];
         digits(v, fa, A, 2 * kPlaneA);
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            const int k = min(16 * c + u, K - 1);
-            v[u] = re[u] * dim[k] + im[u] * dre[k];
-        }
+        for (int u = 0; u < 16; ++u) v[u] = x[u].re * dim[16 * c + u] + x[u].im * dre[16 * c + u];
         digits(v, fa, A + kPlaneA, 2 * kPlaneA);
 #pragma unroll
-        for (int u = 0; u < 16; ++u) re[u] = re[u] * up[min(16 * c + u, K - 1)];
-        digits(re, fb, B, kDigitB);
-        digits(re, fb, B + C::imageB + kHalfB, kDigitB);
+        for (int u = 0; u < 16; ++u) v[u] = x[u].re * up[16 * c + u];
+        digits(v, fb, B, kDigitB);
+        digits(v, fb, B + C::imageB + kHalfB, kDigitB);
 #pragma unroll
-        for (int u = 0; u < 16; ++u) im[u] = im[u] * up[min(16 * c + u, K - 1)];
-        digits(im, fb, B + kHalfB, kDigitB);
-        digits(im, -fb, B + C::imageB, kDigitB);
+        for (int u = 0; u < 16; ++u) v[u] = x[u].im * up[16 * c + u];
+        digits(v, fb, B + kHalfB, kDigitB);
+        digits(v, -fb, B + C::imageB, kDigitB);
     }
 }
 
@@ -653,21 +643,29 @@ __global__ void __launch_bounds__(256) k_i8_split(Sched S, long long item0, cons
 // tiles of Nc columns. Persistent: one CTA per SM (its accumulators are all
 // of TMEM) walks the launch's tiles -- entries outermost, so that one
 // entry's operands stay in L2 -- in three roles that run side by side:
-//   warp 0, lane 0  copies operand stages (two bulk copies each) into the
-//                   ring of buffers, across tile boundaries;
+//   warp 0, lane 0  decodes the tiles into a ring of slots and copies their
+//                   operand stages (two bulk copies each) into the ring of
+//                   buffers, across tile boundaries;
 //   warp 1, lane 0  issues each stage's MMAs;
-//   warps 2 .. 9    read the destination while the tile is computed, then the
+//   warps 2 .. 17   read the destination while the tile is computed, then the
 //                   accumulators, and write the difference.
 // A tile's MMAs wait until the previous tile's accumulators have been read.
 // Every wait is bounded and gives up early once another role has failed.
 //
-// Measured on the 32^3 cylinder, two FP64 entries: the trailing updates of a
-// factorization take 178 ms (75 useful FP64 TFLOP/s, 2.7e15 INT8 operations/s)
-// against 486 ms (27.5) on DMMA with pre-scaled operands; 24^3, eight
-// entries: 117 against 292 ms; 8^3, one entry: 11 against 26 us a launch. It
-// is the faster one from the smallest launches up, so every FP64 trailing
-// update takes it.
-constexpr int kI8Threads = 320;
+// Measured, trailing updates of a factorization (the form that each replaced):
+//   FP64, 32^3, two entries    177 ms (486, DMMA)     76 useful FP64 TFLOP/s
+//   FP64, 24^3, eight entries  112 ms (292)
+//   FP64, 8^3, one entry       10.4 us a launch (26)
+//   FP32, 32^3, six entries    166 ms (311, two TF32 pieces)
+//   FP32, 24^3, six entries     31 ms (56)
+//   FP32, 12^3, six entries    1.0 ms (1.5)
+// It is the faster form from the smallest launches up, so every FP64 trailing
+// update takes it, and every FP32 one that asks for two pieces. In FP64 an
+// SM's shared memory bounds a tile: per stage the MMAs read 240 KB of digits
+// and the copies write 96 KB, 2,700 cycles beside 2,304 of tensor work (K =
+// 256: 22,000 cycles, then 4,000 to read the accumulators); in FP32 the MMAs
+// take 11,000 cycles and the accumulators' reading 3,000.
+constexpr int kI8Threads = 64 + 16 * 32;
 
 template <class R, class C>
 __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long item0, int count, int entries,
@@ -675,13 +673,29 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
                                                              long long cbstride, int kcap, const unsigned char* ws,
                                                              long long ws_stride, int* err) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    constexpr int kHalves = kTcN / C::Nc, kEpWarps = 8;
+    constexpr int kHalves = kTcN / C::Nc, kEpWarps = kI8Threads / 32 - 2;
+    // A tile as the producer decodes it, a few tiles ahead of the others.
+    struct Tile {
+        cx<R>* panel;   // (i0, j0) in the panel, leading dimension m
+        cx<R>* cb;      // (i0, j0) in the contribution block, leading dimension cs
+        const R* scale_a;  // of row i0
+        const R* scale_b;  // of column j0
+        int i0, j0, m, cs, cut, nst;  // cut: columns below the panel's end; nst 0: no more tiles
+    };
+    // A producer loads at most Stages stages beyond the oldest unfinished
+    // MMAs, and those wait for the epilogue's previous tile: it is never
+    // more than Stages + 2 tiles ahead of a reader.
+    constexpr int kSlots = 8;
+    static_assert(C::Stages + 2 < kSlots, "a tile's slot must not be rewritten before everyone has read it");
     uint64_t* full = reinterpret_cast<uint64_t*>(smem_raw + C::Stages * C::stage);
     uint64_t* empty = full + C::Stages;
     uint64_t* acc_full = empty + C::Stages;
     uint64_t* acc_empty = acc_full + 1;
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 1);
+    uint64_t* ready = acc_empty + 1;
+    Tile* slots = reinterpret_cast<Tile*>(ready + kSlots);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slots + kSlots);
     volatile int* state = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] failed, [1] stages committed, [2] stages loaded
+    static_assert((2 * C::Stages + 2 + kSlots) * 8 + kSlots * sizeof(Tile) + 16 <= C::extra, "barriers and slots");
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -689,12 +703,13 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (int b = 0; b < C::Stages; ++b) {
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(full + b)));
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(empty + b)));
-        }
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(acc_full)));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(acc_empty)), "r"(kEpWarps));
+        auto init = [](uint64_t* b, int n) {
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(b)), "r"(n));
+        };
+        for (int b = 0; b < C::Stages; ++b) init(full + b, 1), init(empty + b, 1);
+        for (int b = 0; b < kSlots; ++b) init(ready + b, 1);
+        init(acc_full, 1);
+        init(acc_empty, kEpWarps);
         asm volatile("fence.mbarrier_init.release.cluster;");
         state[0] = 0;
         state[1] = 0;
@@ -704,45 +719,41 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
-
-    // This CTA's tiles: g = blockIdx.x, + gridDim.x, ...; the next one with
-    // entries on or below the front's diagonal.
-    struct Tile {
-        long long g;
-        int entry, s, p0, i0, j0, w, m, K, nst, d;
-    };
-    const long long total = static_cast<long long>(count) * kHalves * entries;
-    auto next = [&](Tile& t, long long g) -> bool {
-        for (; g < total; g += gridDim.x) {
-            t.entry = static_cast<int>(g / (count * kHalves));
-            const int q = static_cast<int>(g - static_cast<long long>(t.entry) * count * kHalves);
-            const Item it = S.items[item0 + q / kHalves];
-            t.s = it.s;
-            t.p0 = it.a;
-            t.i0 = it.b;
-            t.j0 = it.c + (q % kHalves) * C::Nc;
-            t.d = it.d;
-            t.m = S.rows[t.s];
-            if (t.j0 >= t.m || t.i0 + kTcM <= t.j0) continue;
-            t.w = S.first[t.s + 1] - S.first[t.s];
-            t.K = min(kcap, t.w - t.p0);
-            t.nst = (t.K + kI8K - 1) / kI8K;
-            t.g = g;
-            return true;
-        }
-        return false;
+    // Tile n of this CTA once the producer has decoded it; false: failed.
+    auto tile = [&](int n, Tile& t) {
+        if (!mbar_wait_live(smem_u32(ready + n % kSlots), (n / kSlots) & 1, state)) return false;
+        t = slots[n % kSlots];
+        return true;
     };
 
     if (tid == 0) {
-        int c = 0;  // stages loaded so far
-        Tile t;
-        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x)) {
-            const int pe = t.p0 + t.K;
-            const int Rp = (t.m - pe + kTcM - 1) / kTcM * kTcM;
-            const unsigned char* region = ws + ws_stride * t.entry + static_cast<long long>(t.d) * 256;
-            const unsigned char* A = region + i8_a_off<C>(t.nst, t.i0 - pe, 0);
-            const unsigned char* B = region + i8_b_off<C>(Rp, t.nst, t.j0 - pe, 0);
-            for (int k = 0; k < t.nst; ++k, ++c) {
+        int c = 0, n = 0;  // stages loaded, tiles decoded so far
+        auto publish = [&]() {
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(ready + n % kSlots)) : "memory");
+            ++n;
+        };
+        const long long total = static_cast<long long>(count) * kHalves * entries;
+        for (long long g = blockIdx.x; g < total && !state[0]; g += gridDim.x) {
+            const int entry = static_cast<int>(g / (count * kHalves));
+            const int q = static_cast<int>(g - static_cast<long long>(entry) * count * kHalves);
+            const Item it = S.items[item0 + q / kHalves];
+            const int s = it.s, i0 = it.b, j0 = it.c + (q % kHalves) * C::Nc;
+            const int m = S.rows[s];
+            if (j0 >= m || i0 + kTcM <= j0) continue;  // no entry on or below the diagonal
+            const int w = S.first[s + 1] - S.first[s];
+            const int K = min(kcap, w - it.a), pe = it.a + K, cs = m - w;
+            const int nst = (K + kI8K - 1) / kI8K;
+            const int Rp = (m - pe + kTcM - 1) / kTcM * kTcM;
+            const unsigned char* region = ws + ws_stride * entry + static_cast<long long>(it.d) * 256;
+            const R* scale = reinterpret_cast<const R*>(region + i8_scale_off<C>(Rp, nst));
+            slots[n % kSlots] = Tile{Lb + lstride * entry + S.loff[s] + i0 + static_cast<long long>(j0) * m,
+                                     CBb + cbstride * entry + (cs > 0 ? S.cboff[s] : 0) + (i0 - w) +
+                                         static_cast<long long>(j0 - w) * cs,
+                                     scale + (i0 - pe), scale + Rp + (j0 - pe), i0, j0, m, cs, w - j0, nst};
+            publish();
+            const unsigned char* A = region + i8_a_off<C>(nst, i0 - pe, 0);
+            const unsigned char* B = region + i8_b_off<C>(Rp, nst, j0 - pe, 0);
+            for (int k = 0; k < nst; ++k, ++c) {
                 const int b = c % C::Stages;
                 if (c >= C::Stages && !mbar_wait_live(smem_u32(empty + b), ((c / C::Stages) - 1) & 1, state)) {
                     state[0] = 1;
@@ -755,14 +766,17 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
                 state[2] = c + 1;
             }
         }
+        slots[n % kSlots].nst = 0;
+        publish();
     } else if (tid == 32) {
-        int c = 0, n = 0;  // stages, tiles issued so far
+        int c = 0;  // stages issued so far
         Tile t;
-        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x), ++n) {
-            if (n > 0 && !mbar_wait_live(smem_u32(acc_empty), (n - 1) & 1, state)) {
+        for (int n = 0;; ++n) {
+            if (!tile(n, t) || (t.nst > 0 && n > 0 && !mbar_wait_live(smem_u32(acc_empty), (n - 1) & 1, state))) {
                 state[0] = 1;
                 break;
             }
+            if (t.nst == 0) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
             for (int k = 0; k < t.nst; ++k, ++c) {
                 const int b = c % C::Stages;
@@ -775,58 +789,66 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
                 mma_commit(smem_u32(empty + b));
                 state[1] = c + 1;
             }
-            if (!state[0]) mma_commit(smem_u32(acc_full));
+            if (state[0]) break;
+            mma_commit(smem_u32(acc_full));
         }
     } else if (warp >= 2) {
-        constexpr int kCols = C::Nc / 2, kChunk = 4;  // columns per warp, and at a time
-        const int quad = warp & 3, half = (warp - 2) >> 2;
+        constexpr int kCols = C::Nc / (kEpWarps / 4);  // columns per warp
+        constexpr int kChunk = 4;                      // columns per TMEM read
+        constexpr R kLargest = sizeof(R) == 8 ? static_cast<R>(DBL_MAX) : static_cast<R>(FLT_MAX);
+        const int quad = warp & 3, c0 = ((warp - 2) >> 2) * kCols;
         const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
-        int n = 0;
+        const int r = quad * 32 + lane;
         Tile t;
-        for (bool more = next(t, blockIdx.x); more && !state[0]; more = next(t, t.g + gridDim.x), ++n) {
-            const int cs = t.m - t.w, pe = t.p0 + t.K;
-            const int Rp = (t.m - pe + kTcM - 1) / kTcM * kTcM;
-            cx<R>* Ls = Lb + lstride * t.entry + S.loff[t.s];
-            cx<R>* CBs = CBb + cbstride * t.entry + (cs > 0 ? S.cboff[t.s] : 0);
-            const double* scale = reinterpret_cast<const double*>(
-                ws + ws_stride * t.entry + static_cast<long long>(t.d) * 256 + i8_scale_off<C>(Rp, t.nst));
-            const int i = t.i0 + quad * 32 + lane, j0 = t.j0 + half * kCols;
-            // The destination, read while the tile is computed.
-            cx<R> old[kCols];
-            auto at = [&](int j) {
-                return j < t.w ? Ls + i + static_cast<long long>(j) * t.m
-                               : CBs + (i - t.w) + static_cast<long long>(j - t.w) * cs;
-            };
-#pragma unroll
-            for (int q = 0; q < kCols; ++q) {
-                const int j = j0 + q;
-                old[q] = j < t.m && i < t.m && i >= j ? *at(j) : cx<R>{0, 0};
+        for (int n = 0;; ++n) {
+            if (!__all_sync(0xffffffffu, tile(n, t))) {
+                state[0] = 1;
+                break;
             }
-            const double sa = scale[i - pe];
-            const double* sb = scale + Rp + (j0 - pe);
-            bool mine = mbar_wait_live(smem_u32(acc_full), n & 1, state);
-            mine = __all_sync(0xffffffffu, mine);  // the TMEM loads are warp-wide
-            if (!mine) {
+            if (t.nst == 0) break;
+            // This thread's entries: row i0 + r, columns j0 + c0 + q up to the
+            // diagonal (q <= last), those below the cut in the panel, the rest
+            // in the CB.
+            const int last = t.i0 + r < t.m ? min(t.m - 1, t.i0 + r) - t.j0 - c0 : -1;
+            const int cut = t.cut - c0;
+            cx<R>* const in_cb = t.cb + r + static_cast<long long>(c0) * t.cs;
+            cx<R>* const base = cut > 0 ? t.panel + r + static_cast<long long>(c0) * t.m : in_cb;
+            const long long ld = cut > 0 ? t.m : t.cs;
+            const bool mixed = cut > 0 && cut < kCols;
+            auto at = [&](int q) {
+                return mixed && q >= cut ? in_cb + static_cast<long long>(q) * t.cs : base + q * ld;
+            };
+            // The destination and the scales (lane q: column q's), read while
+            // the tile is computed.
+            cx<R> old[kCols];
+#pragma unroll
+            for (int q = 0; q < kCols; ++q) old[q] = q <= last ? *at(q) : cx<R>{0, 0};
+            const R sa = t.scale_a[r], sb = t.scale_b[c0 + lane % kCols];
+            bool live = mbar_wait_live(smem_u32(acc_full), n & 1, state);
+            live = __all_sync(0xffffffffu, live);  // the TMEM loads are warp-wide
+            if (!live) {
                 state[0] = 1;
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;");
 #pragma unroll
             for (int q0 = 0; q0 < kCols; q0 += kChunk) {
-                double re[kChunk], im[kChunk];
+                R re[kChunk], im[kChunk];
 #pragma unroll
-                for (int part = 0; part < 2; ++part) {
+                for (int h = 0; h < 2; ++h) {
                     int v[C::L][kChunk];
 #pragma unroll
-                    for (int l = 0; l < C::L; ++l)
-                        tmem_ld4(tmem + lanes + l * C::W + part * C::Nc + half * kCols + q0, v[l]);
+                    for (int l = 0; l < C::L; ++l) tmem_ld(tmem + lanes + l * C::W + h * C::Nc + c0 + q0, v[l]);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                     for (int q = 0; q < kChunk; ++q) {
-                        int a[C::L];
+                        int d[C::L];
 #pragma unroll
-                        for (int l = 0; l < C::L; ++l) a[l] = v[l][q];
-                        (part ? im : re)[q] = i8_combine<C::L>(a);
+                        for (int l = 0; l < C::L; ++l) {
+                            asm volatile("" : "+r"(v[l][q]));  // not before the wait
+                            d[l] = v[l][q];
+                        }
+                        (h ? im : re)[q] = i8_combine(d);
                     }
                 }
                 if (q0 + kChunk == kCols) {  // everything this warp reads has been read
@@ -837,12 +859,10 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
                 }
 #pragma unroll
                 for (int q = 0; q < kChunk; ++q) {
-                    const int j = j0 + q0 + q;
-                    if (j < t.m && i < t.m && i >= j) {
-                        const double sc = sa * sb[q0 + q];
-                        *at(j) = cx<R>{static_cast<R>(fma(-re[q], sc, static_cast<double>(old[q0 + q].re))),
-                                       static_cast<R>(fma(-im[q], sc, static_cast<double>(old[q0 + q].im)))};
-                    }
+                    R s = sa * __shfl_sync(0xffffffffu, sb, q0 + q);
+                    s = s > kLargest ? kLargest : s;  // so that 0 s is 0 (a NaN stays)
+                    if (q0 + q <= last)
+                        *at(q0 + q) = cx<R>{fma(-re[q], s, old[q0 + q].re), fma(-im[q], s, old[q0 + q].im)};
                 }
             }
         }

@@ -2,8 +2,8 @@
 // products of byte digits, accumulated exactly in 32-bit integers.
 //
 // The update is F -= W B^T over one panel group's K columns (W = L D, B = L,
-// complex). FP64 runs at 37 TFLOP/s on this device, INT8 at over a hundred times
-// that, so the FP64 operands are written as fixed-point numbers and those as
+// complex). FP64 runs at 37 TFLOP/s on this device, INT8 at over a hundred
+// times that, so the FP64 operands are written as fixed-point numbers and those as
 // base-256 digits (the error-free splitting of Ozaki, Ogita, Oishi and Rump,
 // "Error-free transformations of matrix multiplication", 2012):
 //
@@ -23,6 +23,14 @@
 // the 32^3 cylinder at 1 MHz the smallest pivot came out 2e-8 off, and 1e-10
 // from the FP64 FMA chains' with eight, nearer to the reference's (2.9e-10)
 // than theirs (4.0e-10).
+//
+// FP32 operands (the sweep's factors, which a refinement uses) take four
+// digits and four levels: 2^-30 of the row's largest component, against 2^-22
+// of each number with the two TF32 pieces they took before. On the 32^3
+// sweep's first six frequencies the factors' solves are 3 to 10 times more
+// accurate and the refinement needs 3-8 iterations (4-13). Three digits cost
+// 8 % less of the tiles' time and one or two iterations more.
+//
 // The pivots' magnitudes are shared out between the operands (column k of W is
 // divided and of B multiplied by 2^h, h half of D_k's exponent), so that the
 // columns of both have the scale of a Cholesky factor's and one exponent per
@@ -45,6 +53,8 @@
 
 namespace aphi_b200 {
 
+constexpr int kI8FloatShift = 17;  // see i8_combine
+
 // S digits per operand, L levels kept, Nc complex columns per tile, Stages
 // operand buffers.
 template <int S_, int L_, int Nc_, int Stages_>
@@ -55,12 +65,14 @@ struct I8Shape {
     static constexpr int imageB = S * W * kI8K;            // one stage of Nc B rows, one image
     static constexpr int blockB = 2 * imageB;              // [Br | Bi] per digit, then [-Bi | Br] per digit
     static constexpr int stage = blockA + blockB;
-    static constexpr int smem = Stages * stage + 256;
+    static constexpr int extra = 1024;                     // barriers and tile slots
+    static constexpr int smem = Stages * stage + extra;
     static constexpr int tmem = 512;                       // columns allocated (L W of them used)
     static_assert(L * W <= tmem && L >= S && L <= 2 * S - 1, "levels must fit TMEM");
     static_assert(smem <= 227 * 1024, "operand buffers exceed shared memory");
 };
 using I8Fp64 = I8Shape<kI8Digits64, kI8Levels64, kI8Nc64, 2>;
+using I8Fp32 = I8Shape<kI8Digits32, kI8Levels32, kI8Nc32, 3>;
 
 // A front's region (R padded rows, nst stages of 32 columns): the A blocks
 // [R / 128][nst], the B blocks [R / Nc][nst], then a scale per A row and per
@@ -133,25 +145,71 @@ __device__ __forceinline__ void i8_issue(uint32_t stage, uint32_t tmem, bool fir
     }
 }
 
-__device__ __forceinline__ void tmem_ld4(uint32_t taddr, int (&v)[4]) {
+// 32 lanes x N consecutive columns of TMEM into registers.
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, int (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, int (&v)[4]) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0,%1,%2,%3}, [%4];"
                  : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                  : "r"(taddr));
 }
+// The operands' arithmetic in the factor's type: bits ordered like the
+// magnitude (infinities and NaN on top), biased exponents, powers of two, and
+// the nearest integer.
+template <class R>
+struct I8Real;
+template <>
+struct I8Real<double> {
+    // none: infinities and NaN; least: the smallest exponent told apart;
+    // shift: see i8_combine.
+    static constexpr int bias = 1023, none = 0x7ff, least = 200, shift = 0;
+    static __device__ __forceinline__ int size(double x) { return __double2hiint(x) & 0x7fffffff; }
+    static __device__ __forceinline__ int exponent(int size) { return size >> 20; }
+    static __device__ __forceinline__ double pow2(int biased) { return __hiloint2double(biased << 20, 0); }
+    static __device__ __forceinline__ unsigned long long integer(double x) { return __double2ll_rn(x); }
+};
+template <>
+struct I8Real<float> {
+    static constexpr int bias = 127, none = 0xff, least = 30, shift = kI8FloatShift;
+    static __device__ __forceinline__ int size(float x) { return __float_as_int(x) & 0x7fffffff; }
+    static __device__ __forceinline__ int exponent(int size) { return size >> 23; }
+    static __device__ __forceinline__ float pow2(int biased) { return __int_as_float(biased << 23); }
+    static __device__ __forceinline__ unsigned integer(float x) { return __float2int_rn(x); }
+};
 
-// sum_l a_l 256^(L - 1 - l) as a double: exact 64-bit sums of up to four
-// levels, then one rounding.
-template <int L>
-__device__ __forceinline__ double i8_combine(const int (&a)[L]) {
-    constexpr int kLo = L > 4 ? L - 4 : 0;  // levels [kLo, L) in the low word
-    long long lo = a[L - 1];
-#pragma unroll
-    for (int l = L - 2; l >= kLo; --l) lo += static_cast<long long>(a[l]) * (1 << (8 * (L - 1 - l)));
-    if constexpr (kLo == 0) return static_cast<double>(lo);
-    long long hi = a[kLo > 0 ? kLo - 1 : 0];
-#pragma unroll
-    for (int l = kLo - 2; l >= 0; --l) hi += static_cast<long long>(a[l]) * (1 << (8 * (kLo - 1 - l)));
-    return fma(static_cast<double>(hi), 4294967296.0, static_cast<double>(lo));
+// sum_l a_l 256^(3 - l) of the first four levels as hi 2^16 + lo, exactly and
+// in 32-bit steps: the top digits are at most 64, so a_0 is below 2^23, a_1
+// below 2^25 and hi below 2^31 for K = 512.
+__device__ __forceinline__ void i8_top(const int* a, int& hi, int& lo) {
+    hi = (a[0] << 8) + a[1] + (a[2] >> 8);
+    lo = ((a[2] & 255) << 8) + a[3];
+}
+
+// The levels' sum in units of the last one (float: times 2^(-2 kI8FloatShift),
+// so that the rows' scales, larger by 2^kI8FloatShift each, multiply to about
+// the size of the product itself and stay within a float's range with it). The
+// accumulators are read between
+// two tiles' MMAs, so this is on the critical path: the integers become
+// doubles by their place in the mantissa of a power of two (minus that power),
+// not by conversions, and the work is spread over the integer, multiply and
+// FP64 pipes. One rounding (double), or two of parts of the sum (float).
+__device__ __forceinline__ double i8_combine(const int (&a)[8]) {
+    auto real32 = [](int v) { return __hiloint2double(0x43300000, v ^ 0x80000000) - 4503601774854144.0; };
+    auto real51 = [](long long v) { return __longlong_as_double(v + 0x4338000000000000LL) - 6755399441055744.0; };
+    int hi, lo;
+    i8_top(a, hi, lo);
+    // levels 4 .. 7: below 2^51
+    const long long low = a[4] * 16777216LL + (a[5] * 65536LL + (a[6] * 256LL + a[7]));
+    return fma(fma(real32(hi), 65536.0, real32(lo)), 4294967296.0, real51(low));
+}
+__device__ __forceinline__ float i8_combine(const int (&a)[4]) {
+    constexpr float kUnit = 1.0f / (1LL << (2 * kI8FloatShift));
+    int hi, lo;
+    i8_top(a, hi, lo);
+    return fmaf(__int2float_rn(hi), 65536.0f * kUnit, __int2float_rn(lo) * kUnit);
 }
 
 }  // namespace aphi_b200

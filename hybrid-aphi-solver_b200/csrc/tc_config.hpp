@@ -47,6 +47,9 @@ constexpr int kI8K = 32;         // columns of K per stage (one MMA step)
 constexpr int kI8Digits64 = 8;   // base-256 digits per FP64 operand
 constexpr int kI8Levels64 = 8;   // digit-product levels kept
 constexpr int kI8Nc64 = 32;      // complex columns per tile
+constexpr int kI8Digits32 = 4;   // the FP32 trailing update's
+constexpr int kI8Levels32 = 4;
+constexpr int kI8Nc32 = 64;
 // 256-byte units of a front's prepared operands: R (a multiple of 128) rows,
 // K columns; per row and column 2 S bytes of A digits and 4 S of B digits,
 // and two doubles per row.

@@ -281,11 +281,13 @@ int aphi_factor_destroy(aphi_factor* f);
  * entries. Discards the current factorization. For continuous batching,
  * where each batch's size is known only when it is formed. */
 int aphi_factor_set_batch(aphi_factor* f, int batch);
-/* FP32 factors: how many TF32 pieces the tensor-core trailing update splits
- * each FP32 operand into. 3 (the default): hi + mid + lo, six cross products
- * kept, every product more accurate than an FP32 multiply. 2: hi + lo, the
- * products hh + hl + lh, half the tensor-core work, each product to about
- * 2^-21 relative. The environment variable APHI_TC_SPLIT=2 sets the default. */
+/* FP32 factors: the form of the tensor-core trailing update. 3 (the default):
+ * each operand as three TF32 pieces, six cross products kept, every product
+ * more accurate than an FP32 multiply. 2: the faster form, each operand as
+ * four 8-bit digits relative to its row's largest component (2^-30 of it),
+ * summed exactly; with the environment variable APHI_TC_PRESPLIT set when the
+ * factor is made, two TF32 pieces instead (products hh + hl + lh, each to
+ * about 2^-21 relative). APHI_TC_SPLIT=2 sets the default. */
 int aphi_factor_set_tc_split(aphi_factor* f, int split);
 
 typedef struct {

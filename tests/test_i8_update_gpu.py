@@ -1,4 +1,4 @@
-"""The FP64 trailing update on INT8 digits (csrc/i8_update.cuh) at the edges of
+"""The trailing updates on INT8 digits (csrc/i8_update.cuh) at the edges of
 its tiles: rows and columns around multiples of 128, 64 and 32, K around
 multiples of 32, one panel and groups of two and four.
 
@@ -8,7 +8,10 @@ the pivots' magnitudes shared out as the kernel does (|a|, |b| <= A_i, B_j,
 the rows' largest components), an operand is off by at most 2^-62 A_i, so a
 sum of w complex products is off by at most 4 w 2^-62 A_i B_j, plus the
 dropped digit levels (below 2^-56 w A_i B_j) and at most three roundings of a
-sum below 2 w A_i B_j per group: together under 8 w 2^-53 A_i B_j."""
+sum below 2 w A_i B_j per group: together under 8 w 2^-53 A_i B_j. In FP32
+the operands' own products are rounded to 24 bits (8 w 2^-24 A_i B_j over a
+sum), a group's sum twice (4 w) and the destination once for each of up to
+five groups (10 w); digits and dropped levels add less than 2 w: 32 w 2^-24."""
 import numpy as np
 import pytest
 import torch
@@ -43,6 +46,8 @@ def factorize(shapes, panels, precision=ab.PREC_FP64):
     for o, p in zip(fr.panel_offset, panels):
         flat[o:o + p.size] = p.reshape(-1, order="F")
     f = ab.Factor(fr, precision, 1)
+    if precision == ab.PREC_FP32:
+        f.set_tc_split(2)
     ok = f.factorize_fronts(torch.from_numpy(flat).cuda().unsqueeze(0))
     P, C = (t.cpu().numpy() for t in f.read_fronts(0))
     got = []
@@ -52,12 +57,13 @@ def factorize(shapes, panels, precision=ab.PREC_FP64):
     return ok, got
 
 
-@pytest.mark.parametrize("spread", [0, 12])
-def test_trailing_update_at_the_tile_edges(spread, cuda):
+@pytest.mark.parametrize("precision,spread", [(ab.PREC_FP64, 0), (ab.PREC_FP64, 12), (ab.PREC_FP32, 0), (ab.PREC_FP32, 2)])
+def test_trailing_update_at_the_tile_edges(precision, spread, cuda):
     rng = np.random.default_rng(11 + spread)
     panels = panels_of(rng, SHAPES, spread)
-    ok, got = factorize(SHAPES, panels)
+    ok, got = factorize(SHAPES, panels, precision)
     assert ok
+    unit = 8.0 * 2.0 ** -53 if precision == ab.PREC_FP64 else 32.0 * 2.0 ** -24
     for (m, w), (L, C) in zip(SHAPES, got):
         d = np.diag(L[:w, :w])
         h = 2.0 ** np.floor(np.floor(np.log2(np.maximum(abs(d.real), abs(d.imag)))) / 2)
@@ -67,20 +73,21 @@ def test_trailing_update_at_the_tile_edges(spread, cuda):
         want = -(Lx * d.astype(np.clongdouble)) @ Lx.T
         low = np.tril(np.ones(C.shape, bool))
         err = np.abs((C.astype(np.clongdouble) - want)[low]).astype(np.float64)
-        tol = (8.0 * w * 2.0 ** -53 * np.outer(big(A), big(B)))[low]
+        tol = (unit * w * np.outer(big(A), big(B)))[low]
         assert (err <= tol).all(), (m, w, (err / tol).max())
 
 
-def test_a_row_that_is_not_finite_reaches_its_entries_only(cuda):
+@pytest.mark.parametrize("precision", [ab.PREC_FP64, ab.PREC_FP32])
+def test_a_row_that_is_not_finite_reaches_its_entries_only(precision, cuda):
     """A NaN below the pivots makes its row and column of the contribution
     block NaN, as a floating-point update does, and changes nothing else."""
     shapes = [(300, 130)]
     rng = np.random.default_rng(3)
     panels = panels_of(rng, shapes, 0)
-    _, clean = factorize(shapes, panels)
+    _, clean = factorize(shapes, panels, precision)
     bad = panels[0].copy()
     bad[200, 5] = np.nan
-    _, got = factorize(shapes, [bad])
+    _, got = factorize(shapes, [bad], precision)
     C, D = got[0][1], clean[0][1]
     low = np.tril(np.ones(C.shape, bool))
     hit = np.zeros_like(low)
