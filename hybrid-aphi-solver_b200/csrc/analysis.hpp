@@ -84,7 +84,7 @@ struct DeviceSchedule {
     int* ref_of_post = nullptr;
     int* fptr = nullptr;        // both triangles of A: row pointers,
     int* fcol = nullptr;        // columns,
-    long long* fmap = nullptr;  // and the index of each entry in the upper values
+    int* fmap = nullptr;        // and the index of each entry in the upper values
     Item* items = nullptr;
 };
 
@@ -100,7 +100,7 @@ struct aphi_analysis {
     std::vector<long long> h_uoff;
     std::vector<int> h_row_ptr, h_col_idx;
     std::vector<int> h_fptr, h_fcol;
-    std::vector<long long> h_fmap;
+    std::vector<int> h_fmap;
     bool on_device = false;
     void* device_arrays = nullptr;  // the one allocation behind d
     int device = -1;       // the CUDA device holding the device copy (set with it)

@@ -24,41 +24,65 @@ namespace aphi_b200 {
 
 namespace {
 
-constexpr int kEqThreads = 256;
+// Complex128 of the caller: two 8-byte halves, so that the arrays need a
+// double's alignment only.
+using cd = cx<double>;
+
+// The kernels that walk a sparse matrix's rows give each row to eight
+// neighbouring lanes: a row holds some 11 entries of the upper triangle, 22 of
+// both, so its values, columns and destinations are read in contiguous runs
+// and its gathers are in flight together, where one thread per row read 32
+// rows at once, an entry of each at a time.
+constexpr int kRowLanes = 8;
+constexpr int kRowThreads = 256;
+
+__device__ __forceinline__ int row_of_thread() {
+    return static_cast<int>((blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x) / kRowLanes);
+}
+// Sum over a row's lanes, the same in every lane and in a fixed order.
+__device__ __forceinline__ double row_sum(double v) {
+#pragma unroll
+    for (int o = kRowLanes / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+int row_blocks(int n) { return static_cast<int>((std::max(n, 1) * static_cast<long long>(kRowLanes) + kRowThreads - 1) / kRowThreads); }
 
 // ---------------------------------------------------------------- equilibration
 // |a_ij| d_i d_j contributes to the maxima of BOTH row i and row j
 // (src/equilibration.cpp:101-118): the matrix is stored as its upper
-// triangle. Maxima of non-negative doubles are taken as unsigned integers,
-// which orders them exactly, so the result does not depend on the order in
-// which threads arrive.
-__global__ void k_eq_rowmax(int n, const int* row_ptr, const int* col_idx, const double* values,
-                            long long nnz, const double* d, unsigned long long* rowmax) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
-    if (r >= n) return;
-    const double* v = values + 2LL * nnz * b;
-    const double* db = d + static_cast<long long>(n) * b;
-    unsigned long long* mx = rowmax + static_cast<long long>(n) * b;
-    const double dr = db[r];
-    double best = 0.0;
-    for (int k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
-        const int c = col_idx[k];
-        const double mag = hypot(v[2 * k], v[2 * k + 1]) * (dr * db[c]);
-        best = fmax(best, mag);
-        if (c != r) atomicMax(&mx[c], __double_as_longlong(mag));
-    }
-    atomicMax(&mx[r], __double_as_longlong(best));
+// triangle. Every step takes each row's maximum over both triangles (the
+// mirrored pattern) and scales d by it, from one vector into the other: no
+// atomics, one launch a step, and the magnitudes are computed once for all
+// steps. Maxima of non-negative doubles are taken as unsigned integers, which
+// orders them exactly. (6^3, one entry: 29 us a step with a thread per row,
+// atomic maxima and a hypot per entry and step; 3 us now.)
+__global__ void __launch_bounds__(256) k_eq_magnitudes(long long nnz, const cd* values, double* mag) {
+    const long long k = blockIdx.x * 256LL + threadIdx.x;
+    if (k >= nnz) return;
+    const cd v = values[nnz * blockIdx.y + k];
+    mag[nnz * blockIdx.y + k] = hypot(v.re, v.im);
 }
 
-__global__ void k_eq_update(int n, double* d, unsigned long long* rowmax) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
-    if (r >= n) return;
-    const long long at = static_cast<long long>(n) * b + r;
-    const double mx = __longlong_as_double(rowmax[at]);
-    if (mx > 0.0) d[at] *= 1.0 / sqrt(mx);
-    rowmax[at] = 0ULL;
+// d_out = d_in / sqrt(the rows' maxima); d_in null: all ones.
+__global__ void __launch_bounds__(kRowThreads) k_eq_step(int n, const int* fptr, const int* fcol, const int* fmap,
+                                                         const double* mag, long long nnz, const double* d_in,
+                                                         double* d_out) {
+    const int r = row_of_thread(), lane = threadIdx.x % kRowLanes;
+    const double* m = mag + nnz * blockIdx.y;
+    const double* d = d_in ? d_in + static_cast<long long>(n) * blockIdx.y : nullptr;
+    const double dr = d && r < n ? d[r] : 1.0;
+    unsigned long long best = 0;
+    if (r < n)
+        for (int k = fptr[r] + lane; k < fptr[r + 1]; k += kRowLanes) {
+            const int c = fcol[k];
+            const double v = m[fmap[k]] * (dr * (d ? d[c] : 1.0));
+            if (v == v || c < r) best = max(best, static_cast<unsigned long long>(__double_as_longlong(v)));
+        }
+#pragma unroll
+    for (int o = kRowLanes / 2; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (r >= n || lane != 0) return;
+    const double mx = __longlong_as_double(best);
+    d_out[static_cast<long long>(n) * blockIdx.y + r] = mx > 0.0 ? dr * (1.0 / sqrt(mx)) : dr;
 }
 
 __global__ void k_fill(double* p, long long n, double v) {
@@ -68,18 +92,19 @@ __global__ void k_fill(double* p, long long n, double v) {
 
 // Scaled A entries into their panel slots: L[dest[k]] = a_k d_r d_c.
 template <class R>
-__global__ void k_scatter_a(int n, const int* row_ptr, const int* col_idx, const double* values, long long nnz,
-                            const double* d, const long long* dest, cx<R>* Lb, long long lstride) {
-    const int r = blockIdx.x * blockDim.x + threadIdx.x;
-    const int b = blockIdx.y;
+__global__ void __launch_bounds__(kRowThreads) k_scatter_a(int n, const int* row_ptr, const int* col_idx,
+                                                           const cd* values, long long nnz, const double* d,
+                                                           const long long* dest, cx<R>* Lb, long long lstride) {
+    const int r = row_of_thread(), lane = threadIdx.x % kRowLanes;
     if (r >= n) return;
-    const double* v = values + 2LL * nnz * b;
-    const double* db = d + static_cast<long long>(n) * b;
-    cx<R>* L = Lb + lstride * b;
+    const cd* v = values + nnz * blockIdx.y;
+    const double* db = d + static_cast<long long>(n) * blockIdx.y;
+    cx<R>* L = Lb + lstride * blockIdx.y;
     const double dr = db[r];
-    for (int k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
+    for (int k = row_ptr[r] + lane; k < row_ptr[r + 1]; k += kRowLanes) {
         const double s = dr * db[col_idx[k]];
-        L[dest[k]] = cx<R>{static_cast<R>(v[2 * k] * s), static_cast<R>(v[2 * k + 1] * s)};
+        const cd a = v[k];
+        L[dest[k]] = cx<R>{static_cast<R>(a.re * s), static_cast<R>(a.im * s)};
     }
 }
 
@@ -159,57 +184,124 @@ __global__ void k_permute_out(int n, int nrhs, const int* new_of_orig, const dou
 }
 
 // ---------------------------------------------------------------- residuals
-// r = b - A x on the original upper-stored A (both triangles through the
-// mirrored CSR); per-row partial sums of |r|^2, |b|^2, |x|^2 reduced in a
-// fixed order by k_norms_final.
-__global__ void k_residual(int n, int nrhs, const int* fptr, const int* fcol, const long long* fmap,
-                           const double* values, long long nnz, const double* x, const double* b, double* r_out,
-                           double* partial) {
-    __shared__ double sh[3][256];
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int bk = blockIdx.y;
-    const int bb = bk / nrhs;
-    const double* v = values + 2LL * nnz * bb;
-    const double* xb = x + 2LL * n * bk;
-    const double* bb_ = b + 2LL * n * bk;
-    double rr = 0, b2 = 0, x2 = 0;
-    if (i < n) {
-        double ar = 0, ai = 0;
-        for (int k = fptr[i]; k < fptr[i + 1]; ++k) {
-            const long long q = fmap[k];
-            const double vr = v[2 * q], vi = v[2 * q + 1];
-            const double xr = xb[2 * fcol[k]], xi = xb[2 * fcol[k] + 1];
-            ar += vr * xr - vi * xi;
-            ai += vr * xi + vi * xr;
+// Row i of A x_k, k < K, on the original upper-stored A (both triangles
+// through the mirrored CSR), summed over the row's lanes; every lane of a warp
+// calls it. The x_k are n apart: one read of the row serves K right-hand sides.
+template <int K>
+__device__ __forceinline__ void row_times(bool live, int i, int lane, const int* fptr, const int* fcol,
+                                          const int* fmap, const cd* v, const cd* x, int n, cd (&out)[K]) {
+#pragma unroll
+    for (int q = 0; q < K; ++q) out[q] = cd{0, 0};
+    if (live)
+        for (int k = fptr[i] + lane; k < fptr[i + 1]; k += kRowLanes) {
+            const cd a = v[fmap[k]];
+            const int c = fcol[k];
+#pragma unroll
+            for (int q = 0; q < K; ++q) {
+                const cd y = x[static_cast<long long>(n) * q + c];
+                out[q].re += a.re * y.re - a.im * y.im;
+                out[q].im += a.re * y.im + a.im * y.re;
+            }
         }
-        const double er = bb_[2 * i] - ar, ei = bb_[2 * i + 1] - ai;
-        if (r_out) {
-            r_out[2LL * n * bk + 2 * i] = er;
-            r_out[2LL * n * bk + 2 * i + 1] = ei;
-        }
-        rr = er * er + ei * ei;
-        b2 = bb_[2 * i] * bb_[2 * i] + bb_[2 * i + 1] * bb_[2 * i + 1];
-        x2 = xb[2 * i] * xb[2 * i] + xb[2 * i + 1] * xb[2 * i + 1];
-    }
-    sh[0][threadIdx.x] = rr;
-    sh[1][threadIdx.x] = b2;
-    sh[2][threadIdx.x] = x2;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o)
-            for (int q = 0; q < 3; ++q) sh[q][threadIdx.x] += sh[q][threadIdx.x + o];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 3; ++q) partial[(static_cast<long long>(bk) * gridDim.x + blockIdx.x) * 3 + q] = sh[q][0];
+#pragma unroll
+    for (int q = 0; q < K; ++q) out[q] = cd{row_sum(out[q].re), row_sum(out[q].im)};
 }
 
-__global__ void k_amax(const double* values, long long nnz, unsigned long long* out) {
-    const long long k = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x;
-    const int b = blockIdx.y;
-    if (k >= nnz) return;
-    const double* v = values + 2LL * nnz * b;
-    atomicMax(&out[b], __double_as_longlong(hypot(v[2 * k], v[2 * k + 1])));
+// r = b - A x for K right-hand sides of one entry (grid.y: entries x nrhs / K);
+// per-block partial sums of |r|^2, |b|^2, |x|^2 (256 rows a block) reduced in a
+// fixed order by k_norms_final. (Four 24^3 systems, two right-hand sides each:
+// 260 us with a thread per row and right-hand side, 110 us now.)
+constexpr int kResidualRows = 256, kResidualThreads = 512;
+template <int K>
+__global__ void __launch_bounds__(kResidualThreads) k_residual(int n, int nrhs, const int* fptr, const int* fcol,
+                                                               const int* fmap, const double* values, long long nnz,
+                                                               const double* x, const double* b, double* r_out,
+                                                               double* partial) {
+    constexpr int kWarps = kResidualThreads / 32;
+    __shared__ double sh[3 * K][kWarps];
+    const int bk = blockIdx.y * K, lane = threadIdx.x % kRowLanes;
+    const cd* v = reinterpret_cast<const cd*>(values) + nnz * (bk / nrhs);
+    const cd* xb = reinterpret_cast<const cd*>(x) + static_cast<long long>(n) * bk;
+    const cd* bb = reinterpret_cast<const cd*>(b) + static_cast<long long>(n) * bk;
+    cd* rb = r_out ? reinterpret_cast<cd*>(r_out) + static_cast<long long>(n) * bk : nullptr;
+    double s[3 * K] = {};
+    for (int h = 0; h < kResidualRows * kRowLanes / kResidualThreads; ++h) {
+        const int i = blockIdx.x * kResidualRows + h * (kResidualThreads / kRowLanes) + threadIdx.x / kRowLanes;
+        cd ax[K];
+        row_times<K>(i < n, i, lane, fptr, fcol, fmap, v, xb, n, ax);
+        if (i < n && lane == 0)
+#pragma unroll
+            for (int q = 0; q < K; ++q) {
+                const long long at = static_cast<long long>(n) * q + i;
+                const cd bi = bb[at], xi = xb[at], e = bi - ax[q];
+                if (rb) rb[at] = e;
+                s[3 * q] += e.re * e.re + e.im * e.im;
+                s[3 * q + 1] += bi.re * bi.re + bi.im * bi.im;
+                s[3 * q + 2] += xi.re * xi.re + xi.im * xi.im;
+            }
+    }
+#pragma unroll
+    for (int q = 0; q < 3 * K; ++q) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
+        if (threadIdx.x % 32 == 0) sh[q][threadIdx.x / 32] = s[q];
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 * K) {
+        double t = 0;
+        for (int w = 0; w < kWarps; ++w) t += sh[threadIdx.x][w];
+        partial[(static_cast<long long>(bk + threadIdx.x / 3) * gridDim.x + blockIdx.x) * 3 + threadIdx.x % 3] = t;
+    }
+}
+
+// The residual of `systems` (a multiple of nrhs) with as many right-hand sides
+// per CTA as divide nrhs (4, 2 or 1); the bits do not depend on it.
+void launch_residual(int n, int systems, int nrhs, const int* fptr, const int* fcol, const int* fmap,
+                     const double* values, long long nnz, const double* x, const double* b, double* r_out,
+                     double* partial, cudaStream_t st) {
+    const unsigned nb = ceil_div(std::max(n, 1), kResidualRows);
+    auto go = [&](auto kern, int k) {
+        kern<<<dim3(nb, systems / k), kResidualThreads, 0, st>>>(n, nrhs, fptr, fcol, fmap, values, nnz, x, b, r_out,
+                                                                 partial);
+    };
+    if (nrhs % 4 == 0)
+        go(k_residual<4>, 4);
+    else if (nrhs % 2 == 0)
+        go(k_residual<2>, 2);
+    else
+        go(k_residual<1>, 1);
+    APHI_CHECK_LAUNCH();
+}
+
+// max |a_k| per entry of the batch: a block's own maximum first, one atomic
+// per block. (One atomic per entry, all of a system's on one word, took 2.75 ms
+// for four 24^3 systems, ten times the residual itself; 67 MB are read.)
+constexpr int kAmaxPerThread = 8;
+__global__ void __launch_bounds__(256) k_amax(const double* values, long long nnz, unsigned long long* out) {
+    __shared__ unsigned long long sh[8];
+    const cd* v = reinterpret_cast<const cd*>(values) + nnz * blockIdx.y;
+    const long long k0 = blockIdx.x * (256LL * kAmaxPerThread) + threadIdx.x;
+    unsigned long long best = 0;
+#pragma unroll
+    for (int u = 0; u < kAmaxPerThread; ++u) {
+        const long long k = k0 + 256 * u;
+        if (k < nnz) {
+            const cd a = v[k];
+            best = max(best, static_cast<unsigned long long>(__double_as_longlong(hypot(a.re, a.im))));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    if (threadIdx.x % 32 == 0) sh[threadIdx.x / 32] = best;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) best = max(best, sh[w]);
+        atomicMax(&out[blockIdx.y], best);
+    }
+}
+dim3 amax_grid(long long nnz, int batch) {
+    return dim3(static_cast<unsigned>((std::max<long long>(nnz, 1) + 256 * kAmaxPerThread - 1) / (256 * kAmaxPerThread)),
+                batch);
 }
 
 // norms[bk] = {||r||, ||b||, ||x||, max|A|}: fixed-order sums of the partials.
@@ -480,7 +572,6 @@ template <class R>
 void factorize_numeric(aphi_factor* f, const double* values, const double* panels, cudaStream_t st) {
     const aphi_analysis* A = f->an;
     const int n = A->S.n;
-    const dim3 g(ceil_div(std::max(n, 1), 256), f->batch);
     set_smem_limits<R>(A->opt.small_front);
     if (panels) {
         const long long len = A->S.stored * f->batch;
@@ -489,8 +580,9 @@ void factorize_numeric(aphi_factor* f, const double* values, const double* panel
         APHI_CHECK_LAUNCH();
     } else {
         APHI_CUDA(cudaMemsetAsync(f->L, 0, static_cast<size_t>(A->S.stored) * f->batch * f->elem, st));
-        k_scatter_a<R><<<g, 256, 0, st>>>(n, A->d.row_ptr, A->d.col_idx, values, A->S.nnz_a, f->dscale,
-                                          A->d.a_dest, reinterpret_cast<cx<R>*>(f->L), A->S.stored);
+        k_scatter_a<R><<<dim3(row_blocks(n), f->batch), kRowThreads, 0, st>>>(
+            n, A->d.row_ptr, A->d.col_idx, reinterpret_cast<const cd*>(values), A->S.nnz_a, f->dscale,
+            A->d.a_dest, reinterpret_cast<cx<R>*>(f->L), A->S.stored);
         APHI_CHECK_LAUNCH();
     }
     const bool tc = sizeof(R) == 4 && f->use_tc;
@@ -584,7 +676,6 @@ aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
         auto want = [&](auto** p, size_t bytes) { parts.push_back({reinterpret_cast<void**>(p), bytes}); };
         want(&f->L, static_cast<size_t>(S.stored) * batch * f->elem);
         want(&f->dscale, nb * sizeof(double));
-        want(&f->rowmax, nb * sizeof(unsigned long long));
         want(&f->stats, 4 * sizeof(unsigned long long) * batch);
         want(&f->dref, 2 * nb * sizeof(double));
         want(&f->kmax, sizeof(int) * batch);
@@ -662,17 +753,25 @@ int factorize(aphi_factor* f, const double* values, int equil_iters, double pivo
     APHI_CUDA(cudaEventCreate(&e1));
     APHI_CUDA(cudaEventRecord(e0, st));
 
-    // Equilibration (FP64 on the original values).
+    // Equilibration (FP64 on the original values): the steps alternate between
+    // dscale and dref (free until the pivots are extracted), ending in dscale;
+    // the magnitudes sit in the panels' memory, which the scatter clears later.
     const long long nd = static_cast<long long>(n) * B;
-    k_fill<<<ceil_div(std::max<long long>(nd, 1), 256), 256, 0, st>>>(f->dscale, nd, 1.0);
-    APHI_CHECK_LAUNCH();
-    APHI_CUDA(cudaMemsetAsync(f->rowmax, 0, sizeof(unsigned long long) * std::max<long long>(nd, 1), st));
-    const dim3 g(ceil_div(std::max(n, 1), kEqThreads), B);
-    for (int it = 0; it < equil_iters; ++it) {
-        k_eq_rowmax<<<g, kEqThreads, 0, st>>>(n, A->d.row_ptr, A->d.col_idx, values, S.nnz_a, f->dscale, f->rowmax);
+    if (equil_iters == 0) {
+        k_fill<<<ceil_div(std::max<long long>(nd, 1), 256), 256, 0, st>>>(f->dscale, nd, 1.0);
         APHI_CHECK_LAUNCH();
-        k_eq_update<<<g, kEqThreads, 0, st>>>(n, f->dscale, f->rowmax);
+    } else {
+        double* mag = static_cast<double*>(f->L);
+        k_eq_magnitudes<<<dim3(ceil_div(std::max<long long>(S.nnz_a, 1), 256), B), 256, 0, st>>>(
+            S.nnz_a, reinterpret_cast<const cd*>(values), mag);
         APHI_CHECK_LAUNCH();
+        for (int it = 0; it < equil_iters; ++it) {
+            double* to = (equil_iters - it) % 2 ? f->dscale : f->dref;
+            double* from = it == 0 ? nullptr : (to == f->dscale ? f->dref : f->dscale);
+            k_eq_step<<<dim3(row_blocks(n), B), kRowThreads, 0, st>>>(n, A->d.fptr, A->d.fcol, A->d.fmap, mag, S.nnz_a,
+                                                                      from, to);
+            APHI_CHECK_LAUNCH();
+        }
     }
     // The contribution-block pool is only live during a factorization, so it
     // is a workspace owned by the analysis and shared by every factor of the
@@ -817,10 +916,8 @@ void residuals(const aphi_analysis* an, int batch, int nrhs, const double* value
     unsigned long long* amax = reinterpret_cast<unsigned long long*>(partial + np);
     double* norms = partial + np + batch;
     APHI_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * batch, st));
-    k_residual<<<dim3(nb, batch * nrhs), 256, 0, st>>>(n, nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values,
-                                                       an->S.nnz_a, x, b, nullptr, partial);
-    APHI_CHECK_LAUNCH();
-    k_amax<<<dim3(ceil_div(std::max<long long>(an->S.nnz_a, 1), 256), batch), 256, 0, st>>>(values, an->S.nnz_a, amax);
+    launch_residual(n, batch * nrhs, nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values, an->S.nnz_a, x, b, nullptr, partial, st);
+    k_amax<<<amax_grid(an->S.nnz_a, batch), 256, 0, st>>>(values, an->S.nnz_a, amax);
     APHI_CHECK_LAUNCH();
     k_norms_final<<<batch * nrhs, 256, 0, st>>>(nb, nrhs, partial, amax, norms);
     APHI_CHECK_LAUNCH();
@@ -846,7 +943,7 @@ void csr_residuals_host(int n, const int* row_ptr, const int* col_idx, const dou
         throw Error(APHI_ERR_BAD_SHAPE, "relative_residual: n must be >= 1 and nrhs in 1..65535");
     const long long nnz = row_ptr[n];
     std::vector<int> fptr(static_cast<size_t>(n) + 1, 0), fcol;
-    std::vector<long long> fmap;
+    std::vector<int> fmap;
     for (int r = 0; r < n; ++r)
         for (long long k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
             const int c = col_idx[k];
@@ -863,10 +960,10 @@ void csr_residuals_host(int n, const int* row_ptr, const int* col_idx, const dou
             for (long long k = row_ptr[r]; k < row_ptr[r + 1]; ++k) {
                 const int c = col_idx[k];
                 fcol[cur[r]] = c;
-                fmap[cur[r]++] = k;
+                fmap[cur[r]++] = static_cast<int>(k);
                 if (c != r) {
                     fcol[cur[c]] = r;
-                    fmap[cur[c]++] = k;
+                    fmap[cur[c]++] = static_cast<int>(k);
                 }
             }
     }
@@ -882,7 +979,7 @@ void csr_residuals_host(int n, const int* row_ptr, const int* col_idx, const dou
     try {
         const int* d_fptr = static_cast<const int*>(up(fptr.data(), fptr.size() * sizeof(int)));
         const int* d_fcol = static_cast<const int*>(up(fcol.data(), fcol.size() * sizeof(int)));
-        const long long* d_fmap = static_cast<const long long*>(up(fmap.data(), fmap.size() * sizeof(long long)));
+        const int* d_fmap = static_cast<const int*>(up(fmap.data(), fmap.size() * sizeof(int)));
         const double* d_v = static_cast<const double*>(up(values, 16 * static_cast<size_t>(nnz)));
         const double* d_x = static_cast<const double*>(up(x, 16 * static_cast<size_t>(n) * nrhs));
         const double* d_b = static_cast<const double*>(up(b, 16 * static_cast<size_t>(n) * nrhs));
@@ -890,9 +987,8 @@ void csr_residuals_host(int n, const int* row_ptr, const int* col_idx, const dou
         auto* amax = static_cast<unsigned long long*>(up(nullptr, sizeof(unsigned long long)));
         double* norms = static_cast<double*>(up(nullptr, sizeof(double) * 4 * static_cast<size_t>(nrhs)));
         APHI_CUDA(cudaMemset(amax, 0, sizeof(unsigned long long)));
-        k_residual<<<dim3(nb, nrhs), 256>>>(n, nrhs, d_fptr, d_fcol, d_fmap, d_v, nnz, d_x, d_b, nullptr, partial);
-        APHI_CHECK_LAUNCH();
-        k_amax<<<dim3(ceil_div(std::max<long long>(nnz, 1), 256), 1), 256>>>(d_v, nnz, amax);
+        launch_residual(n, nrhs, nrhs, d_fptr, d_fcol, d_fmap, d_v, nnz, d_x, d_b, nullptr, partial, nullptr);
+        k_amax<<<amax_grid(nnz, 1), 256>>>(d_v, nnz, amax);
         APHI_CHECK_LAUNCH();
         k_norms_final<<<nrhs, 256>>>(nb, nrhs, partial, amax, norms);
         APHI_CHECK_LAUNCH();
@@ -994,10 +1090,8 @@ void residuals_noalloc(const aphi_analysis* an, int batch, int nrhs, const doubl
     double* norms = scratch + nb * 3 * q + batch;
     double* ratios = norms + 4 * q;
     APHI_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * batch, st));
-    k_residual<<<dim3(static_cast<unsigned>(nb), static_cast<unsigned>(q)), 256, 0, st>>>(
-        n, nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values, an->S.nnz_a, x, b, nullptr, partial);
-    APHI_CHECK_LAUNCH();
-    k_amax<<<dim3(ceil_div(std::max<long long>(an->S.nnz_a, 1), 256), batch), 256, 0, st>>>(values, an->S.nnz_a, amax);
+    launch_residual(n, static_cast<int>(q), nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values, an->S.nnz_a, x, b, nullptr, partial, st);
+    k_amax<<<amax_grid(an->S.nnz_a, batch), 256, 0, st>>>(values, an->S.nnz_a, amax);
     APHI_CHECK_LAUNCH();
     k_norms_final<<<static_cast<unsigned>(q), 256, 0, st>>>(static_cast<int>(nb), nrhs, partial, amax, norms);
     APHI_CHECK_LAUNCH();
@@ -1036,7 +1130,7 @@ int solve_refined(aphi_factor* f, int nrhs, const double* values, const double* 
     unsigned long long* amax = reinterpret_cast<unsigned long long*>(f->red + static_cast<size_t>(nb) * 3 * B * nrhs);
     solve(f, nrhs, b, x, st);
     APHI_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * B, st));
-    k_amax<<<dim3(ceil_div(std::max<long long>(A->S.nnz_a, 1), 256), B), 256, 0, st>>>(values, A->S.nnz_a, amax);
+    k_amax<<<amax_grid(A->S.nnz_a, B), 256, 0, st>>>(values, A->S.nnz_a, amax);
     APHI_CHECK_LAUNCH();
     const int q = B * nrhs;
     std::vector<double> prev(q, INFINITY), h(4 * static_cast<size_t>(q));
@@ -1044,9 +1138,7 @@ int solve_refined(aphi_factor* f, int nrhs, const double* values, const double* 
     std::vector<char> done(q, 0);
     int status = APHI_OK;
     for (int step = 0;; ++step) {
-        k_residual<<<dim3(nb, q), 256, 0, st>>>(n, nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, x, b,
-                                                r, f->red);
-        APHI_CHECK_LAUNCH();
+        launch_residual(n, static_cast<int>(q), nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, x, b, r, f->red, st);
         k_norms_final<<<q, 256, 0, st>>>(nb, nrhs, f->red, amax, f->norms);
         APHI_CHECK_LAUNCH();
         APHI_CUDA(cudaMemcpyAsync(h.data(), f->norms, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1101,23 +1193,15 @@ constexpr int kCocgPatience = 5;
 // as they converge.
 
 // y = A x for q systems.
-__global__ void k_spmv(int n, int nrhs, const int* fptr, const int* fcol, const long long* fmap,
-                       const double* values, long long nnz, const double* x, double* y) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int k = blockIdx.y;
-    if (i >= n) return;
-    const double* v = values + 2LL * nnz * (k / nrhs);
-    const double* xk = x + 2LL * n * k;
-    double ar = 0, ai = 0;
-    for (int t = fptr[i]; t < fptr[i + 1]; ++t) {
-        const long long q = fmap[t];
-        const double vr = v[2 * q], vi = v[2 * q + 1];
-        const double xr = xk[2 * fcol[t]], xi = xk[2 * fcol[t] + 1];
-        ar += vr * xr - vi * xi;
-        ai += vr * xi + vi * xr;
-    }
-    y[2LL * n * k + 2 * i] = ar;
-    y[2LL * n * k + 2 * i + 1] = ai;
+__global__ void __launch_bounds__(kRowThreads) k_spmv(int n, int nrhs, const int* fptr, const int* fcol,
+                                                      const int* fmap, const double* values, long long nnz,
+                                                      const double* x, double* y) {
+    const int i = row_of_thread(), k = blockIdx.y, lane = threadIdx.x % kRowLanes;
+    const long long at = static_cast<long long>(n) * k;
+    cd s[1];
+    row_times<1>(i < n, i, lane, fptr, fcol, fmap, reinterpret_cast<const cd*>(values) + nnz * (k / nrhs),
+                 reinterpret_cast<const cd*>(x) + at, n, s);
+    if (i < n && lane == 0) reinterpret_cast<cd*>(y)[at + i] = s[0];
 }
 
 // partial[k][blk] = sum over the block's entries of a_i b_i (unconjugated).
@@ -1261,7 +1345,7 @@ int solve_krylov(aphi_factor* f, int nrhs, const double* values, const double* b
     const dim3 gv(nb, q);
 
     APHI_CUDA(cudaMemsetAsync(amax, 0, sizeof(unsigned long long) * B, st));
-    k_amax<<<dim3(ceil_div(std::max<long long>(A->S.nnz_a, 1), 256), B), 256, 0, st>>>(values, A->S.nnz_a, amax);
+    k_amax<<<amax_grid(A->S.nnz_a, B), 256, 0, st>>>(values, A->S.nnz_a, amax);
     APHI_CHECK_LAUNCH();
     std::vector<int> act(q, 1), it(q, 0), since(q, 0), ent;
     std::vector<int> restarted(q, 0), restart_now(q, 0);
@@ -1269,9 +1353,7 @@ int solve_krylov(aphi_factor* f, int nrhs, const double* values, const double* b
     APHI_CUDA(cudaMemcpyAsync(active, act.data(), sizeof(int) * q, cudaMemcpyHostToDevice, st));
 
     auto residual = [&]() {  // r = b - A x; norms to the host
-        k_residual<<<gv, 256, 0, st>>>(n, nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, x, b, r,
-                                       partial);
-        APHI_CHECK_LAUNCH();
+        launch_residual(n, static_cast<int>(q), nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, x, b, r, partial, st);
         k_norms_final<<<q, 256, 0, st>>>(nb, nrhs, partial, amax, norms);
         APHI_CHECK_LAUNCH();
         APHI_CUDA(cudaMemcpyAsync(h.data(), norms, h.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
@@ -1356,7 +1438,7 @@ int solve_krylov(aphi_factor* f, int nrhs, const double* values, const double* b
             k_xpby_sys<<<gv, 256, 0, st>>>(n, active, beta, z, p);
             APHI_CHECK_LAUNCH();
         }
-        k_spmv<<<gv, 256, 0, st>>>(n, nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, p, Ap);
+        k_spmv<<<dim3(row_blocks(n), q), kRowThreads, 0, st>>>(n, nrhs, A->d.fptr, A->d.fcol, A->d.fmap, values, A->S.nnz_a, p, Ap);
         APHI_CHECK_LAUNCH();
         dot(p, Ap, 1);
         k_axpy_sys<<<gv, 256, 0, st>>>(n, alpha, p, x);
@@ -1374,7 +1456,7 @@ void spmv(const aphi_analysis* an, int batch, int nrhs, const double* values, co
         throw Error(APHI_ERR_BAD_SHAPE, "spmv: batch x nrhs exceeds the 65535 systems one call handles");
     const int n = an->S.n;
     if (n == 0) return;
-    k_spmv<<<dim3(ceil_div(n, 256), batch * nrhs), 256, 0, st>>>(n, nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values,
+    k_spmv<<<dim3(row_blocks(n), batch * nrhs), kRowThreads, 0, st>>>(n, nrhs, an->d.fptr, an->d.fcol, an->d.fmap, values,
                                                                an->S.nnz_a, x, y);
     APHI_CHECK_LAUNCH();
 }

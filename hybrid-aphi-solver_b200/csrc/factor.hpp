@@ -19,9 +19,8 @@ struct aphi_factor {
     void* L = nullptr;         // batch x stored
     void* CB = nullptr;        // batch x cb_pool: the analysis's workspace, set at factorize
     double* dscale = nullptr;  // batch x n, original numbering
-    unsigned long long* rowmax = nullptr;  // batch x n (equilibration scratch)
     unsigned long long* stats = nullptr;   // batch x 4 (max|L| bits, ...)
-    double* dref = nullptr;    // batch x n complex128: D in the reference's permuted order
+    double* dref = nullptr;    // batch x n complex128: D in the reference's permuted order (before that, equilibration scratch)
     // Solve scratch, grown on demand: y (batch x nrhs x n), U (batch x nrhs x upool).
     void* solve_arena = nullptr;  // the one allocation behind y, U and part
     void* y = nullptr;
