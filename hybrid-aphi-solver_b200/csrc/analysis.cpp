@@ -233,7 +233,7 @@ void build_plans(aphi_analysis& A, std::vector<Item>& items) {
     // first: partial sums over row chunks, then the triangle.
     //
     // Two forms of each. The split plans give every triangle a launch of its
-    // own. The fused plans (wide = 1, the ones the solves run) fold each
+    // own and are the ones that run. The fused plans (wide = 1) fold each
     // triangle into the launch before it: the gather's CTA solves its
     // supernode's first block; of the CTAs updating the rows below block blk
     // (forward), the last to finish (a per-supernode arrival counter) solves
@@ -254,12 +254,14 @@ void build_plans(aphi_analysis& A, std::vector<Item>& items) {
             const int* lb = S.level_list.data() + S.level_ptr[L];
             const int* le = S.level_list.data() + S.level_ptr[L + 1];
             long long f0 = static_cast<long long>(items.size());
-            int maxb = 0;
+            int maxb = 0, span = 1;
             for (const int* p = lb; p < le; ++p) {
                 items.push_back({*p, 0, 0, 0});
                 maxb = std::max(maxb, nblocks(*p));
+                span = std::max(span, S.sn_rows[*p]);
             }
             pushw(fwd, K_FWD_GATHER, f0, fused);
+            if (!fwd.empty()) fwd.back().span = span;
             for (int blk = 0; blk < maxb; ++blk) {
                 if (!fused) {
                     f0 = static_cast<long long>(items.size());

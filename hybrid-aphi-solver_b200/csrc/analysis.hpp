@@ -40,6 +40,7 @@ struct Launch {
     int kcap = kTcPanel;  // trailing updates: panel columns applied at once (K = min(kcap, w - p0))
     int wide = 0;         // K_UPDATE_PANEL: 128 x 64 tiles on the trailing-update kernels (column cap at the panel's end);
                           // K_FWD_GATHER / K_FWD_UPDATE / K_BWD_UPDATE: fused with the triangle solve (see build_plans)
+    int span = 0;         // K_FWD_GATHER: rows of the launch's tallest front
 };
 
 struct Item {

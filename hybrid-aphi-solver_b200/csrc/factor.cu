@@ -210,7 +210,7 @@ __device__ __forceinline__ void row_times(bool live, int i, int lane, const int*
 // r = b - A x for K right-hand sides of one entry (grid.y: entries x nrhs / K);
 // per-block partial sums of |r|^2, |b|^2, |x|^2 (256 rows a block) reduced in a
 // fixed order by k_norms_final. (Four 24^3 systems, two right-hand sides each:
-// 260 us with a thread per row and right-hand side, 110 us now.)
+// 260 us with a thread per row and right-hand side, 141 us now.)
 constexpr int kResidualRows = 256, kResidualThreads = 512;
 template <int K>
 __global__ void __launch_bounds__(kResidualThreads) k_residual(int n, int nrhs, const int* fptr, const int* fcol,
@@ -353,6 +353,22 @@ void device_parts(void** base, const std::vector<std::pair<void**, size_t>>& par
     }
 }
 
+// A launch that may start before the one before it has finished (pdl_wait).
+template <class... Params, class... Args>
+void chained(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    APHI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+}
+
 template <class R>
 void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_t st, const SolveArgs* sa,
               cx<R>* y, cx<R>* U, cx<R>* part) {
@@ -374,7 +390,7 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
             sizeof(R) == 8 ? f->dws_stride : f->tcws_stride, f->err);
     };
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
-    const size_t bwd_smem = (kTriSmem + kRedSmem) * sizeof(cx<R>);  // backward triangles
+    const size_t bwd_smem = (kTriSmem + (sa ? red_smem(sa->nr) : 0)) * sizeof(cx<R>);  // backward triangles
     // FP64 trailing updates on INT8 digits, prepared once per panel group.
     const bool prescaled = sizeof(R) == 8 && f->dws;
     for (const Launch& l : plan) {
@@ -463,26 +479,30 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                 } else
                     throw Error(APHI_ERR_INVALID, "tensor-core update planned for an FP64 factor");
                 break;
-            case K_FWD_GATHER:
+            case K_FWD_GATHER: {
+                const dim3 g(grid.x, grid.y, (l.span + kGatherRows - 1) / kGatherRows);
                 if (l.wide)
-                    k_fwd_gather<R, true><<<grid, 256, tri_smem, st>>>(S, l.first, *sa, L, ls, y, U);
+                    chained(k_fwd_gather<R, true>, g, 256, tri_smem, st, S, l.first, *sa, L, ls, y, U);
                 else
-                    k_fwd_gather<R, false><<<grid, 256, 0, st>>>(S, l.first, *sa, L, ls, y, U);
+                    chained(k_fwd_gather<R, false>, g, 256, 0, st, S, l.first, *sa, L, ls, y, U);
                 break;
-            case K_FWD_DIAG: k_fwd_diag<R><<<grid, 256, tri_smem, st>>>(S, l.first, *sa, L, ls, y); break;
+            }
+            case K_FWD_DIAG: chained(k_fwd_diag<R>, grid, 256, tri_smem, st, S, l.first, *sa, L, ls, y); break;
             case K_FWD_UPDATE:
                 if (l.wide)
-                    k_fwd_update<R, true><<<grid, 256, tri_smem, st>>>(S, l.first, *sa, L, ls, y, U);
+                    chained(k_fwd_update<R, true>, grid, 256, tri_smem, st, S, l.first, *sa, L, ls, y, U);
                 else
-                    k_fwd_update<R, false><<<grid, 256, 0, st>>>(S, l.first, *sa, L, ls, y, U);
+                    chained(k_fwd_update<R, false>, grid, 256, 0, st, S, l.first, *sa, L, ls, y, U);
                 break;
             case K_BWD_UPDATE:
                 if (l.wide)
-                    k_bwd_update<R, true><<<grid, 256, bwd_smem, st>>>(S, l.first, *sa, L, ls, y, part);
+                    chained(k_bwd_update<R, true>, grid, 256, bwd_smem, st, S, l.first, *sa, L, ls, y, part);
                 else
-                    k_bwd_update<R, false><<<grid, 256, 0, st>>>(S, l.first, *sa, L, ls, y, part);
+                    chained(k_bwd_update<R, false>, grid, 256, tri_smem, st, S, l.first, *sa, L, ls, y, part);
                 break;
-            case K_BWD_DIAG: k_bwd_diag<R><<<grid, 256, bwd_smem, st>>>(S, l.first, *sa, L, ls, y, part); break;
+            case K_BWD_DIAG:
+                chained(k_bwd_diag<R>, grid, kBwdDiagThreads, bwd_smem, st, S, l.first, *sa, L, ls, y, part);
+                break;
         }
         APHI_CHECK_LAUNCH();
         if (timed) APHI_CUDA(cudaEventRecord(fm->prof_events.back(), st));
@@ -541,12 +561,13 @@ void set_smem_limits(int small_front) {
         APHI_CUDA(cudaFuncSetAttribute(k_update_tc_presplit<4, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        TcPreSmem<4>::bytes));
     }
-    const int tri = kTriSmem * static_cast<int>(sizeof(cx<R>)), bwd = (kTriSmem + kRedSmem) * static_cast<int>(sizeof(cx<R>));
+    const int tri = kTriSmem * static_cast<int>(sizeof(cx<R>)), bwd = (kTriSmem + red_smem(8)) * static_cast<int>(sizeof(cx<R>));
     APHI_CUDA(cudaFuncSetAttribute(k_fwd_diag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
     APHI_CUDA(cudaFuncSetAttribute(k_fwd_gather<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
     APHI_CUDA(cudaFuncSetAttribute(k_fwd_update<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
     APHI_CUDA(cudaFuncSetAttribute(k_bwd_diag<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd));
     APHI_CUDA(cudaFuncSetAttribute(k_bwd_update<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bwd));
+    APHI_CUDA(cudaFuncSetAttribute(k_bwd_update<R, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tri));
     (void)small_front;
     done = true;
 }
@@ -615,13 +636,12 @@ void solve_numeric(aphi_factor* f, int nrhs, const double* b, double* x, cudaStr
     const dim3 g(ceil_div(std::max(n, 1), 256), f->batch * nrhs);
     k_permute_in<R><<<g, 256, 0, st>>>(n, nrhs, A->d.orig_of_new, f->dscale, b, y);
     APHI_CHECK_LAUNCH();
-    // The fused plans (half the launches, each triangle in the launch before
-    // it) win while one entry is solved; with more, every CTA's reservation of
-    // a triangle's shared memory costs occupancy and the split plans are
-    // faster (32^3, FP32: 15.4 against 15.9 ms for one entry, 30.4 against
-    // 25.4 ms for six).
-    const int rows = entries ? nentries : f->batch;
-    const bool split = f->solve_form == 1 || (f->solve_form < 0 && rows > 1);
+    // The split plans (a launch per triangle): with launches that overlap their
+    // neighbours' ends, twice as many cost less than the fused plans' hand-over
+    // to a block's last CTA (32^3, FP32, one entry: 7.0 against 9.0 ms; six
+    // entries: 15.9 against 18.6; 24^3, FP64, eight right-hand sides: 10.2
+    // against 10.9; 8^3: equal).
+    const bool split = f->solve_form != 0;
     for (int k0 = 0; k0 < nrhs; k0 += 8) {
         const SolveArgs sa{n,       nrhs, k0, std::min(8, nrhs - k0), A->upool, A->max_parts, entries,
                            entries ? nentries : 0, f->counters, A->S.ns};

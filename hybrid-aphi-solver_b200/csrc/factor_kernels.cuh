@@ -1236,16 +1236,30 @@ __device__ __forceinline__ int solve_nblocks(const Sched& S, int s) {
     return (S.first[s + 1] - S.first[s] + kSolveBlock - 1) / kSolveBlock;
 }
 
-// Shared memory of the solve kernels that hold a triangle: L_bb with leading
-// dimension kTriLd (65: a lane's column-strided reads of the backward solve
-// fall in distinct banks), and for the backward solve the partial-sum
-// reduction's four sub-sums per (column, rhs).
+// A solve is a chain of short launches, each of which needs the one before it
+// for a few vectors only: its items, schedule and panel entries are constants.
+// So the solve kernels are launched with programmatic stream serialization: a
+// kernel lets the next one start as it begins itself (pdl_start_next), which
+// then reads its constants and waits (pdl_wait) until the kernel before it has
+// finished and its writes are visible. Everything that a launch before could
+// have written, or still reads where this one writes, comes after pdl_wait();
+// every solve kernel calls it, so that the wait covers all launches before.
+__device__ __forceinline__ void pdl_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Shared memory of the solve kernels that hold a 64 x 64 block of L, with
+// leading dimension kTriLd (65: column-strided reads fall in distinct banks),
+// and for the backward triangle the partial-sum reduction's kRedGroups
+// sub-sums per (column, rhs).
 constexpr int kTriLd = kSolveBlock + 1;
 constexpr int kTriSmem = kSolveBlock * kTriLd;     // complex entries
-constexpr int kRedSmem = 4 * kSolveBlock * 8;      // complex entries
+constexpr int kRedGroups = 8;
+constexpr int kBwdDiagThreads = 512;
+constexpr int red_smem(int nr) { return kRedGroups * kSolveBlock * nr; }  // complex entries
+constexpr int kGatherRows = 512;                   // front rows per gather CTA
 
-// L_bb (jb x jb, leading dimension m in the panel) into shared memory T
-// (leading dimension kTriLd, zeros outside the jb x jb block) by
+// A block of L (rows x cols at P, leading dimension m) into shared memory T
+// (leading dimension kTriLd, zeros outside the rows x cols block) by
 // asynchronous copies (cp.async, zero-filled where the source size is 0), so
 // the caller's own loads overlap them; the caller waits with
 // triangle_wait() and a __syncthreads() before reading T.
@@ -1256,12 +1270,11 @@ __device__ __forceinline__ void cp_async_entry(uint32_t dst, const cx<float>* sr
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8u : 0u) : "memory");
 }
 template <class R>
-__device__ __forceinline__ void stage_triangle(cx<R>* T, const cx<R>* P, long long m, int jb) {
-    static_assert(kSolveBlock * kSolveBlock % 256 == 0, "the block splits evenly over 256 threads");
+__device__ __forceinline__ void stage_block(cx<R>* T, const cx<R>* P, long long m, int rows, int cols) {
 #pragma unroll 4
-    for (int e = threadIdx.x; e < kSolveBlock * kSolveBlock; e += 256) {
+    for (int e = threadIdx.x; e < kSolveBlock * kSolveBlock; e += blockDim.x) {
         const int i = e % kSolveBlock, j = e / kSolveBlock;
-        const bool in = i < jb && j < jb;
+        const bool in = i < rows && j < cols;
         cp_async_entry(smem_u32(T + i + j * kTriLd), in ? P + i + static_cast<long long>(j) * m : P, in);
     }
     cp_async_commit();
@@ -1270,21 +1283,26 @@ __device__ __forceinline__ void triangle_wait() { cp_async_wait<0>(); }
 
 // Forward triangle of block blk of supernode s: y[blk] = L_bb^-1 y[blk] for
 // the pass's rhs, one warp per rhs, L_bb staged in shared memory (smem:
-// kTriSmem entries). Lane l holds rows l and l + 32 in registers;
-// step j broadcasts y_j from its owner lane and every lane below updates
-// its rows, y_i = y_i - L_ij y_j, in ascending j. Every thread of the CTA
-// calls it (256 threads).
+// kTriSmem entries; fwd_triangle_stage first). Lane l holds rows l and l + 32
+// in registers; step j broadcasts y_j from its owner lane and every lane below
+// updates its rows, y_i = y_i - L_ij y_j, in ascending j. Every thread of the
+// CTA calls it.
 template <class R>
-__device__ void fwd_triangle(const Sched& S, const SolveArgs& a, int eb, const cx<R>* Lb, long long lstride,
-                             cx<R>* yb, int s, int blk, unsigned char* smem) {
+__device__ __forceinline__ void fwd_triangle_stage(const Sched& S, int eb, const cx<R>* Lb, long long lstride, int s,
+                                                   int blk, unsigned char* smem) {
+    const int j0 = blk * kSolveBlock, m = S.rows[s];
+    const int jb = min(kSolveBlock, S.first[s + 1] - S.first[s] - j0);
+    stage_block(reinterpret_cast<cx<R>*>(smem), Lb + lstride * eb + S.loff[s] + j0 + static_cast<long long>(j0) * m, m,
+                jb, jb);
+}
+template <class R>
+__device__ void fwd_triangle(const Sched& S, const SolveArgs& a, int eb, cx<R>* yb, int s, int blk,
+                             unsigned char* smem) {
     static_assert(kSolveBlock == 64, "two rows per lane");
-    cx<R>* T = reinterpret_cast<cx<R>*>(smem);
+    const cx<R>* T = reinterpret_cast<const cx<R>*>(smem);
     const int j0 = blk * kSolveBlock;
-    const int w = S.first[s + 1] - S.first[s];
-    const int m = S.rows[s];
     const int f = S.first[s];
-    const int jb = min(kSolveBlock, w - j0);
-    stage_triangle(T, Lb + lstride * eb + S.loff[s] + j0 + static_cast<long long>(j0) * m, m, jb);
+    const int jb = min(kSolveBlock, S.first[s + 1] - f - j0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     cx<R>* y = yb + vec_at(a, eb, warp) * a.n + f + j0;
     cx<R> y0{0, 0}, y1{0, 0};
@@ -1295,58 +1313,78 @@ __device__ void fwd_triangle(const Sched& S, const SolveArgs& a, int eb, const c
     triangle_wait();
     __syncthreads();
     if (warp < a.nr) {
-        for (int j = 0; j < jb; ++j) {
-            const cx<R> src = j < 32 ? y0 : y1;
+        const int j1 = min(jb, 32);
+#pragma unroll 4
+        for (int j = 0; j < j1; ++j) {
             cx<R> yj;
-            yj.re = __shfl_sync(0xffffffffu, src.re, j & 31);
-            yj.im = __shfl_sync(0xffffffffu, src.im, j & 31);
-            if (lane > j) y0 = fms(y0, T[lane + j * kTriLd], yj);
-            if (lane + 32 > j && lane + 32 < jb) y1 = fms(y1, T[lane + 32 + j * kTriLd], yj);
+            yj.re = __shfl_sync(0xffffffffu, y0.re, j);
+            yj.im = __shfl_sync(0xffffffffu, y0.im, j);
+            const cx<R> l0 = T[lane + j * kTriLd], l1 = T[lane + 32 + j * kTriLd];
+            if (lane > j) y0 = fms(y0, l0, yj);
+            if (lane + 32 < jb) y1 = fms(y1, l1, yj);
+        }
+#pragma unroll 4
+        for (int j = 32; j < jb; ++j) {
+            cx<R> yj;
+            yj.re = __shfl_sync(0xffffffffu, y1.re, j & 31);
+            yj.im = __shfl_sync(0xffffffffu, y1.im, j & 31);
+            const cx<R> l1 = T[lane + 32 + j * kTriLd];
+            if (lane + 32 > j && lane + 32 < jb) y1 = fms(y1, l1, yj);
         }
         if (lane < jb) y[lane] = y0;
         if (lane + 32 < jb) y[lane + 32] = y1;
     }
 }
 
-// Item (s): the children's update vectors added into supernode s's front
-// vector (y at its pivot rows, its own update segment U_s below). Fused: the
-// same CTA then solves the supernode's first block (dynamic shared memory
-// kTriSmem entries).
+// Item (s), blockIdx.z: the children's update vectors added into rows
+// 512 z .. of supernode s's front vector (y at its pivot rows, its own update
+// segment U_s below), children in order, every rhs of the pass at once. A CTA
+// reads each child's map whole and takes the entries in its rows. Fused: the
+// front's first CTA then solves the supernode's first block (dynamic shared
+// memory kTriSmem entries).
 template <class R, bool Fused>
 __global__ void __launch_bounds__(256) k_fwd_gather(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
                                                     long long lstride, cx<R>* yb, cx<R>* Ub) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_start_next();
     const int eb = solve_entry(a);
     const int s = S.items[item0 + blockIdx.x].s;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
-    const int cs = m - w;
     const int f = S.first[s];
-    if constexpr (Fused)  // the first block's triangle, staged after the gather
-        prefetch_triangle(Lb + lstride * eb + S.loff[s], m, min(kSolveBlock, w));
-    for (int k = 0; k < a.nr; ++k) {
-        cx<R>* y = yb + vec_at(a, eb, k) * a.n;
-        cx<R>* U = Ub + vec_at(a, eb, k) * a.upool;
-        cx<R>* Us = U + S.uoff[s];
-        for (int i = threadIdx.x; i < cs; i += blockDim.x) Us[i] = cx<R>{0, 0};
+    const int r0 = blockIdx.z * kGatherRows, r1 = min(r0 + kGatherRows, m);
+    const bool triangle = Fused && blockIdx.z == 0 && w > 0;
+    if constexpr (Fused)
+        if (triangle) fwd_triangle_stage<R>(S, eb, Lb, lstride, s, 0, smem_raw);
+    pdl_wait();
+    if (r0 < m) {
+        cx<R>* const y = yb + vec_at(a, eb, 0) * a.n + f;
+        cx<R>* const U = Ub + vec_at(a, eb, 0) * a.upool;
+        cx<R>* const Us = U + S.uoff[s];
+        for (int i = max(r0, w) + threadIdx.x; i < r1; i += blockDim.x)
+            for (int k = 0; k < a.nr; ++k) Us[k * a.upool + i - w] = cx<R>{0, 0};
         __syncthreads();
         for (int t = S.child_ptr[s]; t < S.child_ptr[s + 1]; ++t) {
             const int c = S.child_list[t];
             const int cc = S.rows[c] - (S.first[c + 1] - S.first[c]);
             const int* rel = S.rel + S.reloff[c];
             const cx<R>* Uc = U + S.uoff[c];
+#pragma unroll 4
             for (int i = threadIdx.x; i < cc; i += blockDim.x) {
                 const int p = rel[i];
-                if (p < w) y[f + p] = y[f + p] + Uc[i];
-                else Us[p - w] = Us[p - w] + Uc[i];
+                if (p < r0 || p >= r1) continue;
+                cx<R>* dst = p < w ? y + p : Us + (p - w);
+                const long long step = p < w ? a.n : a.upool;
+                for (int k = 0; k < a.nr; ++k) dst[k * step] = dst[k * step] + Uc[k * a.upool + i];
             }
             __syncthreads();
         }
     }
     if constexpr (Fused) {
+        if (!triangle) return;
         __threadfence();
         __syncthreads();
-        if (w > 0) fwd_triangle<R>(S, a, eb, Lb, lstride, yb, s, 0, smem_raw);
+        fwd_triangle<R>(S, a, eb, yb, s, 0, smem_raw);
     }
 }
 
@@ -1355,24 +1393,30 @@ template <class R>
 __global__ void __launch_bounds__(256) k_fwd_diag(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
                                                   long long lstride, cx<R>* yb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
-    fwd_triangle<R>(S, a, solve_entry(a), Lb, lstride, yb, it.s, it.a, smem_raw);
+    const int eb = solve_entry(a);
+    fwd_triangle_stage<R>(S, eb, Lb, lstride, it.s, it.a, smem_raw);
+    pdl_wait();
+    fwd_triangle<R>(S, a, eb, yb, it.s, it.a, smem_raw);
 }
 
 // Item (s, blk, row0): rows row0 .. row0 + kSolveRows - 1 of the supernode
 // minus L[rows, blk] y[blk]. Four threads per row, each over 16 of the
-// block's columns with all 16 loads in flight (one round trip); the four
-// column-ordered sub-sums are added in order. Fused: the last of the
-// block's CTAs then solves block blk + 1 (counters: one per supernode and
-// grid row; dynamic shared memory kTriSmem entries).
+// block's columns, all 16 loads in flight before the launch before has
+// finished; the four column-ordered sub-sums are added in order, rhs k by the
+// row's thread k % 4. Fused: the last of the block's CTAs then solves block
+// blk + 1 (counters: one per supernode and grid row; dynamic shared memory
+// kTriSmem entries).
 template <class R, bool Fused>
 __global__ void __launch_bounds__(256) k_fwd_update(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
                                                     long long lstride, cx<R>* yb, cx<R>* Ub) {
     static_assert(kSolveRows * 4 == 256 && kSolveBlock == 64, "four 16-column quarters per row");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int eb = solve_entry(a);
     __shared__ cx<R> ys[8][kSolveBlock];
-    __shared__ cx<R> red[3][8][kSolveRows];  // quarters 1..3's sub-sums
+    __shared__ cx<R> red[4][8][kSolveRows];  // the quarters' sub-sums
+    pdl_start_next();
+    const int eb = solve_entry(a);
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, j0 = it.a * kSolveBlock, row0 = it.b;
     const int w = S.first[s + 1] - S.first[s];
@@ -1382,8 +1426,6 @@ __global__ void __launch_bounds__(256) k_fwd_update(Sched S, long long item0, So
     const int t = threadIdx.x % kSolveRows, qt = threadIdx.x / kSolveRows;
     const int r = row0 + t;
     const int c0 = 16 * qt, nc = min(16, jb - c0);
-    // The panel entries first (they depend on the item only), so their round
-    // trip overlaps the block's y values'.
     cx<R> l[16];
     {
         const bool live = r < m && nc > 0;
@@ -1391,141 +1433,161 @@ __global__ void __launch_bounds__(256) k_fwd_update(Sched S, long long item0, So
 #pragma unroll
         for (int u = 0; u < 16; ++u) l[u] = live && u < nc ? P[static_cast<long long>(u) * m] : cx<R>{0, 0};
     }
-    // The first rhs's destination, read now (only this CTA writes these rows
-    // in this launch).
-    cx<R>* dst0 = r < w ? yb + vec_at(a, eb, 0) * a.n + f + r : Ub + vec_at(a, eb, 0) * a.upool + S.uoff[s] + (r - w);
-    const cx<R> old0 = qt == 0 && r < m ? *dst0 : cx<R>{0, 0};
     if constexpr (Fused) {
         const int jn = j0 + kSolveBlock;  // the next block, which this launch's last CTA solves
         if (row0 == j0 + jb && jn < w)
             prefetch_triangle(Lb + lstride * eb + S.loff[s] + jn + static_cast<long long>(jn) * m, m,
                               min(kSolveBlock, w - jn));
     }
-    for (int e = threadIdx.x; e < jb * a.nr; e += blockDim.x) {
-        const int j = e % jb, k = e / jb;
-        ys[k][j] = yb[vec_at(a, eb, k) * a.n + f + j0 + j];
+    pdl_wait();
+    // The destinations, read now (only this CTA writes these rows in this launch).
+    auto at = [&](int k) {
+        return r < w ? yb + vec_at(a, eb, k) * a.n + f + r : Ub + vec_at(a, eb, k) * a.upool + S.uoff[s] + (r - w);
+    };
+    cx<R> old[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) old[h] = r < m && qt + 4 * h < a.nr ? *at(qt + 4 * h) : cx<R>{0, 0};
+    for (int e = threadIdx.x; e < kSolveBlock * a.nr; e += blockDim.x) {
+        const int j = e % kSolveBlock, k = e / kSolveBlock;
+        if (j < jb) ys[k][j] = yb[vec_at(a, eb, k) * a.n + f + j0 + j];
     }
     __syncthreads();
-    cx<R> acc[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) acc[k] = cx<R>{0, 0};
-    if (r < m && nc > 0) {
+    for (int k = 0; k < 8; ++k) {
+        if (k >= a.nr) break;
+        cx<R> acc{0, 0};
+        if (r < m && nc > 0) {
 #pragma unroll
-        for (int u = 0; u < 16; ++u) {
-            if (u >= nc) break;
-#pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (k < a.nr) acc[k] = acc[k] + l[u] * ys[k][c0 + u];
+            for (int u = 0; u < 16; ++u) {
+                if (u >= nc) break;
+                acc = acc + l[u] * ys[k][c0 + u];
+            }
         }
-    }
-    if (qt > 0) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < a.nr) red[qt - 1][k][t] = acc[k];
+        red[qt][k][t] = acc;
     }
     __syncthreads();
-    if (qt == 0 && r < m) {
+    if (r < m) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (k >= a.nr) break;
-            const cx<R> sum = ((acc[k] + red[0][k][t]) + red[1][k][t]) + red[2][k][t];
-            cx<R>* dst = r < w ? yb + vec_at(a, eb, k) * a.n + f + r
-                               : Ub + vec_at(a, eb, k) * a.upool + S.uoff[s] + (r - w);
-            *dst = (k == 0 ? old0 : *dst) - sum;
+        for (int h = 0; h < 2; ++h) {
+            const int k = qt + 4 * h;
+            if (k < a.nr) *at(k) = old[h] - (((red[0][k][t] + red[1][k][t]) + red[2][k][t]) + red[3][k][t]);
         }
     }
     if constexpr (Fused) {
         const int below = j0 + jb;
         const int chunks = (m - below + kSolveRows - 1) / kSolveRows;
         if (last_to_arrive(a.counters + static_cast<long long>(blockIdx.y) * a.ns + s, chunks) &&
-            it.a + 1 < solve_nblocks(S, s))
-            fwd_triangle<R>(S, a, eb, Lb, lstride, yb, s, it.a + 1, smem_raw);
+            it.a + 1 < solve_nblocks(S, s)) {
+            fwd_triangle_stage<R>(S, eb, Lb, lstride, s, it.a + 1, smem_raw);
+            fwd_triangle<R>(S, a, eb, yb, s, it.a + 1, smem_raw);
+        }
     }
 }
 
 // Backward triangle of block blk of supernode s: x[blk] = L_bb^-T (D^-1
 // y[blk] - sum of the partials in slots p0 .. p0 + np - 1) for the pass's
-// rhs (smem: kTriSmem + kRedSmem entries). The partials are summed by four
-// threads per (column, rhs), each over every fourth slot in slot order, the
-// four sub-sums then added in order. The triangle: one warp per rhs, lane l
-// holding rows l and l + 32; step j (descending) broadcasts x_j from its
-// owner lane and every lane above updates its rows, z_t = z_t - L_jt x_j.
-// Every thread of the CTA calls it (256 threads).
+// rhs (smem: kTriSmem + red_smem(nr) entries, L_bb already being staged at its
+// start). The partials are summed by kRedGroups threads per (column, rhs),
+// each over every kRedGroups-th slot in slot order, the sub-sums then added in
+// order. The triangle: one warp per rhs, lane l holding rows l and l + 32;
+// step j (descending) broadcasts x_j from its owner lane and every lane above
+// updates its rows, z_t = z_t - L_jt x_j. Every thread of the CTA calls it.
 template <class R>
-__device__ void bwd_triangle(const Sched& S, const SolveArgs& a, int eb, const cx<R>* Lb, long long lstride,
-                             cx<R>* yb, const cx<R>* partb, int s, int blk, int p0, int np, unsigned char* smem) {
+__device__ void bwd_triangle(const Sched& S, const SolveArgs& a, int eb, cx<R>* yb, const cx<R>* partb, int s,
+                             int blk, int p0, int np, unsigned char* smem) {
     static_assert(kSolveBlock == 64, "two rows per lane");
-    cx<R>* T = reinterpret_cast<cx<R>*>(smem);
-    cx<R>* red = T + kTriSmem;  // [4][8][kSolveBlock]
+    const cx<R>* T = reinterpret_cast<const cx<R>*>(smem);
+    cx<R>* red = reinterpret_cast<cx<R>*>(smem) + kTriSmem;  // [group][rhs][column]
     const int j0 = blk * kSolveBlock;
-    const int w = S.first[s + 1] - S.first[s];
-    const int m = S.rows[s];
     const int f = S.first[s];
-    const int jb = min(kSolveBlock, w - j0);
-    stage_triangle(T, Lb + lstride * eb + S.loff[s] + j0 + static_cast<long long>(j0) * m, m, jb);
-    const cx<R>* part = partb + static_cast<long long>(eb) * a.max_parts * kSolveBlock * 8;
-    for (int e = threadIdx.x; e < 4 * kSolveBlock * a.nr; e += blockDim.x) {
-        const int g = e & 3, j = (e >> 2) % kSolveBlock, k = (e >> 2) / kSolveBlock;
+    const int jb = min(kSolveBlock, S.first[s + 1] - f - j0);
+    const cx<R>* part = partb + (static_cast<long long>(eb) * a.max_parts + p0) * (kSolveBlock * 8);
+    for (int e = threadIdx.x; e < kRedGroups * kSolveBlock * a.nr; e += blockDim.x) {
+        const int j = e % kSolveBlock, k = e / kSolveBlock % a.nr, g = e / kSolveBlock / a.nr;
         cx<R> sum{0, 0};
         if (j < jb) {
-            constexpr int kU = 16;  // loads in flight per thread
+            const cx<R>* pj = part + k * kSolveBlock + j;
+            constexpr int kU = 16, kSlot = kSolveBlock * 8;  // loads in flight per thread
             int q = g;
-            for (; q + 4 * (kU - 1) < np; q += 4 * kU) {
+            for (; q + kRedGroups * (kU - 1) < np; q += kRedGroups * kU) {
                 cx<R> v[kU];
 #pragma unroll
-                for (int u = 0; u < kU; ++u)
-                    v[u] = ld_l2(part + (static_cast<long long>(p0 + q + 4 * u) * kSolveBlock + j) * 8 + k);
+                for (int u = 0; u < kU; ++u) v[u] = ld_l2(pj + static_cast<long long>(q + kRedGroups * u) * kSlot);
 #pragma unroll
                 for (int u = 0; u < kU; ++u) sum = sum + v[u];
             }
-            for (; q < np; q += 4) sum = sum + ld_l2(part + (static_cast<long long>(p0 + q) * kSolveBlock + j) * 8 + k);
+            if (q < np) {  // the rest, predicated, in flight too
+                cx<R> v[kU];
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (q + kRedGroups * u < np) v[u] = ld_l2(pj + static_cast<long long>(q + kRedGroups * u) * kSlot);
+#pragma unroll
+                for (int u = 0; u < kU; ++u)
+                    if (q + kRedGroups * u < np) sum = sum + v[u];
+            }
         }
-        red[(g * 8 + k) * kSolveBlock + j] = sum;
+        red[e] = sum;  // (g, k, j)
     }
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cx<R>* y = yb + vec_at(a, eb, warp) * a.n + f + j0;
+    cx<R> z[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) z[h] = warp < a.nr && lane + 32 * h < jb ? ld_l2(y + lane + 32 * h) : cx<R>{0, 0};
     triangle_wait();
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp < a.nr) {
-        cx<R>* y = yb + vec_at(a, eb, warp) * a.n + f + j0;
-        cx<R> z[2];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int j = lane + 32 * h;
-            z[h] = cx<R>{0, 0};
             if (j < jb) {
                 const cx<R>* rj = red + warp * kSolveBlock + j;
-                const cx<R> sum = ((rj[0] + rj[8 * kSolveBlock]) + rj[16 * kSolveBlock]) + rj[24 * kSolveBlock];
-                z[h] = ld_l2(y + j) * crecip(T[j * (kTriLd + 1)]) - sum;
+                cx<R> sum = rj[0];
+#pragma unroll
+                for (int g = 1; g < kRedGroups; ++g) sum = sum + rj[g * kSolveBlock * a.nr];
+                z[h] = z[h] * crecip(T[j * (kTriLd + 1)]) - sum;
             }
         }
-        for (int j = jb - 1; j >= 0; --j) {
-            const cx<R> src = j < 32 ? z[0] : z[1];
+#pragma unroll 4
+        for (int j = jb - 1; j >= 32; --j) {
             cx<R> xj;
-            xj.re = __shfl_sync(0xffffffffu, src.re, j & 31);
-            xj.im = __shfl_sync(0xffffffffu, src.im, j & 31);
-            if (lane < j) z[0] = fms(z[0], T[j + lane * kTriLd], xj);
-            if (lane + 32 < j) z[1] = fms(z[1], T[j + (lane + 32) * kTriLd], xj);
+            xj.re = __shfl_sync(0xffffffffu, z[1].re, j & 31);
+            xj.im = __shfl_sync(0xffffffffu, z[1].im, j & 31);
+            const cx<R> l0 = T[j + lane * kTriLd], l1 = T[j + (lane + 32) * kTriLd];
+            z[0] = fms(z[0], l0, xj);
+            if (lane + 32 < j) z[1] = fms(z[1], l1, xj);
+        }
+#pragma unroll 4
+        for (int j = min(jb, 32) - 1; j >= 0; --j) {
+            cx<R> xj;
+            xj.re = __shfl_sync(0xffffffffu, z[0].re, j);
+            xj.im = __shfl_sync(0xffffffffu, z[0].im, j);
+            const cx<R> l0 = T[j + lane * kTriLd];
+            if (lane < j) z[0] = fms(z[0], l0, xj);
         }
         if (lane < jb) y[lane] = z[0];
         if (lane + 32 < jb) y[lane + 32] = z[1];
     }
 }
 
-// Item (s, blk, row0, slot[, p0]): partial[slot][j][k] = sum over rows
+// Item (s, blk, row0, slot[, p0]): partial[slot][k][j] = sum over rows
 // row0 .. row0 + kSolveRows - 1 (below the block) of L[row, j0 + j] x_k[row]
-// (an empty chunk, row0 = m, gives zeros). Warp v takes columns 8v .. 8v + 7,
-// lane l rows l and l + 32: all 16 loads in flight (one round trip); per
-// column the lane's two rows in order, then a butterfly over the warp.
-// Fused: the last of the block's CTAs then reduces the block's partials
-// (slots p0 ..) and solves the block (counters: one per supernode and grid
-// row; dynamic shared memory kTriSmem + kRedSmem entries).
+// (an empty chunk, row0 = m, gives zeros). The rows' block of L is staged in
+// shared memory before the launch before has finished; four threads per
+// column, each over 16 of the rows in order for every rhs, the four sub-sums
+// added in order. (One warp per eight columns with a butterfly per column and
+// rhs took 52 us a launch for eight right-hand sides.) Fused: the last of the
+// block's CTAs then reduces the block's partials (slots p0 ..) and solves the
+// block (counters: one per supernode and grid row). Dynamic shared memory:
+// kTriSmem entries, and red_smem(nr) more when fused.
 template <class R, bool Fused>
 __global__ void __launch_bounds__(256) k_bwd_update(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
                                                     long long lstride, cx<R>* yb, cx<R>* partb) {
-    static_assert(kSolveRows == 64 && kSolveBlock == 64, "two rows per lane, eight columns per warp");
+    static_assert(kSolveRows == 64 && kSolveBlock == 64, "four 16-row quarters per column");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int eb = solve_entry(a);
     __shared__ cx<R> xs[8][kSolveRows];
+    cx<R>* T = reinterpret_cast<cx<R>*>(smem_raw);
+    pdl_start_next();
+    const int eb = solve_entry(a);
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, j0 = it.a * kSolveBlock, row0 = it.b, slot = it.c;
     const int w = S.first[s + 1] - S.first[s];
@@ -1534,68 +1596,69 @@ __global__ void __launch_bounds__(256) k_bwd_update(Sched S, long long item0, So
     const int jb = min(kSolveBlock, w - j0);
     const int nrows = max(0, min(kSolveRows, m - row0));
     const int* st = S.structs + S.soff[s];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // The panel entries first (they depend on the item only), so their round
-    // trip overlaps the gather of x.
+    const cx<R>* P = Lb + lstride * eb + S.loff[s] + static_cast<long long>(j0) * m;
+    stage_block(T, P + row0, m, nrows, jb);
     if constexpr (Fused) {
         if (row0 == j0 + jb)  // the block's triangle, which this launch's last CTA stages
-            prefetch_triangle(Lb + lstride * eb + S.loff[s] + j0 + static_cast<long long>(j0) * m, m, jb);
+            prefetch_triangle(P + j0, m, jb);
     }
-    cx<R> l[8][2];
-    {
-        const cx<R>* P = Lb + lstride * eb + S.loff[s] + static_cast<long long>(j0) * m;
+    const int t = threadIdx.x % kSolveRows, qt = threadIdx.x / kSolveRows;
+    const int g = t < nrows ? (row0 + t < w ? f + row0 + t : st[row0 + t]) : 0;
+    pdl_wait();
+    for (int k = qt; k < a.nr; k += 4)
+        if (t < nrows) xs[k][t] = yb[vec_at(a, eb, k) * a.n + g];
+    triangle_wait();
+    __syncthreads();
+    const int j = t;  // this thread's column
+    cx<R> l[16];
 #pragma unroll
-        for (int c = 0; c < 8; ++c)
+    for (int u = 0; u < 16; ++u) l[u] = T[16 * qt + u + j * kTriLd];
+    __syncthreads();  // T becomes the quarters' sub-sums
+    cx<R>* red = T;   // [quarter][rhs][column]
+    static_assert(4 * 8 * kSolveBlock <= kTriSmem, "the sub-sums fit the block's memory");
+    const int nq = min(16, nrows - 16 * qt);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int j = 8 * warp + c, t = lane + 32 * h;
-                l[c][h] = j < jb && t < nrows ? P[row0 + t + static_cast<long long>(j) * m] : cx<R>{0, 0};
-            }
-    }
-    for (int e = threadIdx.x; e < nrows * a.nr; e += blockDim.x) {
-        const int t = e % nrows, k = e / nrows;
-        const int r = row0 + t;
-        const int g = r < w ? f + r : st[r];
-        xs[k][t] = yb[vec_at(a, eb, k) * a.n + g];
+    for (int k = 0; k < 8; ++k) {
+        if (k >= a.nr) break;
+        cx<R> acc{0, 0};
+#pragma unroll
+        for (int u = 0; u < 16; ++u)
+            if (u < nq) acc = acc + l[u] * xs[k][16 * qt + u];
+        red[(qt * 8 + k) * kSolveBlock + j] = acc;
     }
     __syncthreads();
-    cx<R>* part = partb + static_cast<long long>(eb) * a.max_parts * kSolveBlock * 8 +
-                  static_cast<long long>(slot) * kSolveBlock * 8;
-#pragma unroll
-    for (int c = 0; c < 8; ++c) {
-        const int j = 8 * warp + c;
-        if (j >= jb) break;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            if (k >= a.nr) break;
-            cx<R> v{0, 0};
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                if (lane + 32 * h < nrows) v = v + l[c][h] * xs[k][lane + 32 * h];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                v.re += __shfl_xor_sync(0xffffffffu, v.re, o);
-                v.im += __shfl_xor_sync(0xffffffffu, v.im, o);
-            }
-            if (lane == 0) part[j * 8 + k] = v;
+    cx<R>* part = partb + (static_cast<long long>(eb) * a.max_parts + slot) * (kSolveBlock * 8);
+    if (j < jb)
+        for (int k = qt; k < a.nr; k += 4) {
+            const cx<R>* rk = red + k * kSolveBlock + j;
+            part[k * kSolveBlock + j] =
+                ((rk[0] + rk[8 * kSolveBlock]) + rk[16 * kSolveBlock]) + rk[24 * kSolveBlock];
         }
-    }
     if constexpr (Fused) {
         const int below = j0 + jb;
         const int chunks = max(1, (m - below + kSolveRows - 1) / kSolveRows);
-        if (last_to_arrive(a.counters + static_cast<long long>(blockIdx.y) * a.ns + s, chunks))
-            bwd_triangle<R>(S, a, eb, Lb, lstride, yb, partb, s, it.a, it.d, chunks, smem_raw);
+        if (last_to_arrive(a.counters + static_cast<long long>(blockIdx.y) * a.ns + s, chunks)) {
+            stage_block(T, P + j0, m, jb, jb);
+            bwd_triangle<R>(S, a, eb, yb, partb, s, it.a, it.d, chunks, smem_raw);
+        }
     }
 }
 
 // Item (s, blk, first_slot, nslots): x[blk] = L_bb^-T (D^-1 y[blk] - sum of
 // partials) (the split plan's triangle launch).
 template <class R>
-__global__ void __launch_bounds__(256) k_bwd_diag(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
-                                                  long long lstride, cx<R>* yb, const cx<R>* partb) {
+__global__ void __launch_bounds__(kBwdDiagThreads) k_bwd_diag(Sched S, long long item0, SolveArgs a, const cx<R>* Lb,
+                                                              long long lstride, cx<R>* yb, const cx<R>* partb) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
-    bwd_triangle<R>(S, a, solve_entry(a), Lb, lstride, yb, partb, it.s, it.a, it.b, it.c, smem_raw);
+    const int eb = solve_entry(a);
+    const int j0 = it.a * kSolveBlock, m = S.rows[it.s];
+    const int jb = min(kSolveBlock, S.first[it.s + 1] - S.first[it.s] - j0);
+    stage_block(reinterpret_cast<cx<R>*>(smem_raw),
+                Lb + lstride * eb + S.loff[it.s] + j0 + static_cast<long long>(j0) * m, m, jb, jb);
+    pdl_wait();
+    bwd_triangle<R>(S, a, eb, yb, partb, it.s, it.a, it.b, it.c, smem_raw);
 }
 
 }  // namespace aphi_b200
