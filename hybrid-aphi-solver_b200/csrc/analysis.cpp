@@ -46,13 +46,13 @@ struct Uploads {
 
 // The factorization plans: per level, extend-add items, then one-CTA fronts,
 // then the blocked steps of the large fronts. A large front is processed in
-// 128-column panels; each 32-column step of a panel factors its diagonal
+// 128-column panels; each 64-column step of a panel factors its diagonal
 // block, solves the panel rows below it and updates the rest of the panel's
 // own columns. Once a panel is complete, its trailing update -- every column
 // to its right, K = panel width -- runs as 128 x 64 tiles: `trailing` is
 // K_UPDATE_WIDE (DMMA for FP64, SIMT for FP32) or K_UPDATE_TC (tensor cores, FP32).
-// Updating the trailing front once per 128 columns instead of once per 32
-// reads and writes it a quarter as often.
+// Updating the trailing front once per 128 columns instead of once per 64
+// reads and writes it half as often.
 void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing, std::vector<Launch>& plan) {
     const Symbolic& S = A.S;
     auto push = [&](int kind, long long first, int kcap = kTcPanel, int wide = 0) {
@@ -60,7 +60,7 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
         if (count > 0) plan.push_back({kind, first, count, kcap, wide});
     };
     // The FP64 plan (and the SIMT FP32 one) runs the in-panel updates on the
-    // trailing-update kernel as 128 x 64 tiles of K = 32, its columns capped
+    // trailing-update kernel as 128 x 64 tiles of K = 64, its columns capped
     // at the panel's end; the tensor-core plan keeps the 64 x 64 SIMT tiles.
     const bool panel_wide = trailing == K_UPDATE_WIDE;
     // Trailing updates whose operands are prepared once per front and panel
@@ -140,7 +140,7 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
                 }
             }
             push(K_UPDATE_PANEL, f0, panel_wide ? kStep : kTcPanel, panel_wide ? 1 : 0);
-            // A panel's trailing update follows its last 32-column step. Tiles
+            // A panel's trailing update follows its last 64-column step. Tiles
             // cover rows and columns [pe, jend) x ..., lower part only.
             // One launch per K cap: a group's last panel applies the whole group.
             for (int cap_group : {1, 2, 4}) {

@@ -49,9 +49,9 @@ struct Item {
                 // of an entry's workspace (K_UPDATE_TC / K_TC_SPLIT; K_UPDATE_WIDE / K_DMMA_SCALE)
 };
 
-constexpr int kStep = 32;        // pivot block width of the blocked factorization
+constexpr int kStep = 64;        // pivot block width of the blocked factorization
 constexpr int kTile = 64;        // update tile
-constexpr int kTrsmRows = 128;   // rows per TRSM block
+constexpr int kTrsmRows = 64;    // rows per TRSM block
 constexpr int kPanelGroup = 4;                 // most panels per trailing update of the rest of a front
 constexpr int kWidePair = kPanelGroup * kTcPanel;  // the most panel columns one trailing update applies
 // Fronts this tall group 4 panels, smaller ones 2. A build may lower the

@@ -377,7 +377,7 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     cx<R>* L = reinterpret_cast<cx<R>*>(f->L);
     cx<R>* CB = reinterpret_cast<cx<R>*>(f->CB);
     const long long ls = A->S.stored, cs = A->S.cb_pool;
-    const int smallsm = A->opt.small_front * A->opt.small_front * static_cast<int>(sizeof(cx<R>));
+    const int smallsm = small_smem<R>(A->opt.small_front);
     aphi_factor* fm = const_cast<aphi_factor*>(f);
     const bool prof = f->profile;
     const bool presplit = sizeof(R) == 4 && f->tc_split == 2 && f->presplit && f->tcws;
@@ -385,9 +385,9 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     auto update_i8 = [&](const Launch& l) {
         using C = std::conditional_t<sizeof(R) == 8, I8Fp64, I8Fp32>;
         const long long tiles = static_cast<long long>(l.count) * (kTcN / C::Nc) * f->batch;
-        k_update_i8<R, C><<<static_cast<unsigned>(std::min<long long>(tiles, f->sms)), kI8Threads, C::smem, st>>>(
-            S, l.first, l.count, f->batch, L, CB, ls, cs, l.kcap, sizeof(R) == 8 ? f->dws : f->tcws,
-            sizeof(R) == 8 ? f->dws_stride : f->tcws_stride, f->err);
+        chained(k_update_i8<R, C>, dim3(static_cast<unsigned>(std::min<long long>(tiles, f->sms))), kI8Threads, C::smem,
+                st, S, l.first, l.count, f->batch, L, CB, ls, cs, l.kcap, sizeof(R) == 8 ? f->dws : f->tcws,
+                sizeof(R) == 8 ? f->dws_stride : f->tcws_stride, f->err);
     };
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
     const size_t bwd_smem = (kTriSmem + (sa ? red_smem(sa->nr) : 0)) * sizeof(cx<R>);  // backward triangles
@@ -410,38 +410,38 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
             APHI_CUDA(cudaEventRecord(e[0], st));
         }
         switch (l.kind) {
-            case K_EXTEND_ADD: k_extend_add<R><<<grid, 256, 0, st>>>(S, l.first, L, CB, ls, cs); break;
-            case K_SMALL: k_small_front<R><<<grid, 256, smallsm, st>>>(S, l.first, L, CB, ls, cs); break;
-            case K_DIAG: k_diag_block<R><<<grid, 128, 0, st>>>(S, l.first, L, ls); break;
-            case K_TRSM: k_panel_trsm<R><<<grid, kTrsmRows, 0, st>>>(S, l.first, L, ls); break;
+            case K_EXTEND_ADD: chained(k_extend_add<R>, grid, 256, 0, st, S, l.first, L, CB, ls, cs); break;
+            case K_SMALL: chained(k_small_front<R>, grid, kLdltThreads, smallsm, st, S, l.first, L, CB, ls, cs); break;
+            case K_DIAG: chained(k_diag_block<R>, grid, kDiagThreads, diag_smem<R>(), st, S, l.first, L, ls); break;
+            case K_TRSM: chained(k_panel_trsm<R>, grid, kTrsmThreads, trsm_smem<R>(), st, S, l.first, L, ls); break;
             case K_UPDATE_WIDE:
             case K_UPDATE_PANEL:
                 if (l.kind == K_UPDATE_PANEL && !l.wide) {
-                    k_update_panel<R><<<grid, 256, 2 * kStep * kTile * sizeof(cx<R>), st>>>(S, l.first, L, CB, ls, cs);
+                    chained(k_update_panel<R>, grid, 256, 2 * kStep * kTile * sizeof(cx<R>), st, S, l.first, L, CB, ls, cs);
                     break;
                 }
                 if constexpr (sizeof(R) == 8) {
                     if (l.kind == K_UPDATE_WIDE && prescaled)
                         update_i8(l);
                     else
-                        k_update_wide_dmma<<<grid, 256, kDmmaSmem, st>>>(S, l.first, L, CB, ls, cs, l.kcap,
-                                                                         l.kind == K_UPDATE_PANEL ? 1 : 0);
+                        chained(k_update_wide_dmma, grid, 256, kDmmaSmem, st, S, l.first, L, CB, ls, cs, l.kcap,
+                                l.kind == K_UPDATE_PANEL ? 1 : 0);
                 } else
                     k_update_wide<R><<<grid, 256, wide_smem<R>(), st>>>(S, l.first, L, CB, ls, cs, l.kcap,
                                                                       l.kind == K_UPDATE_PANEL ? 1 : 0);
                 break;
             case K_DMMA_SCALE:
                 if constexpr (sizeof(R) == 8)
-                    k_i8_split<double, I8Fp64><<<dim3(grid.x, grid.y, kTcM / 32), 256, 0, st>>>(
-                        S, l.first, L, ls, f->dws, f->dws_stride, l.kcap);
+                    chained(k_i8_split<double, I8Fp64>, dim3(grid.x, grid.y, kTcM / 32), 256, 0, st, S, l.first, L, ls,
+                            f->dws, f->dws_stride, l.kcap);
                 else
                     throw Error(APHI_ERR_INVALID, "operand scaling planned for an FP32 factor");
                 break;
             case K_TC_SPLIT:
                 if constexpr (sizeof(R) == 4) {
                     if (i8) {
-                        k_i8_split<float, I8Fp32><<<dim3(grid.x, grid.y, kTcM / 32), 256, 0, st>>>(
-                            S, l.first, L, ls, f->tcws, f->tcws_stride, l.kcap);
+                        chained(k_i8_split<float, I8Fp32>, dim3(grid.x, grid.y, kTcM / 32), 256, 0, st, S, l.first, L,
+                                ls, f->tcws, f->tcws_stride, l.kcap);
                         break;
                     }
                     k_tc_split<<<dim3(grid.x, grid.y, (l.kcap + 8 * kTcK - 1) / (8 * kTcK)), kTcThreads, 0, st>>>(
@@ -532,7 +532,9 @@ void set_smem_limits(int small_front) {
     std::lock_guard<std::mutex> lock(mu);
     if (done) return;
     APHI_CUDA(cudaFuncSetAttribute(k_small_front<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   96 * 96 * static_cast<int>(sizeof(cx<R>))));
+                                   small_smem<R>(96)));
+    APHI_CUDA(cudaFuncSetAttribute(k_diag_block<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, diag_smem<R>()));
+    APHI_CUDA(cudaFuncSetAttribute(k_panel_trsm<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, trsm_smem<R>()));
     APHI_CUDA(cudaFuncSetAttribute(k_update_panel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    2 * kStep * kTile * static_cast<int>(sizeof(cx<R>))));
     APHI_CUDA(cudaFuncSetAttribute(k_update_wide<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, wide_smem<R>()));

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <cfloat>
+#include <type_traits>
 
 #include "analysis.hpp"
 #include "common.cuh"
@@ -82,6 +83,47 @@ inline Sched sched_of(const DeviceSchedule& d) {
                  d.child_ptr, d.child_list, d.uoff, d.items};
 }
 
+// A factorization or a solve is a chain of short launches, and much of a short
+// launch is its start: items, schedule, and in a solve the panel entries, all
+// of them constants. So these kernels are launched with programmatic stream
+// serialization: a kernel lets the next one start as it begins itself
+// (pdl_start_next), which then reads its constants and waits (pdl_wait) until
+// the kernel before it has finished and its writes are visible. Everything
+// that a launch before could have written, or still reads where this one
+// writes, comes after pdl_wait(); every kernel launched this way calls it, so
+// that the wait covers all launches before.
+__device__ __forceinline__ void pdl_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// ---------------------------------------------------------------- 64 x 64 blocks
+// Blocks of L in shared memory have leading dimension kTriLd (65: column-
+// strided reads fall in distinct banks).
+constexpr int kTriLd = kSolveBlock + 1;
+constexpr int kTriSmem = kSolveBlock * kTriLd;  // complex entries
+
+// A block of L (rows x cols at P, leading dimension m) into shared memory T
+// (leading dimension kTriLd, zeros outside the rows x cols block) by
+// asynchronous copies (cp.async, zero-filled where the source size is 0), so
+// the caller's own loads overlap them; the caller waits with
+// triangle_wait() and a __syncthreads() before reading T.
+__device__ __forceinline__ void cp_async_entry(uint32_t dst, const cx<double>* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_async_entry(uint32_t dst, const cx<float>* src, bool in) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8u : 0u) : "memory");
+}
+template <class R>
+__device__ __forceinline__ void stage_block(cx<R>* T, const cx<R>* P, long long m, int rows, int cols) {
+#pragma unroll 4
+    for (int e = threadIdx.x; e < kSolveBlock * kSolveBlock; e += blockDim.x) {
+        const int i = e % kSolveBlock, j = e / kSolveBlock;
+        const bool in = i < rows && j < cols;
+        cp_async_entry(smem_u32(T + i + j * kTriLd), in ? P + i + static_cast<long long>(j) * m : P, in);
+    }
+    cp_async_commit();
+}
+__device__ __forceinline__ void triangle_wait() { cp_async_wait<0>(); }
+
 // ---------------------------------------------------------------- extend-add
 // Item (s, c0): front columns [c0, c0 + 32) of supernode s. Zeroes the CB
 // columns in that range, then adds every child's contribution block entries
@@ -89,6 +131,7 @@ inline Sched sched_of(const DeviceSchedule& d) {
 template <class R>
 __global__ void __launch_bounds__(256) k_extend_add(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
                                                     long long lstride, long long cbstride) {
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, c0 = it.a;
     cx<R>* L = Lb + lstride * blockIdx.y;
@@ -100,6 +143,7 @@ __global__ void __launch_bounds__(256) k_extend_add(Sched S, long long item0, cx
     cx<R>* Ls = L + S.loff[s];
     cx<R>* CBs = CB + (cs > 0 ? S.cboff[s] : 0);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    pdl_wait();
     for (int j = max(c0, w) + warp; j < c1; j += 8)
         for (int i = j + lane; i < m; i += 32) CBs[(i - w) + static_cast<long long>(j - w) * cs] = cx<R>{0, 0};
     __syncthreads();
@@ -139,135 +183,279 @@ __global__ void __launch_bounds__(256) k_extend_add(Sched S, long long item0, cx
 }
 
 // ---------------------------------------------------------------- small fronts
+// 1 / d by one division where |d|^2 is far from the type's limits.
+__device__ __forceinline__ cx<double> crecip_fast(cx<double> d) {
+    const double n = d.re * d.re + d.im * d.im;
+    if (!(n > 1e-250 && n < 1e250)) return crecip(d);
+    const double r = 1.0 / n;
+    return {d.re * r, -d.im * r};
+}
+__device__ __forceinline__ cx<float> crecip_fast(cx<float> d) {
+    const float n = d.re * d.re + d.im * d.im;
+    if (!(n > 1e-30f && n < 1e30f)) return crecip(d);
+    const float r = 1.0f / n;
+    return {d.re * r, -d.im * r};
+}
+
+// The right-looking LDL^T of the leading w columns of an m x m lower triangle F
+// in shared memory (leading dimension ld, m <= 32 H), by 256 threads. The
+// triangle sits in registers: lane l holds rows l + 32 h, warp v the columns
+// v + 8 c, and a step needs one column of it in shared memory, which its warp
+// publishes at the end of the step before. So a column costs one barrier, its
+// pivot's reciprocal and a burst of independent updates. (With the triangle in
+// shared memory a step's loads, one entry after the other, made it 0.8-0.9 us;
+// unrolled over a block's columns instead, the code itself is fetched once a
+// launch and takes as long.) The columns' registers move down as blocks of
+// eight are finished, so that every register index is a constant in a short
+// loop. Columns stay unscaled in F: the multipliers are F[i, j] inv[j].
+// Measured per launch: 64-column diagonal blocks of 24^3 (eight FP64 entries)
+// 39 us, FP32 29 us, against 24 and 19 us for each 32 columns before; one-CTA
+// fronts of 8^3 29 us (52).
+constexpr int kLdltThreads = 256;
+template <int H, class R>
+__device__ __forceinline__ void ldlt_columns(cx<R>* F, int ld, int m, int w, cx<R>* inv) {
+    constexpr int C = 4 * H;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    cx<R> a[C][H];
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const int i = lane + 32 * h, j = warp + 8 * c;
+            a[c][h] = i < m && j <= i ? F[i + j * ld] : cx<R>{0, 0};
+        }
+    for (int k = 0; k < w; ++k) {
+        const cx<R>* col = F + k * ld;
+        const int base = k & ~7;
+        const cx<R> r = crecip_fast(col[k]);
+        if (threadIdx.x == 0) inv[k] = r;
+        cx<R> x[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) x[h] = lane + 32 * h < m ? col[lane + 32 * h] : cx<R>{0, 0};
+        // Half of the columns at a time, without branches between them: their
+        // loads are in flight together (past the triangle: the last row's).
+        auto update = [&](auto half) {
+            constexpr int c0 = half.value * C / 2;
+            cx<R> l[C / 2];
+#pragma unroll
+            for (int c = 0; c < C / 2; ++c) l[c] = col[min(warp + base + 8 * (c0 + c), m - 1)];
+#pragma unroll
+            for (int c = 0; c < C / 2; ++c) {
+                l[c] = l[c] * r;
+#pragma unroll
+                for (int h = 0; h < H; ++h) a[c0 + c][h] = fms(a[c0 + c][h], x[h], l[c]);
+            }
+        };
+        update(std::integral_constant<int, 0>{});
+        if (base + 4 * C < m) update(std::integral_constant<int, 1>{});
+        if (k + 1 < w && warp == ((k + 1) & 7)) {
+            const bool same = (k & 7) != 7;  // the next column's block of eight
+#pragma unroll
+            for (int h = 0; h < H; ++h)
+                if (lane + 32 * h < m && lane + 32 * h > k) F[lane + 32 * h + (k + 1) * ld] = same ? a[0][h] : a[1][h];
+        }
+        if ((k & 7) == 7)
+#pragma unroll
+            for (int c = 0; c + 1 < C; ++c)
+#pragma unroll
+                for (int h = 0; h < H; ++h) a[c][h] = a[c + 1][h];
+        __syncthreads();
+    }
+    // What is left of the triangle: columns w ..
+#pragma unroll
+    for (int c = 0; c < C; ++c)
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+            const int i = lane + 32 * h, j = warp + (w & ~7) + 8 * c;
+            if (j >= w && j <= i && i < m) F[i + j * ld] = a[c][h];
+        }
+    __syncthreads();
+}
+
 // One CTA factorizes a whole front (m <= 96) in shared memory.
 template <class R>
-__global__ void __launch_bounds__(256) k_small_front(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
+constexpr int small_smem(int rows) { return rows * (rows | 1) * static_cast<int>(sizeof(cx<R>)); }
+template <class R>
+__global__ void __launch_bounds__(kLdltThreads) k_small_front(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
                                                      long long lstride, long long cbstride) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    cx<R>* F = reinterpret_cast<cx<R>*>(smem_raw);
+    __shared__ cx<R> inv[96];
+    pdl_start_next();
     const int s = S.items[item0 + blockIdx.x].s;
-    cx<R>* L = Lb + lstride * blockIdx.y;
-    cx<R>* CB = CBb + cbstride * blockIdx.y;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
     const int cs = m - w;
-    cx<R>* Ls = L + S.loff[s];
-    cx<R>* CBs = CB + (cs > 0 ? S.cboff[s] : 0);
-    const int nt = blockDim.x;
-    for (int e = threadIdx.x; e < m * m; e += nt) {
-        const int i = e % m, j = e / m;
-        cx<R> v{0, 0};
-        if (i >= j) v = (j < w) ? Ls[e] : CBs[(i - w) + static_cast<long long>(j - w) * cs];
-        F[e] = v;
-    }
+    const int ld = m | 1;
+    cx<R>* F = reinterpret_cast<cx<R>*>(smem_raw);
+    cx<R>* Ls = Lb + lstride * blockIdx.y + S.loff[s];
+    cx<R>* CBs = CBb + cbstride * blockIdx.y + (cs > 0 ? S.cboff[s] : 0);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    auto at = [&](int i, int j) {
+        return j < w ? Ls + i + static_cast<long long>(j) * m : CBs + (i - w) + static_cast<long long>(j - w) * cs;
+    };
+    pdl_wait();
+#pragma unroll 4
+    for (int j = warp; j < m; j += nw)
+        for (int i = j + lane; i < m; i += 32) F[i + j * ld] = *at(i, j);
     __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = nt >> 5;
-    for (int k = 0; k < w; ++k) {
-        const cx<R> inv = crecip(F[k + k * m]);
-        for (int j = k + 1 + warp; j < m; j += nw) {
-            const cx<R> ljk = F[j + k * m] * inv;
-            for (int i = j + lane; i < m; i += 32) F[i + j * m] = fms(F[i + j * m], F[i + k * m], ljk);
-        }
-        __syncthreads();
-        for (int i = k + 1 + threadIdx.x; i < m; i += nt) F[i + k * m] = F[i + k * m] * inv;
-        __syncthreads();
-    }
-    for (int e = threadIdx.x; e < m * m; e += nt) {
-        const int i = e % m, j = e / m;
-        if (i < j) continue;
-        if (j < w)
-            Ls[e] = F[e];
-        else
-            CBs[(i - w) + static_cast<long long>(j - w) * cs] = F[e];
-    }
+    if (m <= 32)
+        ldlt_columns<1>(F, ld, m, w, inv);
+    else if (m <= 64)
+        ldlt_columns<2>(F, ld, m, w, inv);
+    else
+        ldlt_columns<3>(F, ld, m, w, inv);
+    for (int j = warp; j < m; j += nw)
+        for (int i = j + lane; i < m; i += 32) *at(i, j) = j < w && i > j ? F[i + j * ld] * inv[j] : F[i + j * ld];
 }
 
 // ---------------------------------------------------------------- blocked fronts
-// Step k0 of a large front: factor the kb x kb diagonal block in place. The
-// block is staged with every thread's loads in flight. At step k warp v
-// updates columns k + 1 + v, k + 5 + v, ... and lane l the entry l rows below
-// each column's diagonal (the lower triangle only, no index division); each
-// entry gets the same arithmetic, in the same order of k, as before.
+// A front's panels advance 64 columns a step: the step's diagonal block, the
+// rows below it, then the rest of the panel's own columns.
+
+// Step k0 of a large front: factor the kb x kb diagonal block (kb <= 64) in place.
+constexpr int kDiagThreads = kLdltThreads;
 template <class R>
-__global__ void __launch_bounds__(128) k_diag_block(Sched S, long long item0, cx<R>* Lb, long long lstride) {
-    static_assert(kStep == 32 && kStep * kStep % 128 == 0, "one lane per row, eight entries per thread");
-    __shared__ cx<R> F[kStep * kStep];
+constexpr int diag_smem() { return (kTriSmem + kStep) * static_cast<int>(sizeof(cx<R>)); }
+template <class R>
+__global__ void __launch_bounds__(kDiagThreads) k_diag_block(Sched S, long long item0, cx<R>* Lb, long long lstride) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cx<R>* T = reinterpret_cast<cx<R>*>(smem_raw);
+    cx<R>* inv = T + kTriSmem;  // reciprocals of the pivots
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, k0 = it.a;
-    cx<R>* L = Lb + lstride * blockIdx.y;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
     const int kb = min(kStep, w - k0);
-    cx<R>* D = L + S.loff[s] + k0 + static_cast<long long>(k0) * m;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    {
-        cx<R> v[kStep * kStep / 128];
-#pragma unroll
-        for (int u = 0; u < kStep * kStep / 128; ++u) {
-            const int e = tid + 128 * u, i = e % kStep, j = e / kStep;
-            v[u] = i < kb && j < kb ? D[i + static_cast<long long>(j) * m] : cx<R>{0, 0};
-        }
-#pragma unroll
-        for (int u = 0; u < kStep * kStep / 128; ++u) F[tid + 128 * u] = v[u];
-    }
+    cx<R>* D = Lb + lstride * blockIdx.y + S.loff[s] + k0 + static_cast<long long>(k0) * m;
+    pdl_wait();
+    stage_block(T, D, m, kb, kb);
+    triangle_wait();
     __syncthreads();
-    for (int k = 0; k < kb; ++k) {
-        const cx<R> inv = crecip(F[k + k * kStep]);
-        for (int j = k + 1 + warp; j < kb; j += 4) {
-            const int i = j + lane;
-            if (i < kb) F[i + j * kStep] = fms(F[i + j * kStep], F[i + k * kStep], F[j + k * kStep] * inv);
-        }
-        __syncthreads();
-        for (int i = k + 1 + tid; i < kb; i += blockDim.x) F[i + k * kStep] = F[i + k * kStep] * inv;
-        __syncthreads();
-    }
-#pragma unroll
-    for (int u = 0; u < kStep * kStep / 128; ++u) {
-        const int e = tid + 128 * u, i = e % kStep, j = e / kStep;
-        if (i < kb && j < kb && i >= j) D[i + static_cast<long long>(j) * m] = F[e];
-    }
+    if (kb <= 32)
+        ldlt_columns<1>(T, kTriLd, kb, kb, inv);
+    else
+        ldlt_columns<2>(T, kTriLd, kb, kb, inv);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int j = warp; j < kb; j += kDiagThreads / 32)
+        for (int i = j + lane; i < kb; i += 32)
+            D[i + static_cast<long long>(j) * m] = i > j ? T[i + j * kTriLd] * inv[j] : T[i + j * kTriLd];
 }
 
-// Rows row0 .. row0+127 of the panel below the diagonal block of step k0:
-// L21 = A21 L11^-T D^-1, one row per thread.
+// Rows row0 .. row0 + 63 of the panel below the diagonal block of step k0:
+// L21 = A21 L11^-T D^-1. Four neighbouring lanes take two rows, 32 apart; 16
+// columns at a time, lane q of them holding four (4 u + q) of either row in
+// registers: first the finished columns' products (left-looking, their values
+// in shared memory), then the 16 columns' own chain, each value broadcast to
+// the rows' lanes. Where rows are many, shared memory bounds it: six loads for
+// eight complex multiply-adds (with a row per four lanes five for four: 24^3,
+// eight FP64 entries, 75 us a launch against 63). L11 is kept as its lower triangle by blocks of 16
+// columns, which leaves room for two CTAs per SM (four in FP32).
+constexpr int kTrsmCols = 16, kTrsmThreads = 2 * kTrsmRows;
+// Entry (row, col) of L11, row >= 16 (col / 16): block b's columns are 64 - 16 b long.
+__device__ __forceinline__ int trsm_block(int b) { return kTrsmCols * (kStep * b - kTrsmCols * b * (b - 1) / 2); }
+constexpr int kTrsmTri = kTrsmCols * (64 + 48 + 32 + 16);
 template <class R>
-__global__ void __launch_bounds__(kTrsmRows) k_panel_trsm(Sched S, long long item0, cx<R>* Lb, long long lstride) {
-    __shared__ cx<R> T[kStep * kStep];
-    __shared__ cx<R> Dinv[kStep];
+constexpr int trsm_smem() { return (kTrsmTri + kStep + 48 * (kTrsmRows + 1)) * static_cast<int>(sizeof(cx<R>)); }
+template <class R>
+__global__ void __launch_bounds__(kTrsmThreads) k_panel_trsm(Sched S, long long item0, cx<R>* Lb,
+                                                                 long long lstride) {
+    static_assert(kStep == 64, "four blocks of 16 columns");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cx<R>* T = reinterpret_cast<cx<R>*>(smem_raw);
+    cx<R>* Dinv = T + kTrsmTri;
+    cx<R>* X = Dinv + kStep;  // [column][row]: the rows' finished columns, unscaled
+    constexpr int kLdX = kTrsmRows + 1;
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, k0 = it.a, row0 = it.b;
-    cx<R>* L = Lb + lstride * blockIdx.y;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
     const int kb = min(kStep, w - k0);
-    cx<R>* P = L + S.loff[s] + static_cast<long long>(k0) * m;  // column k0 of the panel
-    for (int e = threadIdx.x; e < kb * kb; e += blockDim.x) {
-        const int i = e % kb, j = e / kb;
-        T[i + j * kStep] = P[k0 + i + static_cast<long long>(j) * m];
+    cx<R>* P = Lb + lstride * blockIdx.y + S.loff[s] + static_cast<long long>(k0) * m;  // column k0 of the panel
+    const int q = threadIdx.x & 3, quad = threadIdx.x & 28, r = threadIdx.x >> 2, i = row0 + r;
+    constexpr int kApart = kTrsmRows / 2;
+    auto load = [&](int c0, cx<R> (&x)[2][4]) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = c0 + 4 * u + q;
+                x[h][u] = i + kApart * h < m && c < kb ? P[i + kApart * h + static_cast<long long>(c) * m] : cx<R>{0, 0};
+            }
+    };
+    pdl_wait();
+#pragma unroll 4
+    for (int e = threadIdx.x; e < kStep * kStep; e += kTrsmThreads) {
+        const int row = e % kStep, col = e / kStep, b = col / kTrsmCols;
+        if (row < b * kTrsmCols) continue;
+        const bool in = row < kb && col < kb;
+        cp_async_entry(smem_u32(T + trsm_block(b) + (row - b * kTrsmCols) + (col % kTrsmCols) * (kStep - b * kTrsmCols)),
+                       in ? P + k0 + row + static_cast<long long>(col) * m : P, in);
+    }
+    cp_async_commit();
+    cx<R> x[2][4], ahead[2][4];
+    load(0, ahead);
+    triangle_wait();
+    __syncthreads();
+    if (threadIdx.x < kb) {
+        const int b = threadIdx.x / kTrsmCols, c = threadIdx.x % kTrsmCols;
+        Dinv[threadIdx.x] = crecip(T[trsm_block(b) + c + c * (kStep - b * kTrsmCols)]);
     }
     __syncthreads();
-    if (threadIdx.x < kb) Dinv[threadIdx.x] = crecip(T[threadIdx.x * (kStep + 1)]);
-    __syncthreads();
-    const int i = row0 + threadIdx.x;
-    if (i >= m) return;
-    cx<R> x[kStep];
+#pragma unroll 1
+    for (int c0 = 0; c0 < kb; c0 += kTrsmCols) {
 #pragma unroll
-    for (int j = 0; j < kStep; ++j)
-        if (j < kb) x[j] = P[i + static_cast<long long>(j) * m];
+        for (int u = 0; u < 4; ++u) x[0][u] = ahead[0][u], x[1][u] = ahead[1][u];
+        if (c0 + kTrsmCols < kb) load(c0 + kTrsmCols, ahead);
+#pragma unroll 1
+        for (int b = 0; b < c0 / kTrsmCols; ++b) {
+            const int ld = kStep - b * kTrsmCols;
+            const cx<R>* Tb = T + trsm_block(b) + (c0 + q - b * kTrsmCols);
+            const cx<R>* Xb = X + b * kTrsmCols * kLdX + r;
+#pragma unroll 4
+            for (int t = 0; t < kTrsmCols; ++t) {
+                const cx<R> v0 = Xb[t * kLdX], v1 = Xb[t * kLdX + kApart];
 #pragma unroll
-    for (int j = 0; j < kStep; ++j) {
-        if (j >= kb) break;
-        cx<R> v = x[j];
-#pragma unroll
-        for (int t = 0; t < kStep; ++t) {
-            if (t >= j) break;
-            v = fms(v, T[j + t * kStep], x[t]);
+                for (int u = 0; u < 4; ++u) {
+                    const cx<R> l = Tb[4 * u + t * ld];
+                    x[0][u] = fms(x[0][u], l, v0);
+                    x[1][u] = fms(x[1][u], l, v1);
+                }
+            }
         }
-        x[j] = v;
-    }
+        const int ld = kStep - c0;
+        const cx<R>* Tc = T + trsm_block(c0 / kTrsmCols) + q;
 #pragma unroll
-    for (int j = 0; j < kStep; ++j)
-        if (j < kb) P[i + static_cast<long long>(j) * m] = x[j] * Dinv[j];
+        for (int j = 0; j < kTrsmCols; ++j) {
+            const int uj = j / 4;
+            cx<R> xj[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                xj[h] = cx<R>{__shfl_sync(0xffffffffu, x[h][uj].re, quad | (j & 3)),
+                              __shfl_sync(0xffffffffu, x[h][uj].im, quad | (j & 3))};
+            const cx<R>* col = Tc + j * ld;
+#pragma unroll
+            for (int u = uj; u < 4; ++u) {
+                const cx<R> l = col[4 * u];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const cx<R> v = fms(x[h][u], l, xj[h]);
+                    if (u > uj || q > (j & 3)) x[h][u] = v;
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int c = c0 + 4 * u + q;
+                if (c < 48) X[c * kLdX + r + kApart * h] = x[h][u];
+                if (i + kApart * h < m && c < kb)
+                    P[i + kApart * h + static_cast<long long>(c) * m] = x[h][u] * Dinv[c];
+            }
+        __syncwarp();  // the row's lanes read one another's columns
+    }
 }
 
 // In-panel update tile (i0, j0) of step k0: F[i, j] -= sum_t L[i,t] D[t] L[j,t]
@@ -280,6 +468,7 @@ __global__ void __launch_bounds__(256) k_update_panel(Sched S, long long item0, 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* As = reinterpret_cast<cx<R>*>(smem_raw);  // [kStep][kTile], scaled by D
     cx<R>* Bs = As + kStep * kTile;                  // [kStep][kTile]
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, k0 = it.a, i0 = it.b, j0 = it.c;
     cx<R>* L = Lb + lstride * blockIdx.y;
@@ -289,6 +478,7 @@ __global__ void __launch_bounds__(256) k_update_panel(Sched S, long long item0, 
     const int cs = m - w;
     const int kb = min(kStep, w - k0);
     const cx<R>* P = L + S.loff[s] + static_cast<long long>(k0) * m;
+    pdl_wait();
     for (int e = threadIdx.x; e < kStep * kTile; e += blockDim.x) {
         const int r = e % kTile, t = e / kTile;
         cx<R> a{0, 0}, b{0, 0};
@@ -529,6 +719,7 @@ __global__ void __launch_bounds__(256, 2) k_i8_split(Sched S, long long item0, c
     constexpr int kWarps = 8;
     __shared__ R dre[kWidePair], dim[kWidePair], up[kWidePair];  // D 2^-h, 2^h
     __shared__ int top[2][kWarps][32];                           // largest sizes of A, B
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, p0 = it.a;
     const int w = S.first[s + 1] - S.first[s];
@@ -542,6 +733,7 @@ __global__ void __launch_bounds__(256, 2) k_i8_split(Sched S, long long item0, c
     const int r = it.b + 32 * blockIdx.z + lane;  // row within the trailing part
     const bool in = pe + r < m;
     const cx<R>* X = P + (in ? pe + r : pe) + static_cast<long long>(p0) * m;
+    pdl_wait();
     for (int k = threadIdx.x; k < kWidePair; k += 256) {
         const cx<R> d = k < K ? P[(p0 + k) + static_cast<long long>(p0 + k) * m] : cx<R>{0, 0};
         const int e = max(Real::exponent(Real::size(d.re)), Real::exponent(Real::size(d.im)));
@@ -696,6 +888,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(slots + kSlots);
     volatile int* state = reinterpret_cast<volatile int*>(tmem_slot + 1);  // [0] failed, [1] stages committed, [2] stages loaded
     static_assert((2 * C::Stages + 2 + kSlots) * 8 + kSlots * sizeof(Tile) + 16 <= C::extra, "barriers and slots");
+    pdl_start_next();
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
@@ -719,6 +912,7 @@ __global__ void __launch_bounds__(kI8Threads, 1) k_update_i8(Sched S, long long 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = *tmem_slot;
+    pdl_wait();
     // Tile n of this CTA once the producer has decoded it; false: failed.
     auto tile = [&](int n, Tile& t) {
         if (!mbar_wait_live(smem_u32(ready + n % kSlots), (n / kSlots) & 1, state)) return false;
@@ -890,6 +1084,7 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<double>* Ds = reinterpret_cast<cx<double>*>(smem_raw);  // [kWidePair] pivots of the group's panels
     cx<double>* Ring = Ds + kWidePair;                           // [stage][A: KC x ldA | B: KC x ldB]
+    pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, p0 = it.a, i0 = it.b, j0 = it.c;
     cx<double>* L = Lb + lstride * blockIdx.y;
@@ -933,6 +1128,7 @@ __global__ void __launch_bounds__(256) k_update_wide_dmma(Sched S, long long ite
 #pragma unroll
         for (int b = 0; b < 4; ++b) cr[a][b][0] = cr[a][b][1] = ci[a][b][0] = ci[a][b][1] = 0.0;
     const int nc = (K + kDmmaKC - 1) / kDmmaKC;
+    pdl_wait();
     fetch(0);
     cp_async_commit();
     if (nc > 1) fetch(1);
@@ -1236,50 +1432,14 @@ __device__ __forceinline__ int solve_nblocks(const Sched& S, int s) {
     return (S.first[s + 1] - S.first[s] + kSolveBlock - 1) / kSolveBlock;
 }
 
-// A solve is a chain of short launches, each of which needs the one before it
-// for a few vectors only: its items, schedule and panel entries are constants.
-// So the solve kernels are launched with programmatic stream serialization: a
-// kernel lets the next one start as it begins itself (pdl_start_next), which
-// then reads its constants and waits (pdl_wait) until the kernel before it has
-// finished and its writes are visible. Everything that a launch before could
-// have written, or still reads where this one writes, comes after pdl_wait();
-// every solve kernel calls it, so that the wait covers all launches before.
-__device__ __forceinline__ void pdl_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Shared memory of the solve kernels that hold a 64 x 64 block of L, with
 // leading dimension kTriLd (65: column-strided reads fall in distinct banks),
 // and for the backward triangle the partial-sum reduction's kRedGroups
 // sub-sums per (column, rhs).
-constexpr int kTriLd = kSolveBlock + 1;
-constexpr int kTriSmem = kSolveBlock * kTriLd;     // complex entries
 constexpr int kRedGroups = 8;
 constexpr int kBwdDiagThreads = 512;
 constexpr int red_smem(int nr) { return kRedGroups * kSolveBlock * nr; }  // complex entries
 constexpr int kGatherRows = 512;                   // front rows per gather CTA
-
-// A block of L (rows x cols at P, leading dimension m) into shared memory T
-// (leading dimension kTriLd, zeros outside the rows x cols block) by
-// asynchronous copies (cp.async, zero-filled where the source size is 0), so
-// the caller's own loads overlap them; the caller waits with
-// triangle_wait() and a __syncthreads() before reading T.
-__device__ __forceinline__ void cp_async_entry(uint32_t dst, const cx<double>* src, bool in) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16u : 0u) : "memory");
-}
-__device__ __forceinline__ void cp_async_entry(uint32_t dst, const cx<float>* src, bool in) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(in ? 8u : 0u) : "memory");
-}
-template <class R>
-__device__ __forceinline__ void stage_block(cx<R>* T, const cx<R>* P, long long m, int rows, int cols) {
-#pragma unroll 4
-    for (int e = threadIdx.x; e < kSolveBlock * kSolveBlock; e += blockDim.x) {
-        const int i = e % kSolveBlock, j = e / kSolveBlock;
-        const bool in = i < rows && j < cols;
-        cp_async_entry(smem_u32(T + i + j * kTriLd), in ? P + i + static_cast<long long>(j) * m : P, in);
-    }
-    cp_async_commit();
-}
-__device__ __forceinline__ void triangle_wait() { cp_async_wait<0>(); }
 
 // Forward triangle of block blk of supernode s: y[blk] = L_bb^-1 y[blk] for
 // the pass's rhs, one warp per rhs, L_bb staged in shared memory (smem:

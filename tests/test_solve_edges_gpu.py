@@ -47,3 +47,31 @@ def test_solves_match_numpy(precision, tol, n, cuda):
         part = f.solve(torch.from_numpy(np.ascontiguousarray(b[:, :k])).cuda()).cpu().numpy()
         np.testing.assert_array_equal(part, got[:, :k])
     f.close()
+
+
+@pytest.mark.parametrize("small_front", [96, 8])
+@pytest.mark.parametrize("n", [2, 8, 9, 31, 32, 33, 63, 64, 65, 95, 96, 97, 127, 128, 129, 191, 193])
+def test_dense_factors_reconstruct(n, small_front, cuda):
+    """One dense front of n rows through the one-CTA and the blocked kernels:
+    L D L^T is the matrix to n eps of its largest entry (its growth is below
+    2: diagonally dominant), multipliers and pivots match a host LDL^T."""
+    rng = np.random.default_rng([n, small_front])
+    a = dense_and_tails(n, 0, rng)
+    r, c = np.nonzero(np.triu(a))
+    rp = np.concatenate([[0], np.cumsum(np.bincount(r, minlength=n))]).astype(np.int32)
+    o = ab.default_analysis_options()
+    o.small_front = small_front
+    an = ab.Analysis(rp, c.astype(np.int32), np.arange(n, dtype=np.int32), options=o)
+    f = ab.Factor(an)
+    assert f.factorize(torch.from_numpy(a[r, c]).cuda().unsqueeze(0), 0)
+    e = f.export()
+    low, host = np.eye(n, dtype=np.complex128), a.copy()
+    for j in range(n):
+        t = slice(e["col_ptr"][j], e["col_ptr"][j + 1])
+        low[e["row_index"][t], j] = e["value"][t]
+        host[j + 1:, j] /= host[j, j]
+        host[j + 1:, j + 1:] -= np.outer(host[j + 1:, j] * host[j, j], host[j + 1:, j])
+    assert np.abs((low * e["diagonal"]) @ low.T - a).max() <= 2.3e-16 * 4 * n * np.abs(a).max()
+    np.testing.assert_allclose(e["diagonal"], np.diag(host), rtol=1e-12)
+    assert np.abs(np.tril(low, -1) - np.tril(host, -1)).max() <= 1e-12
+    f.close()
