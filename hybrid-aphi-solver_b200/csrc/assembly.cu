@@ -8,20 +8,25 @@
 //
 // Design. The reference accumulates `values[slot] += term` while it walks
 // bodies -> tets -> (AA, A-Phi/Phi-A, Phi-Phi) blocks. Here
-//   K1 (k_tet_terms): one warp per tet, for every frequency of the batch,
-//       stages the tet's tables and its frequency-independent geometry
-//       (barycentric gradients, curls, Whitney values and P2 gradients at the
-//       quadrature points) in shared memory, enumerates the tet's terms in
-//       the reference's emission order, and computes (term, frequency) pairs
-//       across its lanes -- each already scaled exactly as the reference forms
-//       the addend -- into a term array, stored frequency-minor. Terms bound
-//       for the right-hand side are stored negated (the reference subtracts
-//       them).
+//   K1 (k_tet_terms): the tets' geometry, one thread a tet, then one warp per
+//       tet, for every frequency of the batch: it enumerates the tet's terms in
+//       the reference's emission order, forms for each what does not depend on
+//       the frequency (the four quadrature points' integrands, the stiffness
+//       entry, the DOF coefficients' product), and computes (term, frequency)
+//       pairs across its lanes -- each already scaled exactly as the reference
+//       forms the addend -- into a term array, stored frequency-minor. Terms
+//       bound for the right-hand side are stored negated (the reference
+//       subtracts them).
 //   K2 (k_slot_sum): one thread per (destination, frequency) -- CSR slot or
 //       rhs row -- sums its terms in increasing term order through a slot ->
 //       term list built once per mesh. Increasing term order IS the
 //       reference's accumulation order, so the sums are bitwise those of the
 //       reference: no float atomics, no order that depends on scheduling.
+// (Writing the frequency-independent part only, 64 bytes a term, and forming
+// the values in K2 moves half the bytes but was slower: dependent uncontracted
+// FP64 operations by slots of one to 24 terms side by side took 1.15 ms for 16
+// frequencies of 32^3, where K2 takes 0.6 and the values cost K1 0.25; 34 us
+// against 5 on the 8^3 mesh.)
 // This file is compiled with -fmad=false and uses explicitly rounded
 // intrinsics for complex products, so every element entry and every addend is
 // rounded exactly as the host's std::complex<double> arithmetic rounds it.
@@ -357,229 +362,41 @@ __device__ __forceinline__ bool tet_geometry_reg(const double (&p)[4][3], double
 // (Phi,Phi) or its prescribed-Phi rhs term.
 enum : int { T_AA = 0, T_AP = 1, T_AP_FIXED = 2, T_PA = 3, T_PP = 4, T_PP_FIXED = 5 };
 
-constexpr int kTetWarps = 4;          // tets (warps) per block
+constexpr int kTetWarps = 8;          // warps per block
 constexpr int kTetMaxTerms = 256;     // 36 + 120 + 100 at most (full storage)
 
-// Per-warp staging: the tet's tables, geometry and the frequency-independent
-// vectors of its element blocks (curls; Whitney values and P2 gradients at
-// the four quadrature points), and its term list.
+// A term without its frequency: the integrands at the four quadrature points
+// times their weight; the stiffness entry (A, A) or a prescribed value; the
+// product of the DOF coefficients (one of them beside a prescribed value).
+struct TermParts {
+    double s[4], a, im, p;
+    int kind;
+};
+
+// Per-warp staging: the tet's tables and the vectors of its element blocks
+// (curls; Whitney values and P2 gradients at the four quadrature points), its
+// term list, 32 terms' parts and the body's coefficients per frequency.
 struct TetStage {
-    double grad[4][3];
     double curl[6][3];
     double wv[4][6][3];
     double gr[4][10][3];
     double fixed[10][2];
     double co[16];
-    double p[4][3];
-    double mat[3];
-    double volume;
+    TermParts parts[32];
     int idx[16];
     unsigned short rec[kTetMaxTerms];  // kind << 8 | i << 4 | j
-    // per frequency of the batch: the body's coefficients and the scalings
-    Coeff cf[kMaxBatchOmegas];
-    cplx col[kMaxBatchOmegas], rjw[kMaxBatchOmegas], rc[kMaxBatchOmegas];
+};
+// Per block: the tets' geometry, and behind it per frequency the formulation's
+// scalings and, for every warp, its body's coefficients.
+template <int Tets>
+struct TetBlock {
+    double grad[Tets][4][3];
+    double vol[Tets];  // negative: degenerate
+    TetStage stage[kTetWarps];
+    static int bytes(int nf) { return static_cast<int>(sizeof(TetBlock) + sizeof(cplx) * nf * (3 + 2 * kTetWarps)); }
 };
 
 __device__ __forceinline__ double dot3s(const double* u, const double* v) { return dot3(u, v); }
-
-// K1: one warp per tet (in the reference's body -> tet visit order), all the
-// batch's frequencies. The warp stages the tet once, enumerates its terms in
-// the reference's emission order (a warp scan over the 36 + 60 + 100 block
-// positions), then computes (term, frequency) pairs across its lanes: each
-// pair's element entry is rebuilt from the staged vectors with the reference's
-// accumulation over the quadrature points, and scaled exactly as the reference
-// forms its addend. Terms are stored frequency-minor, terms[t * nf + f], so a
-// warp's stores are contiguous and the slot sums read 16 * nf contiguous
-// bytes per term.
-__global__ void __launch_bounds__(32 * kTetWarps) k_tet_terms(TetArgs A, Omegas om, int cond, Quad quad,
-                                                              cplx* terms) {
-    __shared__ TetStage stage[kTetWarps];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int v = blockIdx.x * kTetWarps + warp;
-    if (v >= A.num_tets) return;  // uniform per warp
-    TetStage& S = stage[warp];
-    const int t = A.visit_tet[v];
-    const int b = A.visit_body[v];
-    if (lane < 16) {
-        S.idx[lane] = A.tet_idx[16LL * t + lane];
-        S.co[lane] = A.tet_coeff[16LL * t + lane];
-    }
-    if (lane < 20) (&S.fixed[0][0])[lane] = A.tet_fixed[20LL * t + lane];
-    if (lane < 12) S.p[lane / 3][lane % 3] = A.xyz[3LL * A.tets[4LL * t + lane / 3] + lane % 3];
-    if (lane < 3) S.mat[lane] = A.material[3 * b + lane];
-    __syncwarp();
-    const bool fixed_lane = lane < 10 && !(S.fixed[lane][0] == 0.0 && S.fixed[lane][1] == 0.0);
-    const unsigned fixed_mask = __ballot_sync(0xffffffffu, fixed_lane);
-    const bool need_phi = __ballot_sync(0xffffffffu, lane < 10 && (S.idx[6 + lane] >= 0 || fixed_lane)) != 0;
-
-    // Geometry: every lane computes it (uniform control flow); lane 0 stages it.
-    {
-        double p[4][3], grad[4][3], vol;
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int k = 0; k < 3; ++k) p[r][k] = S.p[r][k];
-        if (!tet_geometry_reg(p, grad, vol)) {
-            if (lane == 0) atomicExch(&A.err[0], 1);
-            return;
-        }
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int k = 0; k < 3; ++k) S.grad[r][k] = grad[r][k];
-            S.volume = vol;
-        }
-    }
-    __syncwarp();
-    // Curls (6), Whitney values (4 points x 6 edges), P2 gradients (4 x 10).
-    const int nvec = need_phi ? 70 : 30;
-    for (int it = lane; it < nvec; it += 32) {
-        if (it < 6) {
-            const double* u = S.grad[c_edge_verts[it][0]];
-            const double* w = S.grad[c_edge_verts[it][1]];
-            S.curl[it][0] = __dmul_rn(__dsub_rn(__dmul_rn(u[1], w[2]), __dmul_rn(u[2], w[1])), 2.0);
-            S.curl[it][1] = __dmul_rn(__dsub_rn(__dmul_rn(u[2], w[0]), __dmul_rn(u[0], w[2])), 2.0);
-            S.curl[it][2] = __dmul_rn(__dsub_rn(__dmul_rn(u[0], w[1]), __dmul_rn(u[1], w[0])), 2.0);
-        } else {
-            const int q = it < 30 ? (it - 6) / 6 : (it - 30) / 10;
-            // barycentric coordinate i of quadrature point q: (a, b, b, b) permuted
-            auto L = [&](int i) { return i == q ? quad.a : quad.b; };
-            if (it < 30) {
-                const int e = (it - 6) % 6;
-                const int vi = c_edge_verts[e][0], vj = c_edge_verts[e][1];
-#pragma unroll
-                for (int k = 0; k < 3; ++k)
-                    S.wv[q][e][k] = __dsub_rn(__dmul_rn(S.grad[vj][k], L(vi)), __dmul_rn(S.grad[vi][k], L(vj)));
-            } else {
-                const int bb = (it - 30) % 10;
-                if (bb < 4) {
-                    const double sc = __dsub_rn(__dmul_rn(4.0, L(bb)), 1.0);
-#pragma unroll
-                    for (int k = 0; k < 3; ++k) S.gr[q][bb][k] = __dmul_rn(S.grad[bb][k], sc);
-                } else {
-                    const int v0 = c_edge_verts[bb - 4][0], v1 = c_edge_verts[bb - 4][1];
-                    const double s0 = __dmul_rn(4.0, L(v1)), s1 = __dmul_rn(4.0, L(v0));
-#pragma unroll
-                    for (int k = 0; k < 3; ++k)
-                        S.gr[q][bb][k] = __dadd_rn(__dmul_rn(S.grad[v0][k], s0), __dmul_rn(S.grad[v1][k], s1));
-                }
-            }
-        }
-    }
-    // The tet's terms in emission order: block positions AA (36), then
-    // (A,Phi) pairs (60, up to two terms each) and (Phi,Phi) (100).
-    const bool up = A.upper_only != 0;
-    const int ncand = need_phi ? 196 : 36;
-    int total = 0;
-    for (int c0 = 0; c0 < ncand; c0 += 32) {
-        const int c = c0 + lane;
-        int n = 0, r0 = 0, r1 = 0;
-        if (c < 36) {
-            const int pi = c / 6, qi = c % 6;
-            if (S.idx[pi] >= 0 && S.idx[qi] >= 0 && !(up && S.idx[qi] < S.idx[pi])) {
-                n = 1;
-                r0 = T_AA << 8 | pi << 4 | qi;
-            }
-        } else if (c < 96) {
-            const int pi = (c - 36) / 10, qi = (c - 36) % 10;
-            const int row = S.idx[pi], col = S.idx[6 + qi];
-            if (row >= 0) {
-                if (col >= 0) {
-                    if (!(up && col < row)) r0 = T_AP << 8 | pi << 4 | qi, n = 1;
-                    if (!(up && row < col)) (n ? r1 : r0) = T_PA << 8 | pi << 4 | qi, ++n;
-                } else if ((fixed_mask >> qi) & 1u) {
-                    r0 = T_AP_FIXED << 8 | pi << 4 | qi;
-                    n = 1;
-                }
-            }
-        } else if (c < 196) {
-            const int pi = (c - 96) / 10, qi = (c - 96) % 10;
-            const int row = S.idx[6 + pi], col = S.idx[6 + qi];
-            if (row >= 0) {
-                if (col >= 0) {
-                    if (!(up && col < row)) r0 = T_PP << 8 | pi << 4 | qi, n = 1;
-                } else if ((fixed_mask >> qi) & 1u) {
-                    r0 = T_PP_FIXED << 8 | pi << 4 | qi;
-                    n = 1;
-                }
-            }
-        }
-        int incl = n;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const int at = total + incl - n;
-        if (n > 0) S.rec[at] = static_cast<unsigned short>(r0);
-        if (n > 1) S.rec[at + 1] = static_cast<unsigned short>(r1);
-        total += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    const long long off = A.term_off[v];
-    if (total != A.term_off[v + 1] - off) {
-        if (lane == 0) atomicExch(&A.err[1], 1);
-        return;
-    }
-    __syncwarp();
-    const int nf = om.n;
-    // The body's coefficients and the formulation's scalings, once per
-    // frequency (they hold divisions), for every term of the tet.
-    for (int f = lane; f < nf; f += 32) {
-        const double omega = om.w[f];
-        S.cf[f] = body_coefficients(S.mat[0], S.mat[1], S.mat[2], omega);
-        const Scales sc = scales_of(cond, omega);
-        S.col[f] = sc.col;
-        S.rjw[f] = cmul_exact(sc.row, sc.jw);
-        S.rc[f] = cmul_exact(sc.row, sc.col);
-    }
-    __syncwarp();
-    const double vol = S.volume;
-    const double w = __dmul_rn(0.25, vol);
-    cplx* out = terms + off * nf;
-    for (int it = lane; it < total * nf; it += 32) {
-        const int k = it / nf, f = it - k * nf;
-        const int r = S.rec[k];
-        const int kind = r >> 8, i = (r >> 4) & 15, j = r & 15;
-        const Coeff& c = S.cf[f];
-        cplx blk{0.0, 0.0};
-        if (kind == T_AA) {
-            // kernel_AA: nu V curl.curl, then the mass term point by point.
-            blk = cplx{__dmul_rn(__dmul_rn(c.nu, vol), dot3s(S.curl[i], S.curl[j])), 0.0};
-            if (!(c.alpha.re == 0.0 && c.alpha.im == 0.0))
-#pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    blk = cadd_exact(blk, cscale_exact(c.alpha, __dmul_rn(w, dot3s(S.wv[q][i], S.wv[q][j]))));
-        } else if (!(c.beta.re == 0.0 && c.beta.im == 0.0)) {
-            // kernel_APhi / kernel_PhiPhi
-            const bool pp = kind >= T_PP;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const double* u = pp ? S.gr[q][i] : S.wv[q][i];
-                blk = cadd_exact(blk, cscale_exact(c.beta, __dmul_rn(w, dot3s(u, S.gr[q][j]))));
-            }
-        }
-        const cplx col = S.col[f];
-        cplx term;
-        switch (kind) {
-            case T_AA: term = cscale_exact(blk, __dmul_rn(S.co[i], S.co[j])); break;
-            case T_AP: term = cmul_exact(cscale_exact(col, __dmul_rn(S.co[i], S.co[6 + j])), blk); break;
-            case T_AP_FIXED: {
-                const cplx fx = cdiv_smith(cplx{S.fixed[j][0], S.fixed[j][1]}, col);
-                term = cneg(cmul_exact(cmul_exact(cscale_exact(col, S.co[i]), blk), fx));
-                break;
-            }
-            case T_PA: term = cmul_exact(cscale_exact(S.rjw[f], __dmul_rn(S.co[6 + j], S.co[i])), blk); break;
-            case T_PP: term = cmul_exact(cscale_exact(S.rc[f], __dmul_rn(S.co[6 + i], S.co[6 + j])), blk); break;
-            default: {
-                const cplx fx = cdiv_smith(cplx{S.fixed[j][0], S.fixed[j][1]}, col);
-                term = cneg(cmul_exact(cmul_exact(cscale_exact(S.rc[f], S.co[6 + i]), blk), fx));
-                break;
-            }
-        }
-        out[it] = term;
-    }
-}
 
 struct PortArgs {
     int num_ports;
@@ -591,19 +408,244 @@ struct PortArgs {
 
 // Port rows, src/assembly.cpp:396-421: a voltage port's unit diagonal and
 // rhs V / c; a current port's rhs r * I. One thread per frequency.
-__global__ void k_port_terms(PortArgs P, Omegas om, int cond, cplx* terms) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ void port_terms(const PortArgs& P, const Omegas& om, int cond, cplx* terms) {
     const int nf = om.n;
-    if (f >= nf) return;
-    const Scales sc = scales_of(cond, om.w[f]);
-    cplx* out = terms + P.first_term * nf + f;
-    long long k = 0;
-    for (int p = 0; p < P.num_ports; ++p) {
-        if (P.current[p]) {
-            out[nf * k++] = cmul_exact(sc.row, cplx{P.amplitude[2 * p], P.amplitude[2 * p + 1]});
+    for (int f = threadIdx.x; f < nf; f += blockDim.x) {
+        const Scales sc = scales_of(cond, om.w[f]);
+        cplx* out = terms + P.first_term * nf + f;
+        long long k = 0;
+        for (int p = 0; p < P.num_ports; ++p) {
+            if (P.current[p]) {
+                out[nf * k++] = cmul_exact(sc.row, cplx{P.amplitude[2 * p], P.amplitude[2 * p + 1]});
+            } else {
+                out[nf * k++] = cplx{1.0, 0.0};
+                out[nf * k++] = cdiv_smith(cplx{P.value[2 * p], P.value[2 * p + 1]}, sc.col);
+            }
+        }
+    }
+}
+
+// K1. Block b takes 8 Rounds tets (in the reference's body -> tet visit
+// order): their geometry by its first threads, one a tet -- on a whole warp
+// per tet the inverse's divisions alone took more than half of the kernel --
+// then tet by tet a warp stages the vectors, enumerates the terms in the
+// reference's emission order (a ballot scan over the 36 + 60 + 100 block
+// positions) and computes (term, frequency) pairs across its lanes. Terms are
+// stored frequency-minor, terms[t * nf + f], so a warp's stores are contiguous
+// and the slot sums read 16 * nf contiguous bytes per term. One block more
+// writes the ports' terms. 16 frequencies of 32^3: 0.68 ms (1.23 with the
+// geometry on a warp and the integrands formed again for every frequency), of
+// which the term array's writes take 0.23.
+template <int Rounds>
+__global__ void __launch_bounds__(32 * kTetWarps) k_tet_terms(TetArgs A, PortArgs P, Omegas om, int cond, Quad quad,
+                                                              cplx* terms) {
+    constexpr int kTets = kTetWarps * Rounds;
+    static_assert(kTets <= 32, "one warp's threads take the geometry");
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    auto& B = *reinterpret_cast<TetBlock<kTets>*>(smem_raw);
+    cplx* const f_col = reinterpret_cast<cplx*>(smem_raw + sizeof(TetBlock<kTets>));
+    cplx* const f_rjw = f_col + om.n;
+    cplx* const f_rc = f_rjw + om.n;
+    pdl_start_next();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (blockIdx.x == gridDim.x - 1) {
+        port_terms(P, om, cond, terms);
+        return;
+    }
+    const int nf = om.n;
+    const int v0 = blockIdx.x * kTets;
+    if (threadIdx.x < kTets && v0 + static_cast<int>(threadIdx.x) < A.num_tets) {
+        const int t = A.visit_tet[v0 + threadIdx.x];
+        double p[4][3], grad[4][3], vol;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int node = A.tets[4LL * t + r];
+#pragma unroll
+            for (int k = 0; k < 3; ++k) p[r][k] = A.xyz[3LL * node + k];
+        }
+        const bool ok = tet_geometry_reg(p, grad, vol);
+        B.vol[threadIdx.x] = ok ? vol : -1.0;
+        if (ok) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int k = 0; k < 3; ++k) B.grad[threadIdx.x][r][k] = grad[r][k];
         } else {
-            out[nf * k++] = cplx{1.0, 0.0};
-            out[nf * k++] = cdiv_smith(cplx{P.value[2 * p], P.value[2 * p + 1]}, sc.col);
+            atomicExch(&A.err[0], 1);
+        }
+    }
+    // The formulation's scalings (they hold divisions), by the last warps.
+    for (int f = static_cast<int>(blockDim.x) - 1 - static_cast<int>(threadIdx.x); f < nf; f += blockDim.x) {
+        const Scales sc = scales_of(cond, om.w[f]);
+        f_col[f] = sc.col;
+        f_rjw[f] = cmul_exact(sc.row, sc.jw);
+        f_rc[f] = cmul_exact(sc.row, sc.col);
+    }
+    __syncthreads();
+    TetStage& S = B.stage[warp];
+    cplx* const f_alpha = f_rc + nf + 2 * nf * warp;
+    cplx* const f_beta = f_alpha + nf;
+    const int step_k = 32 / nf, step_f = 32 - step_k * nf;
+#pragma unroll 1
+    for (int round = 0; round < Rounds; ++round) {
+        const int at_tet = round * kTetWarps + warp, v = v0 + at_tet;
+        if (v >= A.num_tets) return;  // uniform per warp; no barrier follows
+        const double vol = B.vol[at_tet];
+        if (vol < 0.0) continue;
+        const double(*grad)[3] = B.grad[at_tet];
+        const int t = A.visit_tet[v];
+        const int b = A.visit_body[v];
+        __syncwarp();
+        if (lane < 16) {
+            S.idx[lane] = A.tet_idx[16LL * t + lane];
+            S.co[lane] = A.tet_coeff[16LL * t + lane];
+        }
+        if (lane < 20) (&S.fixed[0][0])[lane] = A.tet_fixed[20LL * t + lane];
+        const double mat_sigma = A.material[3 * b], mat_eps = A.material[3 * b + 1], mat_mu = A.material[3 * b + 2];
+        const long long off = A.term_off[v], planned = A.term_off[v + 1] - off;
+        for (int f = lane; f < nf; f += 32) {
+            const Coeff c = body_coefficients(mat_sigma, mat_eps, mat_mu, om.w[f]);
+            f_alpha[f] = c.alpha;
+            f_beta[f] = c.beta;
+        }
+        __syncwarp();
+        const bool fixed_lane = lane < 10 && !(S.fixed[lane][0] == 0.0 && S.fixed[lane][1] == 0.0);
+        const unsigned fixed_mask = __ballot_sync(0xffffffffu, fixed_lane);
+        const bool need_phi = __ballot_sync(0xffffffffu, lane < 10 && (S.idx[6 + lane] >= 0 || fixed_lane)) != 0;
+        // Curls (6), Whitney values (4 points x 6 edges), P2 gradients (4 x 10).
+        const int nvec = need_phi ? 70 : 30;
+        for (int it = lane; it < nvec; it += 32) {
+            if (it < 6) {
+                const double* u = grad[c_edge_verts[it][0]];
+                const double* w = grad[c_edge_verts[it][1]];
+                S.curl[it][0] = __dmul_rn(__dsub_rn(__dmul_rn(u[1], w[2]), __dmul_rn(u[2], w[1])), 2.0);
+                S.curl[it][1] = __dmul_rn(__dsub_rn(__dmul_rn(u[2], w[0]), __dmul_rn(u[0], w[2])), 2.0);
+                S.curl[it][2] = __dmul_rn(__dsub_rn(__dmul_rn(u[0], w[1]), __dmul_rn(u[1], w[0])), 2.0);
+            } else {
+                const int q = it < 30 ? (it - 6) / 6 : (it - 30) / 10;
+                // barycentric coordinate i of quadrature point q: (a, b, b, b) permuted
+                auto L = [&](int i) { return i == q ? quad.a : quad.b; };
+                if (it < 30) {
+                    const int e = (it - 6) % 6;
+                    const int vi = c_edge_verts[e][0], vj = c_edge_verts[e][1];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k)
+                        S.wv[q][e][k] = __dsub_rn(__dmul_rn(grad[vj][k], L(vi)), __dmul_rn(grad[vi][k], L(vj)));
+                } else {
+                    const int bb = (it - 30) % 10;
+                    if (bb < 4) {
+                        const double sc = __dsub_rn(__dmul_rn(4.0, L(bb)), 1.0);
+#pragma unroll
+                        for (int k = 0; k < 3; ++k) S.gr[q][bb][k] = __dmul_rn(grad[bb][k], sc);
+                    } else {
+                        const int e0 = c_edge_verts[bb - 4][0], e1 = c_edge_verts[bb - 4][1];
+                        const double s0 = __dmul_rn(4.0, L(e1)), s1 = __dmul_rn(4.0, L(e0));
+#pragma unroll
+                        for (int k = 0; k < 3; ++k)
+                            S.gr[q][bb][k] = __dadd_rn(__dmul_rn(grad[e0][k], s0), __dmul_rn(grad[e1][k], s1));
+                    }
+                }
+            }
+        }
+        // The tet's terms in emission order: block positions AA (36), then
+        // (A,Phi) pairs (60, up to two terms each) and (Phi,Phi) (100).
+        const bool up = A.upper_only != 0;
+        const int ncand = need_phi ? 196 : 36;
+        const unsigned before = (1u << lane) - 1u;
+        int total = 0;
+        for (int c0 = 0; c0 < ncand; c0 += 32) {
+            const int c = c0 + lane;
+            int n = 0, r0 = 0, r1 = 0;
+            if (c < 36) {
+                const int pi = c / 6, qi = c % 6;
+                if (S.idx[pi] >= 0 && S.idx[qi] >= 0 && !(up && S.idx[qi] < S.idx[pi])) {
+                    n = 1;
+                    r0 = T_AA << 8 | pi << 4 | qi;
+                }
+            } else if (c < min(96, ncand)) {
+                const int pi = (c - 36) / 10, qi = (c - 36) % 10;
+                const int row = S.idx[pi], col = S.idx[6 + qi];
+                if (row >= 0) {
+                    if (col >= 0) {
+                        if (!(up && col < row)) r0 = T_AP << 8 | pi << 4 | qi, n = 1;
+                        if (!(up && row < col)) (n ? r1 : r0) = T_PA << 8 | pi << 4 | qi, ++n;
+                    } else if ((fixed_mask >> qi) & 1u) {
+                        r0 = T_AP_FIXED << 8 | pi << 4 | qi;
+                        n = 1;
+                    }
+                }
+            } else if (c < ncand) {
+                const int pi = (c - 96) / 10, qi = (c - 96) % 10;
+                const int row = S.idx[6 + pi], col = S.idx[6 + qi];
+                if (row >= 0) {
+                    if (col >= 0) {
+                        if (!(up && col < row)) r0 = T_PP << 8 | pi << 4 | qi, n = 1;
+                    } else if ((fixed_mask >> qi) & 1u) {
+                        r0 = T_PP_FIXED << 8 | pi << 4 | qi;
+                        n = 1;
+                    }
+                }
+            }
+            const unsigned one = __ballot_sync(0xffffffffu, n > 0), two = __ballot_sync(0xffffffffu, n > 1);
+            const int at = total + __popc(one & before) + __popc(two & before);
+            if (n > 0) S.rec[at] = static_cast<unsigned short>(r0);
+            if (n > 1) S.rec[at + 1] = static_cast<unsigned short>(r1);
+            total += __popc(one) + __popc(two);
+        }
+        if (total != planned) {
+            if (lane == 0) atomicExch(&A.err[1], 1);
+            continue;
+        }
+        __syncwarp();
+        const double w = __dmul_rn(0.25, vol);
+        const double nv = __dmul_rn(body_coefficients(mat_sigma, mat_eps, mat_mu, 0.0).nu, vol);
+        for (int k0 = 0; k0 < total; k0 += 32) {
+            const int cnt = min(32, total - k0);
+            if (lane < cnt) {
+                const int r = S.rec[k0 + lane];
+                const int kind = r >> 8, i = (r >> 4) & 15, j = r & 15;
+                TermParts& T = S.parts[lane];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const double* x = kind >= T_PP ? S.gr[q][i] : S.wv[q][i];
+                    const double* y = kind == T_AA ? S.wv[q][j] : S.gr[q][j];
+                    T.s[q] = __dmul_rn(w, dot3s(x, y));
+                }
+                T.a = kind == T_AA ? __dmul_rn(nv, dot3s(S.curl[i], S.curl[j])) : S.fixed[j][0];
+                T.im = kind == T_AA ? 0.0 : S.fixed[j][1];
+                const double ci = S.co[kind >= T_PP ? 6 + i : i], cj = S.co[kind == T_AA ? j : 6 + j];
+                T.p = kind == T_AP_FIXED || kind == T_PP_FIXED ? ci : __dmul_rn(ci, cj);
+                T.kind = kind;
+            }
+            __syncwarp();
+            cplx* out = terms + (off + k0) * nf;
+            int k = lane / nf, f = lane - k * nf;
+            for (int it = lane; it < cnt * nf; it += 32) {
+                const TermParts& T = S.parts[k];
+                const int kind = T.kind;
+                const bool aa = kind == T_AA;
+                // kernel_AA: nu V curl.curl, then the mass term point by point;
+                // kernel_APhi / kernel_PhiPhi: the points alone.
+                const cplx c = aa ? f_alpha[f] : f_beta[f];
+                cplx blk{aa ? T.a : 0.0, 0.0};
+                if (!(c.re == 0.0 && c.im == 0.0))
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) blk = cadd_exact(blk, cscale_exact(c, T.s[q]));
+                cplx term;
+                if (aa) {
+                    term = cscale_exact(blk, T.p);
+                } else {
+                    const cplx sc = kind <= T_AP_FIXED ? f_col[f] : (kind == T_PA ? f_rjw[f] : f_rc[f]);
+                    term = cmul_exact(cscale_exact(sc, T.p), blk);
+                    if (kind == T_AP_FIXED || kind == T_PP_FIXED)
+                        term = cneg(cmul_exact(term, cdiv_smith(cplx{T.a, T.im}, f_col[f])));
+                }
+                out[it] = term;
+                k += step_k;
+                f += step_f;
+                if (f >= nf) f -= nf, ++k;
+            }
+            __syncwarp();
         }
     }
 }
@@ -611,34 +653,52 @@ __global__ void k_port_terms(PortArgs P, Omegas om, int cond, cplx* terms) {
 // K2: fixed-order sum of each destination's terms (increasing term index,
 // the reference's accumulation order), for every frequency of the batch.
 // Thread (slot, frequency) with the frequency fastest, so one term's nf
-// values are read as one contiguous run; the sums are transposed through
-// shared memory so that each frequency's values are written as a contiguous
-// run of slots.
+// values are read as one contiguous run, kAhead terms in flight; the sums are
+// transposed through shared memory so that each frequency's values are written
+// as a contiguous run of slots.
 constexpr int kSlotThreads = 256;
-__global__ void __launch_bounds__(kSlotThreads) k_slot_sum(int ndest, int nnz, int n, int nf, const int* dest_ptr,
-                                                           const int* dest_terms, const cplx* terms,
-                                                           cplx* values, cplx* rhs) {
+template <int kAhead>
+__global__ void __launch_bounds__(kSlotThreads, kAhead == 1 ? 8 : 4) k_slot_sum(int ndest, int nnz, int n, int nf,
+                                                                                const int* dest_ptr,
+                                                                                const int* dest_terms,
+                                                                                const cplx* terms, cplx* values,
+                                                                                cplx* rhs) {
     __shared__ cplx sh[kSlotThreads];
+    pdl_start_next();
     const int spb = kSlotThreads / nf;  // slots per block
     const int dl = threadIdx.x / nf, f = threadIdx.x - dl * nf;
     const int d0 = blockIdx.x * spb;
     const int d = d0 + dl;
-    if (dl < spb && d < ndest) {
-        cplx s{0.0, 0.0};
-        const int e = dest_ptr[d + 1];
-        for (int k = dest_ptr[d]; k < e; ++k) s = cadd_exact(s, terms[static_cast<long long>(dest_terms[k]) * nf + f]);
-        sh[f * spb + dl] = s;
+    const bool live = dl < spb && d < ndest;
+    int k = live ? dest_ptr[d] : 0;
+    const int e = live ? dest_ptr[d + 1] : 0;
+    pdl_wait();
+    cplx s{0.0, 0.0};
+    if constexpr (kAhead == 1) {
+        for (; k < e; ++k) s = cadd_exact(s, terms[static_cast<long long>(dest_terms[k]) * nf + f]);
+    } else {
+        while (k < e) {
+            cplx v[kAhead];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (k + u < e) v[u] = terms[static_cast<long long>(dest_terms[k + u]) * nf + f];
+#pragma unroll
+            for (int u = 0; u < kAhead; ++u)
+                if (k + u < e) s = cadd_exact(s, v[u]);
+            k += kAhead;
+        }
     }
+    if (live) sh[f * spb + dl] = s;
     __syncthreads();
     const int cnt = min(spb, ndest - d0);
-    for (int e = threadIdx.x; e < nf * spb; e += kSlotThreads) {
-        const int ff = e / spb, x = e - ff * spb;
+    for (int e2 = threadIdx.x; e2 < nf * spb; e2 += kSlotThreads) {
+        const int ff = e2 / spb, x = e2 - ff * spb;
         if (x >= cnt) continue;
         const int dd = d0 + x;
         if (dd < nnz)
-            values[static_cast<long long>(ff) * nnz + dd] = sh[e];
+            values[static_cast<long long>(ff) * nnz + dd] = sh[e2];
         else
-            rhs[static_cast<long long>(ff) * n + (dd - nnz)] = sh[e];
+            rhs[static_cast<long long>(ff) * n + (dd - nnz)] = sh[e2];
     }
 }
 
@@ -889,6 +949,7 @@ void assembly_refill(Assembly& A, int nfreq, const double* omegas, int cond, dou
     if (A.terms_capacity < chunk) {
         if (A.d_terms) APHI_CUDA(cudaFree(A.d_terms));
         A.d_terms = nullptr;
+        A.terms_capacity = 0;
         APHI_CUDA(cudaMalloc(&A.d_terms, static_cast<size_t>(chunk) * A.num_terms * sizeof(cplx)));
         A.terms_capacity = chunk;
     }
@@ -901,21 +962,31 @@ void assembly_refill(Assembly& A, int nfreq, const double* omegas, int cond, dou
         om.n = std::min(chunk, nfreq - f0);
         for (int i = 0; i < om.n; ++i) om.w[i] = omegas[f0 + i];
         cplx* terms = reinterpret_cast<cplx*>(A.d_terms);
-        if (A.T > 0) {
-            k_tet_terms<<<ceil_div(A.T, kTetWarps), 32 * kTetWarps, 0, stream>>>(ta, om, cond, q, terms);
+        // Few tets: one a warp, so that every multiprocessor has some; many:
+        // four a warp, whose geometry then shares a warp's instructions.
+        auto tet_terms = [&](auto kern, int rounds, int smem) {
+            APHI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            kern<<<ceil_div(A.T, kTetWarps * rounds) + 1, 32 * kTetWarps, smem, stream>>>(ta, pa, om, cond, q, terms);
             APHI_CHECK_LAUNCH();
-        }
-        if (A.num_ports > 0) {
-            k_port_terms<<<1, 64, 0, stream>>>(pa, om, cond, terms);
-            APHI_CHECK_LAUNCH();
-        }
+        };
+        if (A.T <= kTetWarps * 8 * kNumSMs)
+            tet_terms(k_tet_terms<1>, 1, TetBlock<kTetWarps>::bytes(om.n));
+        else
+            tet_terms(k_tet_terms<4>, 4, TetBlock<4 * kTetWarps>::bytes(om.n));
         const int ndest = A.nnz + A.N;
         const int spb = kSlotThreads / om.n;
-        k_slot_sum<<<ceil_div(ndest, spb), kSlotThreads, 0, stream>>>(
-            ndest, A.nnz, A.N, om.n, A.d_dest_ptr, A.d_dest_terms, terms,
-            reinterpret_cast<cplx*>(values_dev) + static_cast<long long>(f0) * A.nnz,
-            reinterpret_cast<cplx*>(rhs_dev) + static_cast<long long>(f0) * A.N);
-        APHI_CHECK_LAUNCH();
+        auto slot_sum = [&](auto kern) {
+            chained(kern, dim3(ceil_div(ndest, spb)), kSlotThreads, 0, stream, ndest, A.nnz, A.N, om.n, A.d_dest_ptr,
+                    A.d_dest_terms, terms, reinterpret_cast<cplx*>(values_dev) + static_cast<long long>(f0) * A.nnz,
+                    reinterpret_cast<cplx*>(rhs_dev) + static_cast<long long>(f0) * A.N);
+            APHI_CHECK_LAUNCH();
+        };
+        // Many frequencies: most slots have one or two terms and there are
+        // enough threads, so fewer terms in flight and more of them resident.
+        if (om.n >= 4)
+            slot_sum(k_slot_sum<1>);
+        else
+            slot_sum(k_slot_sum<4>);
     }
 }
 

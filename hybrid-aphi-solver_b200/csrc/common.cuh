@@ -69,6 +69,36 @@ __device__ __forceinline__ cplx cadd(cplx a, cplx b) { return cplx{a.re + b.re, 
 __device__ __forceinline__ cplx csub(cplx a, cplx b) { return cplx{a.re - b.re, a.im - b.im}; }
 #endif
 
+#ifdef __CUDACC__
+// A factorization or a solve is a chain of short launches, and much of a short
+// launch is its start: items, schedule, and in a solve the panel entries, all
+// of them constants. So these kernels are launched with programmatic stream
+// serialization: a kernel lets the next one start as it begins itself
+// (pdl_start_next), which then reads its constants and waits (pdl_wait) until
+// the kernel before it has finished and its writes are visible. Everything
+// that a launch before could have written, or still reads where this one
+// writes, comes after pdl_wait(); every kernel launched this way calls it, so
+// that the wait covers all launches before.
+__device__ __forceinline__ void pdl_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A launch that may start before the one before it has finished (pdl_wait).
+template <class... Params, class... Args>
+void chained(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    APHI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
+}
+#endif
+
 inline int ceil_div(long long a, long long b) { return static_cast<int>((a + b - 1) / b); }
 
 constexpr int kNumSMs = 148;

@@ -353,22 +353,6 @@ void device_parts(void** base, const std::vector<std::pair<void**, size_t>>& par
     }
 }
 
-// A launch that may start before the one before it has finished (pdl_wait).
-template <class... Params, class... Args>
-void chained(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    APHI_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...));
-}
-
 template <class R>
 void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_t st, const SolveArgs* sa,
               cx<R>* y, cx<R>* U, cx<R>* part) {

@@ -83,18 +83,6 @@ inline Sched sched_of(const DeviceSchedule& d) {
                  d.child_ptr, d.child_list, d.uoff, d.items};
 }
 
-// A factorization or a solve is a chain of short launches, and much of a short
-// launch is its start: items, schedule, and in a solve the panel entries, all
-// of them constants. So these kernels are launched with programmatic stream
-// serialization: a kernel lets the next one start as it begins itself
-// (pdl_start_next), which then reads its constants and waits (pdl_wait) until
-// the kernel before it has finished and its writes are visible. Everything
-// that a launch before could have written, or still reads where this one
-// writes, comes after pdl_wait(); every kernel launched this way calls it, so
-// that the wait covers all launches before.
-__device__ __forceinline__ void pdl_start_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // ---------------------------------------------------------------- 64 x 64 blocks
 // Blocks of L in shared memory have leading dimension kTriLd (65: column-
 // strided reads fall in distinct banks).
