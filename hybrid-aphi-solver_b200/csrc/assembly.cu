@@ -126,22 +126,22 @@ __device__ __forceinline__ double dot3(const double* u, const double* v) {
 }
 
 // Whitney edge function at barycentric point L: grad(L_j) L_i - grad(L_i) L_j.
-__device__ __forceinline__ void whitney(const Geometry& g, int e, const double* L, double* out) {
+__device__ __forceinline__ void whitney(const double (*grad)[3], int e, const double* L, double* out) {
     const int vi = c_edge_verts[e][0], vj = c_edge_verts[e][1];
     for (int k = 0; k < 3; ++k)
-        out[k] = __dsub_rn(__dmul_rn(g.grad[vj][k], L[vi]), __dmul_rn(g.grad[vi][k], L[vj]));
+        out[k] = __dsub_rn(__dmul_rn(grad[vj][k], L[vi]), __dmul_rn(grad[vi][k], L[vj]));
 }
 
 // Gradient of P2 nodal function b at L.
-__device__ __forceinline__ void p2_grad(const Geometry& g, int b, const double* L, double* out) {
+__device__ __forceinline__ void p2_grad(const double (*grad)[3], int b, const double* L, double* out) {
     if (b < 4) {
         const double s = __dsub_rn(__dmul_rn(4.0, L[b]), 1.0);
-        for (int k = 0; k < 3; ++k) out[k] = __dmul_rn(g.grad[b][k], s);
+        for (int k = 0; k < 3; ++k) out[k] = __dmul_rn(grad[b][k], s);
     } else {
         const int v0 = c_edge_verts[b - 4][0], v1 = c_edge_verts[b - 4][1];
         const double s0 = __dmul_rn(4.0, L[v1]), s1 = __dmul_rn(4.0, L[v0]);
         for (int k = 0; k < 3; ++k)
-            out[k] = __dadd_rn(__dmul_rn(g.grad[v0][k], s0), __dmul_rn(g.grad[v1][k], s1));
+            out[k] = __dadd_rn(__dmul_rn(grad[v0][k], s0), __dmul_rn(grad[v1][k], s1));
     }
 }
 
@@ -203,7 +203,7 @@ __device__ void element_blocks(const Geometry& g, const Coeff& c, const Quad& q,
         for (int i = 0; i < 4; ++i) L[i] = (i == k) ? q.a : q.b;
         const double w = __dmul_rn(0.25, g.volume);
         double wv[6][3];
-        for (int e = 0; e < 6; ++e) whitney(g, e, L, wv[e]);
+        for (int e = 0; e < 6; ++e) whitney(g.grad, e, L, wv[e]);
         if (mass) {
             for (int i = 0; i < 6; ++i)
                 for (int j = 0; j < 6; ++j) {
@@ -213,7 +213,7 @@ __device__ void element_blocks(const Geometry& g, const Coeff& c, const Quad& q,
         }
         if (coupling) {
             double gr[10][3];
-            for (int b = 0; b < 10; ++b) p2_grad(g, b, L, gr[b]);
+            for (int b = 0; b < 10; ++b) p2_grad(g.grad, b, L, gr[b]);
             for (int i = 0; i < 6; ++i)
                 for (int b = 0; b < 10; ++b) {
                     const double s = __dmul_rn(w, dot3(wv[i], gr[b]));
@@ -1030,19 +1030,52 @@ void element_blocks_host(int ntets, const double* xyz, double nu, const double* 
 // ---------------------------------------------------------------- post-solve fields
 // compute_fields and the potential of potential_at_nodes (src/postprocess.cpp:
 // 42-126, 223-486) on the device.
-//   k_field_tets: one thread per tet. Geometry, A's and Phi's coefficients
-//     for this tet (a cut's side already resolved by the tet's DOF table),
-//     B = curl A (constant), A and E = -j w A - grad Phi at the centroid and
-//     at each of the ten P2 nodes, J = sigma E. The node values go, with the
-//     tet's volume, to a contribution array.
-//   k_field_nodes: one thread per P2 node sums its contributions in
-//     increasing tet order -- the reference's accumulation order -- with the
-//     reference's side selection (E over the most conducting tets, B over the
-//     most permeable), normalises each by its own weight, and forms J and H.
+//   k_tet_geometry; k_field_tets: 16 tets a block. A's and Phi's coefficients
+//     for the tet (a cut's side already resolved by the tet's DOF table), one
+//     thread each; then one thread per (tet, point): A and E = -j w A - grad
+//     Phi at the ten P2 nodes and the centroid, J = sigma E, and B = curl A
+//     (constant). The node values go, with the tet's volume, to a
+//     contribution array.
+//   k_field_nodes: four threads per P2 node (one a component, one for Phi)
+//     sum its contributions in increasing tet order -- the reference's
+//     accumulation order -- with the reference's side selection (E over the
+//     most conducting tets, B over the most permeable), normalise each by its
+//     own weight, and form J and H.
+// Chains of dependent uncontracted FP64 operations and gathers bound them, so
+// the work is spread over as many threads as there are results. 16^3 torus: 41
+// + 66 us with one thread a tet and one a node, 6 + 26 + 29 (overlapping) so.
 // Every operation is the reference's, in its order, rounded explicitly.
 namespace {
 
-constexpr int kFieldContrib = 13;  // volume, A (3 complex), E (3 complex)
+constexpr int kFieldContrib = 14;  // volume, nothing, A (3 complex), E (3 complex)
+
+// Gradients (12) and volume (negative: degenerate) of every tet, one thread a
+// tet: a chain of dependent divisions, which a block of k_field_tets would run
+// on 16 of its threads while the others wait (46 us for both so, 31 apart).
+constexpr int kGeoStride = 16;  // doubles per tet
+__global__ void __launch_bounds__(64) k_tet_geometry(int T, const int* tets, const double* xyz, double* geo,
+                                                     int* err) {
+    pdl_start_next();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= T) return;
+    double p[4][3], grad[4][3], vol;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const int node = tets[4LL * t + r];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[r][k] = xyz[3LL * node + k];
+    }
+    double2* out = reinterpret_cast<double2*>(geo + static_cast<long long>(t) * kGeoStride);
+    if (!tet_geometry_reg(p, grad, vol)) {
+        atomicExch(err, 1);
+        out[6] = make_double2(-1.0, 0.0);
+        return;
+    }
+#pragma unroll
+    for (int e = 0; e < 6; ++e)
+        out[e] = make_double2(grad[(2 * e) / 3][(2 * e) % 3], grad[(2 * e + 1) / 3][(2 * e + 1) % 3]);
+    out[6] = make_double2(vol, 0.0);
+}
 
 struct FieldArgs {
     int T, P, nv;
@@ -1056,6 +1089,7 @@ struct FieldArgs {
     const double* tet_fixed;
     const cplx* x;
     cplx scale, mjw;
+    const double* geo;  // kGeoStride doubles per tet
     double* contrib;
     const int* inc_ptr;
     const int* inc;
@@ -1073,8 +1107,8 @@ __device__ __forceinline__ void cross_rn(const double* a, const double* b, doubl
 }
 
 // A and E of one tet at barycentric point L.
-__device__ void field_at(const Geometry& g, const cplx (&a)[6], const double (&sgn)[6], const cplx (&ph)[10],
-                         cplx mjw, const double* L, cplx (&av)[3], cplx (&ev)[3]) {
+__device__ void field_at(const double (*g)[3], const cplx* a, const double* sgn, const cplx* ph, cplx mjw,
+                         const double* L, cplx (&av)[3], cplx (&ev)[3]) {
     cplx gp[3];
     for (int i = 0; i < 3; ++i) av[i] = gp[i] = cplx{0.0, 0.0};
     for (int k = 0; k < 6; ++k) {
@@ -1093,75 +1127,78 @@ __device__ void field_at(const Geometry& g, const cplx (&a)[6], const double (&s
     }
 }
 
-__global__ void __launch_bounds__(128) k_field_tets(FieldArgs A, cplx* a_tet, cplx* b_tet, cplx* e_tet, cplx* j_tet,
-                                                    double* sigma_tet) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= A.T) return;
-    double p[4][3];
-    for (int q = 0; q < 4; ++q) {
-        const int node = A.tets[4LL * t + q];
-        for (int k = 0; k < 3; ++k) p[q][k] = A.xyz[3LL * node + k];
+constexpr int kFieldTets = 16, kFieldThreads = 256;
+__global__ void __launch_bounds__(kFieldThreads) k_field_tets(FieldArgs A, cplx* a_tet, cplx* b_tet, cplx* e_tet,
+                                                              cplx* j_tet, double* sigma_tet) {
+    static_assert(kFieldThreads == 16 * kFieldTets, "one thread per tet and coefficient");
+    __shared__ double s_geo[kFieldTets][kGeoStride + 1];  // gradients, volume (banks: 17 apart)
+    __shared__ cplx s_a[kFieldTets][6], s_ph[kFieldTets][10];
+    __shared__ double s_sgn[kFieldTets][6];
+    __shared__ double s_L[11][4];  // the points' barycentric coordinates
+    pdl_start_next();
+    const int t0 = blockIdx.x * kFieldTets;
+    if (threadIdx.x >= 32 && threadIdx.x < 32 + 44) {
+        const int q = (threadIdx.x - 32) / 4, i = threadIdx.x % 4;
+        s_L[q][i] = q == 10 ? 0.25
+                    : q < 4 ? (i == q ? 1.0 : 0.0)
+                            : (i == c_edge_verts[q - 4][0] || i == c_edge_verts[q - 4][1] ? 0.5 : 0.0);
     }
-    Geometry g;
-    if (!tet_geometry(p, g)) {
-        atomicExch(A.err, 1);
+    {
+        const int lt = threadIdx.x / 16, n = threadIdx.x % 16, t = t0 + lt;
+        if (t < A.T) {
+            const int idx = A.tet_idx[16LL * t + n];
+            const double co = A.tet_coeff[16LL * t + n];
+            if (n < 6) {
+                // A: the raw global unknown of each live edge; the edge sign goes
+                // with the basis function (whitney_edge_value_global).
+                s_sgn[lt][n] = co;
+                s_a[lt][n] = idx >= 0 ? A.x[idx] : cplx{0.0, 0.0};
+            } else {
+                // Phi: (scale * coeff) * x for an unknown, the prescribed value otherwise.
+                s_ph[lt][n - 6] = idx >= 0 ? cmul_exact(cscale_exact(A.scale, co), A.x[idx])
+                                           : cplx{A.tet_fixed[20LL * t + 2 * (n - 6)], A.tet_fixed[20LL * t + 2 * (n - 6) + 1]};
+            }
+        }
+    }
+    pdl_wait();
+    {
+        const int lt = threadIdx.x / 16, c = threadIdx.x % 16;
+        if (t0 + lt < A.T && c < 13) s_geo[lt][c] = A.geo[static_cast<long long>(t0 + lt) * kGeoStride + c];
+    }
+    __syncthreads();
+    // Point 0 .. 9: the P2 nodes; 10: the centroid; 11: B.
+    const int lt = threadIdx.x % kFieldTets, point = threadIdx.x / kFieldTets, t = t0 + lt;
+    if (t >= A.T || point > 11 || s_geo[lt][12] < 0.0) return;
+    const auto* grad = reinterpret_cast<const double(*)[3]>(s_geo[lt]);
+    if (point == 11) {
+        // B = curl A = sum_e a_e * 2 (grad L_i x grad L_j) * sign_e.
+        cplx b[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
+        for (int k = 0; k < 6; ++k) {
+            double c[3];
+            cross_rn(grad[c_edge_verts[k][0]], grad[c_edge_verts[k][1]], c);
+            for (int i = 0; i < 3; ++i)
+                b[i] = cadd_exact(b[i], cscale_exact(s_a[lt][k], __dmul_rn(__dmul_rn(c[i], 2.0), s_sgn[lt][k])));
+        }
+        for (int i = 0; i < 3; ++i) b_tet[3LL * t + i] = b[i];
         return;
     }
-    // A: the raw global unknown of each live edge; the edge sign goes with the
-    // basis function (whitney_edge_value_global).
-    cplx a[6];
-    double sgn[6];
-    for (int k = 0; k < 6; ++k) {
-        const int idx = A.tet_idx[16LL * t + k];
-        sgn[k] = A.tet_coeff[16LL * t + k];
-        a[k] = idx >= 0 ? A.x[idx] : cplx{0.0, 0.0};
-    }
-    // Phi: (scale * coeff) * x for an unknown, the prescribed value otherwise.
-    cplx ph[10];
-    for (int n = 0; n < 10; ++n) {
-        const int idx = A.tet_idx[16LL * t + 6 + n];
-        if (idx >= 0)
-            ph[n] = cmul_exact(cscale_exact(A.scale, A.tet_coeff[16LL * t + 6 + n]), A.x[idx]);
-        else
-            ph[n] = cplx{A.tet_fixed[20LL * t + 2 * n], A.tet_fixed[20LL * t + 2 * n + 1]};
-    }
-    // B = curl A = sum_e a_e * 2 (grad L_i x grad L_j) * sign_e.
-    cplx b[3] = {{0.0, 0.0}, {0.0, 0.0}, {0.0, 0.0}};
-    for (int k = 0; k < 6; ++k) {
-        double c[3];
-        cross_rn(g.grad[c_edge_verts[k][0]], g.grad[c_edge_verts[k][1]], c);
-        for (int i = 0; i < 3; ++i) b[i] = cadd_exact(b[i], cscale_exact(a[k], __dmul_rn(__dmul_rn(c[i], 2.0), sgn[k])));
-    }
-    const int body = A.body_of_tet[t];
-    const double sigma = A.material[3 * body];
-    sigma_tet[t] = sigma;
     cplx av[3], ev[3];
-    const double Lc[4] = {0.25, 0.25, 0.25, 0.25};
-    field_at(g, a, sgn, ph, A.mjw, Lc, av, ev);
-    for (int i = 0; i < 3; ++i) {
-        a_tet[3LL * t + i] = av[i];
-        b_tet[3LL * t + i] = b[i];
-        e_tet[3LL * t + i] = ev[i];
-        j_tet[3LL * t + i] = cscale_exact(ev[i], sigma);
-    }
-    const double vol = g.volume;
-    for (int k = 0; k < 10; ++k) {
-        double L[4] = {0.0, 0.0, 0.0, 0.0};
-        if (k < 4) {
-            L[k] = 1.0;
-        } else {
-            L[c_edge_verts[k - 4][0]] = 0.5;
-            L[c_edge_verts[k - 4][1]] = 0.5;
-        }
-        field_at(g, a, sgn, ph, A.mjw, L, av, ev);
-        double* o = A.contrib + (10LL * t + k) * kFieldContrib;
-        o[0] = vol;
+    field_at(grad, s_a[lt], s_sgn[lt], s_ph[lt], A.mjw, s_L[point], av, ev);
+    if (point == 10) {
+        const double sigma = A.material[3 * A.body_of_tet[t]];
+        sigma_tet[t] = sigma;
         for (int i = 0; i < 3; ++i) {
-            o[1 + 2 * i] = av[i].re;
-            o[2 + 2 * i] = av[i].im;
-            o[7 + 2 * i] = ev[i].re;
-            o[8 + 2 * i] = ev[i].im;
+            a_tet[3LL * t + i] = av[i];
+            e_tet[3LL * t + i] = ev[i];
+            j_tet[3LL * t + i] = cscale_exact(ev[i], sigma);
         }
+        return;
+    }
+    double2* o = reinterpret_cast<double2*>(A.contrib + (10LL * t + point) * kFieldContrib);
+    o[0] = make_double2(s_geo[lt][12], 0.0);
+    for (int i = 0; i < 3; ++i) {
+        o[1 + i] = make_double2(av[i].re, av[i].im);
+        o[4 + i] = make_double2(ev[i].re, ev[i].im);
     }
 }
 
@@ -1169,72 +1206,93 @@ __global__ void __launch_bounds__(256) k_field_nodes(FieldArgs A, const cplx* b_
                                                      cplx* phi_node, cplx* a_node, cplx* b_node, cplx* h_node,
                                                      cplx* e_node, cplx* j_node, double* vertex_weight,
                                                      unsigned char* on_interface) {
-    const int u = blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= A.P) return;
-    const bool sig_u = A.sig_uniform[u] != 0, mu_u = A.mu_uniform[u] != 0;
+    constexpr int kAhead = 4;  // contributions in flight
+    pdl_start_next();
+    const int u = (blockIdx.x * blockDim.x + threadIdx.x) / 4, i = threadIdx.x % 4;  // i = 3: Phi and the weights
+    const bool live = u < A.P;
+    const int q0 = live ? A.inc_ptr[u] : 0, q1 = live ? A.inc_ptr[u + 1] : 0;
+    const bool sig_u = live && A.sig_uniform[u] != 0, mu_u = live && A.mu_uniform[u] != 0;
+    const double sig_max = live ? A.sig_max[u] : 0.0, mu_max = live ? A.mu_max[u] : 0.0;
+    pdl_wait();
+    if (!live) return;
     double vw = 0.0, ew = 0.0, bw = 0.0;
-    cplx an[3], en[3], bn[3];
-    for (int i = 0; i < 3; ++i) an[i] = en[i] = bn[i] = cplx{0.0, 0.0};
-    cplx phi{0.0, 0.0};
+    cplx an{0.0, 0.0}, en{0.0, 0.0}, bn{0.0, 0.0}, phi{0.0, 0.0};
     bool phi_unknown = false, phi_fixed = false;
-    for (int q = A.inc_ptr[u]; q < A.inc_ptr[u + 1]; ++q) {
-        const int e = A.inc[q];
-        const int t = e / 10, k = e % 10;
-        const double* c = A.contrib + static_cast<long long>(e) * kFieldContrib;
-        const double vol = c[0];
-        vw = __dadd_rn(vw, vol);
-        for (int i = 0; i < 3; ++i) an[i] = cadd_exact(an[i], cscale_exact(cplx{c[1 + 2 * i], c[2 + 2 * i]}, vol));
-        if (sig_u || sigma_tet[t] == A.sig_max[u]) {
-            ew = __dadd_rn(ew, vol);
-            for (int i = 0; i < 3; ++i) en[i] = cadd_exact(en[i], cscale_exact(cplx{c[7 + 2 * i], c[8 + 2 * i]}, vol));
+    for (int q = q0; q < q1; q += kAhead) {
+        int tet[kAhead], node[kAhead];
+        double vol[kAhead], sig[kAhead], mu[kAhead];
+        double2 ac[kAhead], ec[kAhead];
+        cplx bc[kAhead];
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            if (q + j >= q1) continue;
+            const int e = A.inc[q + j];
+            tet[j] = e / 10;
+            node[j] = e % 10;
+            const double2* c = reinterpret_cast<const double2*>(A.contrib + static_cast<long long>(e) * kFieldContrib);
+            vol[j] = c[0].x;
+            sig[j] = sigma_tet[tet[j]];
+            mu[j] = __dmul_rn(kMu0, A.material[3 * A.body_of_tet[tet[j]] + 2]);
+            if (i < 3) {
+                ac[j] = c[1 + i];
+                ec[j] = c[4 + i];
+                bc[j] = b_tet[3LL * tet[j] + i];
+            }
         }
-        const double mu = __dmul_rn(kMu0, A.material[3 * A.body_of_tet[t] + 2]);
-        if (mu_u || mu == A.mu_max[u]) {
-            bw = __dadd_rn(bw, vol);
-            for (int i = 0; i < 3; ++i) bn[i] = cadd_exact(bn[i], cscale_exact(b_tet[3LL * t + i], vol));
-        }
-        // Phi at the node: the unknown any incident tet reads (a cut's plus
-        // side), else the first nonzero prescribed value.
-        {
-            const int idx = A.tet_idx[16LL * t + 6 + k];
-            if (idx >= 0 && !phi_unknown) {
-                phi = cmul_exact(A.scale, A.x[idx]);
-                phi_unknown = true;
-            } else if (idx < 0 && !phi_unknown && !phi_fixed) {
-                const cplx f{A.tet_fixed[20LL * t + 2 * k], A.tet_fixed[20LL * t + 2 * k + 1]};
-                if (f.re != 0.0 || f.im != 0.0) {
-                    phi = f;
-                    phi_fixed = true;
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j) {
+            if (q + j >= q1) continue;
+            const bool with_e = sig_u || sig[j] == sig_max, with_b = mu_u || mu[j] == mu_max;
+            vw = __dadd_rn(vw, vol[j]);
+            if (with_e) ew = __dadd_rn(ew, vol[j]);
+            if (with_b) bw = __dadd_rn(bw, vol[j]);
+            if (i < 3) {
+                an = cadd_exact(an, cscale_exact(cplx{ac[j].x, ac[j].y}, vol[j]));
+                if (with_e) en = cadd_exact(en, cscale_exact(cplx{ec[j].x, ec[j].y}, vol[j]));
+                if (with_b) bn = cadd_exact(bn, cscale_exact(bc[j], vol[j]));
+            } else if (!phi_unknown) {
+                // Phi at the node: the unknown any incident tet reads (a cut's plus
+                // side), else the first nonzero prescribed value.
+                const int idx = A.tet_idx[16LL * tet[j] + 6 + node[j]];
+                if (idx >= 0) {
+                    phi = cmul_exact(A.scale, A.x[idx]);
+                    phi_unknown = true;
+                } else if (!phi_fixed) {
+                    const double* f = A.tet_fixed + 20LL * tet[j] + 2 * node[j];
+                    if (f[0] != 0.0 || f[1] != 0.0) {
+                        phi = cplx{f[0], f[1]};
+                        phi_fixed = true;
+                    }
                 }
             }
         }
     }
-    phi_node[u] = phi;
-    vertex_weight[u] = vw;
-    on_interface[u] = (A.inc_ptr[u + 1] > A.inc_ptr[u]) && (!sig_u || !mu_u) ? 1 : 0;
+    if (i == 3) {
+        phi_node[u] = phi;
+        vertex_weight[u] = vw;
+        on_interface[u] = q1 > q0 && (!sig_u || !mu_u) ? 1 : 0;
+        return;
+    }
     if (vw > 0.0) {
-        for (int i = 0; i < 3; ++i) an[i] = cplx{__ddiv_rn(an[i].re, vw), __ddiv_rn(an[i].im, vw)};
-        if (ew > 0.0)
-            for (int i = 0; i < 3; ++i) en[i] = cplx{__ddiv_rn(en[i].re, ew), __ddiv_rn(en[i].im, ew)};
-        if (bw > 0.0)
-            for (int i = 0; i < 3; ++i) bn[i] = cplx{__ddiv_rn(bn[i].re, bw), __ddiv_rn(bn[i].im, bw)};
+        an = cplx{__ddiv_rn(an.re, vw), __ddiv_rn(an.im, vw)};
+        if (ew > 0.0) en = cplx{__ddiv_rn(en.re, ew), __ddiv_rn(en.im, ew)};
+        if (bw > 0.0) bn = cplx{__ddiv_rn(bn.re, bw), __ddiv_rn(bn.im, bw)};
     }
-    const double nu_node = vw > 0.0 ? __ddiv_rn(1.0, A.mu_max[u]) : 0.0;
-    const double smax = vw > 0.0 ? A.sig_max[u] : 0.0;
-    for (int i = 0; i < 3; ++i) {
-        a_node[3LL * u + i] = an[i];
-        e_node[3LL * u + i] = en[i];
-        b_node[3LL * u + i] = bn[i];
-        j_node[3LL * u + i] = vw > 0.0 ? cscale_exact(en[i], smax) : cplx{0.0, 0.0};
-        h_node[3LL * u + i] = vw > 0.0 ? cscale_exact(bn[i], nu_node) : cplx{0.0, 0.0};
-    }
+    const double nu_node = vw > 0.0 ? __ddiv_rn(1.0, mu_max) : 0.0;
+    const double smax = vw > 0.0 ? sig_max : 0.0;
+    a_node[3LL * u + i] = an;
+    e_node[3LL * u + i] = en;
+    b_node[3LL * u + i] = bn;
+    j_node[3LL * u + i] = vw > 0.0 ? cscale_exact(en, smax) : cplx{0.0, 0.0};
+    h_node[3LL * u + i] = vw > 0.0 ? cscale_exact(bn, nu_node) : cplx{0.0, 0.0};
 }
 
 }  // namespace
 
 Fields::~Fields() {
     for (void* p : {(void*)d_tet_edges, (void*)d_body_of_tet, (void*)d_inc_ptr, (void*)d_inc, (void*)d_sig_max,
-                    (void*)d_mu_max, (void*)d_sig_uniform, (void*)d_mu_uniform, (void*)d_contrib, (void*)d_err})
+                    (void*)d_mu_max, (void*)d_sig_uniform, (void*)d_mu_uniform, (void*)d_contrib,
+                    (void*)d_geo, (void*)d_err})
         if (p) cudaFree(p);
 }
 
@@ -1306,6 +1364,7 @@ std::unique_ptr<Fields> fields_create(const Assembly& A, int num_nodes, int num_
     F->d_sig_uniform = upload(su.data(), su.size());
     F->d_mu_uniform = upload(mu.data(), mu.size());
     APHI_CUDA(cudaMalloc(&F->d_contrib, std::max<size_t>(1, 10ULL * T * kFieldContrib) * sizeof(double)));
+    APHI_CUDA(cudaMalloc(&F->d_geo, sizeof(double) * kGeoStride * std::max(T, 1)));
     APHI_CUDA(cudaMalloc(&F->d_err, sizeof(int)));
     APHI_CUDA(cudaMemset(F->d_err, 0, sizeof(int)));
     return F;
@@ -1337,6 +1396,7 @@ void fields_compute(Fields& F, double omega, int conditioning, const double* x, 
     fa.scale.im = conditioning == APHI_COND_SCALED_PHI ? omega : 0.0;
     fa.mjw.re = -0.0;                                                 // -(j omega)
     fa.mjw.im = -omega;
+    fa.geo = F.d_geo;
     fa.contrib = F.d_contrib;
     fa.inc_ptr = F.d_inc_ptr;
     fa.inc = F.d_inc;
@@ -1346,15 +1406,17 @@ void fields_compute(Fields& F, double omega, int conditioning, const double* x, 
     fa.mu_uniform = F.d_mu_uniform;
     fa.err = F.d_err;
     if (F.T > 0) {
-        k_field_tets<<<ceil_div(F.T, 128), 128, 0, st>>>(fa, reinterpret_cast<cplx*>(o.a_tet),
-                                                        reinterpret_cast<cplx*>(o.b_tet), reinterpret_cast<cplx*>(o.e_tet),
-                                                        reinterpret_cast<cplx*>(o.j_tet), o.sigma_tet);
+        k_tet_geometry<<<ceil_div(F.T, 64), 64, 0, st>>>(F.T, A.d_tets, A.d_xyz, F.d_geo, F.d_err);
+        APHI_CHECK_LAUNCH();
+        chained(k_field_tets, dim3(ceil_div(F.T, kFieldTets)), kFieldThreads, 0, st, fa,
+                reinterpret_cast<cplx*>(o.a_tet), reinterpret_cast<cplx*>(o.b_tet), reinterpret_cast<cplx*>(o.e_tet),
+                reinterpret_cast<cplx*>(o.j_tet), o.sigma_tet);
         APHI_CHECK_LAUNCH();
     }
-    k_field_nodes<<<ceil_div(std::max(F.P, 1), 256), 256, 0, st>>>(
-        fa, reinterpret_cast<const cplx*>(o.b_tet), o.sigma_tet, reinterpret_cast<cplx*>(o.phi_node),
-        reinterpret_cast<cplx*>(o.a_node), reinterpret_cast<cplx*>(o.b_node), reinterpret_cast<cplx*>(o.h_node),
-        reinterpret_cast<cplx*>(o.e_node), reinterpret_cast<cplx*>(o.j_node), o.vertex_weight, o.on_interface);
+    chained(k_field_nodes, dim3(ceil_div(4LL * std::max(F.P, 1), 256)), 256, 0, st, fa,
+            reinterpret_cast<const cplx*>(o.b_tet), o.sigma_tet, reinterpret_cast<cplx*>(o.phi_node),
+            reinterpret_cast<cplx*>(o.a_node), reinterpret_cast<cplx*>(o.b_node), reinterpret_cast<cplx*>(o.h_node),
+            reinterpret_cast<cplx*>(o.e_node), reinterpret_cast<cplx*>(o.j_node), o.vertex_weight, o.on_interface);
     APHI_CHECK_LAUNCH();
     int err = 0;
     APHI_CUDA(cudaMemcpyAsync(&err, F.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -55,6 +55,7 @@ struct Fields {
     unsigned char* d_sig_uniform = nullptr;
     unsigned char* d_mu_uniform = nullptr;
     double* d_contrib = nullptr;
+    double* d_geo = nullptr;  // the tets' gradients and volumes
     int* d_err = nullptr;
     ~Fields();
 };
