@@ -394,7 +394,13 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
             APHI_CUDA(cudaEventRecord(e[0], st));
         }
         switch (l.kind) {
-            case K_EXTEND_ADD: chained(k_extend_add<R>, grid, 256, 0, st, S, l.first, L, CB, ls, cs); break;
+            case K_EXTEND_ADD: {
+                // Few items (they do not fill the chip): four blocks each, so that a
+                // warp has one column; many: one, which builds the maps once.
+                const bool few = static_cast<long long>(grid.x) * grid.y <= 4LL * f->sms;
+                chained(k_extend_add<R>, dim3(grid.x, grid.y, few ? 4 : 1), 256, 0, st, S, l.first, L, CB, ls, cs);
+                break;
+            }
             case K_SMALL: chained(k_small_front<R>, grid, kLdltThreads, smallsm, st, S, l.first, L, CB, ls, cs); break;
             case K_DIAG: chained(k_diag_block<R>, grid, kDiagThreads, diag_smem<R>(), st, S, l.first, L, ls); break;
             case K_TRSM: chained(k_panel_trsm<R>, grid, kTrsmThreads, trsm_smem<R>(), st, S, l.first, L, ls); break;

@@ -113,12 +113,31 @@ __device__ __forceinline__ void stage_block(cx<R>* T, const cx<R>* P, long long 
 __device__ __forceinline__ void triangle_wait() { cp_async_wait<0>(); }
 
 // ---------------------------------------------------------------- extend-add
-// Item (s, c0): front columns [c0, c0 + 32) of supernode s. Zeroes the CB
-// columns in that range, then adds every child's contribution block entries
-// that land in it, children in ascending order (a fixed summation order).
+// Item (s, c0): front columns [c0, c0 + 32) of supernode s, of which block z of
+// gridDim.z takes every gridDim.z-th eight. Every entry becomes itself (L) or
+// zero (CB) plus its children's contribution block entries, children in
+// ascending order (a fixed summation order).
+//
+// Bound by memory: latency low in the tree, traffic at its top. The block turns
+// two children's row maps around (front row -> child row, kEaRows rows at a
+// time, in shared memory, and before it waits for the launch before it: the maps
+// never change); then an entry is gathered from both, several of a thread at
+// once, and written once. Scattering child by child instead (binary searches
+// for the child's columns, a pass of zeros, a read and a write per entry and
+// child, a barrier per child) took 28 us a launch on 8^3, where this takes 12;
+// for eight matrices of 24^3 24 ms FP64, now 17.7, of about 12 that one read and
+// one write of the children's blocks take; for six of 32^3 in FP32 39.5 ms,
+// now 25. Three blocks a multiprocessor are best in FP64 (four 18.6 ms, two 21;
+// with twice the entries in flight 19.8); in FP32 fewer entries in flight or a
+// bound on the registers cost 10 %.
+constexpr int kEaRows = 4096, kEaKids = 2;
+static_assert(kEaKids == 2, "an entry's two maps are named");
 template <class R>
-__global__ void __launch_bounds__(256) k_extend_add(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
+__global__ void __launch_bounds__(256, sizeof(R) == 8 ? 3 : 0) k_extend_add(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
                                                     long long lstride, long long cbstride) {
+    constexpr int kUnroll = sizeof(R) == 8 ? 2 : 4;  // entries of a thread in flight
+    __shared__ int row_of[kEaKids][kEaRows];  // front row r0 + i -> child row, or -1
+    __shared__ int col_of[kEaKids][kEaCols];  // front column c0 + i -> child column, or -1
     pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, c0 = it.a;
@@ -130,43 +149,79 @@ __global__ void __launch_bounds__(256) k_extend_add(Sched S, long long item0, cx
     const int c1 = min(c0 + kEaCols, m);
     cx<R>* Ls = L + S.loff[s];
     cx<R>* CBs = CB + (cs > 0 ? S.cboff[s] : 0);
+    const int t0 = S.child_ptr[s], t1 = S.child_ptr[s + 1];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    pdl_wait();
-    for (int j = max(c0, w) + warp; j < c1; j += 8)
-        for (int i = j + lane; i < m; i += 32) CBs[(i - w) + static_cast<long long>(j - w) * cs] = cx<R>{0, 0};
-    __syncthreads();
-    for (int t = S.child_ptr[s]; t < S.child_ptr[s + 1]; ++t) {
-        const int c = S.child_list[t];
-        const int cw = S.first[c + 1] - S.first[c];
-        const int cc = S.rows[c] - cw;
-        if (cc <= 0) continue;
-        const int* rel = S.rel + S.reloff[c];
-        const cx<R>* CBc = CB + S.cboff[c];
-        // Child columns whose parent position falls in [c0, c1): binary search.
-        int lo = 0, hi = cc;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (rel[mid] < c0) lo = mid + 1; else hi = mid;
-        }
-        const int j0 = lo;
-        hi = cc;
-        while (lo < hi) {
-            const int mid = (lo + hi) >> 1;
-            if (rel[mid] < c1) lo = mid + 1; else hi = mid;
-        }
-        const int j1 = lo;
-        for (int j = j0 + warp; j < j1; j += 8) {
-            const int pj = rel[j];
-            const cx<R>* src = CBc + static_cast<long long>(j) * cc;
-            if (pj < w) {
-                cx<R>* dst = Ls + static_cast<long long>(pj) * m;
-                for (int i = j + lane; i < cc; i += 32) dst[rel[i]] = dst[rel[i]] + src[i];
-            } else {
-                cx<R>* dst = CBs + static_cast<long long>(pj - w) * cs - w;
-                for (int i = j + lane; i < cc; i += 32) dst[rel[i]] = dst[rel[i]] + src[i];
+    bool waited = false;
+    for (int r0 = c0; r0 < m; r0 += kEaRows) {
+        const int r1 = min(r0 + kEaRows, m);
+        for (int t = t0; t == t0 || t < t1; t += kEaKids) {
+            const int kids = min(kEaKids, t1 - t);
+            const cx<R>* kid_cb[kEaKids];
+            int kid_rows[kEaKids];
+            for (int k = 0; k < kids; ++k)
+                for (int i = threadIdx.x; i < r1 - r0; i += 256) row_of[k][i] = -1;
+            if (threadIdx.x < kEaKids * kEaCols) col_of[threadIdx.x / kEaCols][threadIdx.x % kEaCols] = -1;
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < kEaKids; ++k) {
+                kid_cb[k] = CB;
+                kid_rows[k] = 0;
+                if (k >= kids) continue;
+                const int c = S.child_list[t + k];
+                const int cc = S.rows[c] - (S.first[c + 1] - S.first[c]);
+                if (cc <= 0) continue;
+                const int* rel = S.rel + S.reloff[c];
+                kid_cb[k] = CB + S.cboff[c];
+                kid_rows[k] = cc;
+                for (int i = threadIdx.x; i < cc; i += 256) {
+                    const int r = rel[i];
+                    if (r >= r0 && r < r1) row_of[k][r - r0] = i;
+                    if (r >= c0 && r < c1) col_of[k][r - c0] = i;
+                }
             }
+            if (!waited) pdl_wait();
+            waited = true;
+            __syncthreads();
+            for (int j = c0 + warp + 8 * blockIdx.z; j < c1; j += 8 * gridDim.z) {
+                const bool in_l = j < w;
+                const bool fresh = !in_l && t == t0;  // starts from zero
+                const cx<R>* src[kEaKids];
+                bool live[kEaKids], any = false;
+#pragma unroll
+                for (int k = 0; k < kEaKids; ++k) {
+                    const int cj = col_of[k][j - c0];
+                    live[k] = cj >= 0;
+                    any |= live[k];
+                    src[k] = kid_cb[k] + static_cast<long long>(max(cj, 0)) * kid_rows[k];
+                }
+                if (!any && !fresh) continue;
+                cx<R>* dst = in_l ? Ls + static_cast<long long>(j) * m : CBs + static_cast<long long>(j - w) * cs - w;
+                for (int rb = max(j, r0) + lane; rb < r1; rb += 32 * kUnroll) {
+                    int at[kUnroll][kEaKids];
+                    cx<R> v[kUnroll], x[kUnroll][kEaKids];
+#pragma unroll
+                    for (int u = 0; u < kUnroll; ++u) {
+                        const int r = rb + 32 * u;
+#pragma unroll
+                        for (int k = 0; k < kEaKids; ++k) {
+                            at[u][k] = live[k] && r < r1 ? row_of[k][r - r0] : -1;
+                            if (at[u][k] >= 0) x[u][k] = src[k][at[u][k]];
+                        }
+                        v[u] = cx<R>{0, 0};
+                        if (!fresh && max(at[u][0], at[u][1]) >= 0) v[u] = dst[r];
+                    }
+#pragma unroll
+                    for (int u = 0; u < kUnroll; ++u) {
+                        const int r = rb + 32 * u;
+#pragma unroll
+                        for (int k = 0; k < kEaKids; ++k)
+                            if (at[u][k] >= 0) v[u] = v[u] + x[u][k];
+                        if (r < r1 && (fresh || max(at[u][0], at[u][1]) >= 0)) dst[r] = v[u];
+                    }
+                }
+            }
+            __syncthreads();
         }
-        __syncthreads();
     }
 }
 
