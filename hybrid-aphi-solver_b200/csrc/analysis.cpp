@@ -50,7 +50,7 @@ struct Uploads {
 // block, solves the panel rows below it and updates the rest of the panel's
 // own columns. Once a panel is complete, its trailing update -- every column
 // to its right, K = panel width -- runs as 128 x 64 tiles: `trailing` is
-// K_UPDATE_WIDE (DMMA for FP64, SIMT for FP32) or K_UPDATE_TC (tensor cores, FP32).
+// K_UPDATE_WIDE (FP64: tensor cores; FP32: SIMT) or K_UPDATE_TC (FP32 on tensor cores).
 // Updating the trailing front once per 128 columns instead of once per 64
 // reads and writes it half as often.
 void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing, std::vector<Launch>& plan) {
@@ -59,9 +59,10 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
         const int count = static_cast<int>(items.size() - first);
         if (count > 0) plan.push_back({kind, first, count, kcap, wide});
     };
-    // The FP64 plan (and the SIMT FP32 one) runs the in-panel updates on the
-    // trailing-update kernel as 128 x 64 tiles of K = 64, its columns capped
-    // at the panel's end; the tensor-core plan keeps the 64 x 64 SIMT tiles.
+    // The FP64 plan (and the SIMT FP32 one) runs the in-panel updates on
+    // k_update_wide_dmma (k_update_wide) as 128 x 64 tiles of K = 64, their
+    // columns capped at the panel's end; the tensor-core plan keeps the 64 x
+    // 64 SIMT tiles.
     const bool panel_wide = trailing == K_UPDATE_WIDE;
     // Trailing updates whose operands are prepared once per front and panel
     // group (K_TC_SPLIT / K_DMMA_SCALE launches) rather than inside every tile.
@@ -202,6 +203,7 @@ void build_factor_plan(aphi_analysis& A, std::vector<Item>& items, int trailing,
                         for (int r0 = 0; r0 < m - sf.pe; r0 += kTcM) items.push_back({sf.s, sf.p0, r0, 0, sf.d});
                     }
                     push(trailing == K_UPDATE_TC ? K_TC_SPLIT : K_DMMA_SCALE, f0, cap_group * kTcPanel);
+                    plan.back().units = static_cast<int>(region);
                     long long& units_max = trailing == K_UPDATE_TC ? A.tc_ws_units : A.dmma_ws_units;
                     units_max = std::max(units_max, region);
                     f0 = static_cast<long long>(items.size());

@@ -41,6 +41,7 @@ struct Launch {
     int wide = 0;         // K_UPDATE_PANEL: 128 x 64 tiles on the trailing-update kernels (column cap at the panel's end);
                           // K_FWD_GATHER / K_FWD_UPDATE / K_BWD_UPDATE: fused with the triangle solve (see build_plans)
     int span = 0;         // K_FWD_GATHER: rows of the launch's tallest front
+    int units = 0;        // K_TC_SPLIT / K_DMMA_SCALE: an entry's regions together, in 256-byte units
 };
 
 struct Item {

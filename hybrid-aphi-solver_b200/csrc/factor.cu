@@ -366,12 +366,30 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     const bool prof = f->profile;
     const bool presplit = sizeof(R) == 4 && f->tc_split == 2 && f->presplit && f->tcws;
     const bool i8 = presplit && f->tc_i8;  // FP32 trailing updates on INT8 digits
+    // The digits of a trailing update (split), and the update, which goes through
+    // the batch in as many passes as the digits' workspace asks for.
+    using Digits = std::conditional_t<sizeof(R) == 8, I8Fp64, I8Fp32>;
+    unsigned char* const digits = sizeof(R) == 8 ? f->dws : f->tcws;
+    auto split_i8 = [&](const Launch& l, int b0, int nb) {
+        chained(k_i8_split<R, Digits>, dim3(l.count, nb, kTcM / 32), 256, 0, st, S, l.first, L + ls * b0, ls, digits,
+                l.units * 256LL, l.kcap);
+    };
+    const Launch* operands = nullptr;  // of the next update
+    int pass = f->batch;               // entries whose digits fit the workspace at once
+    auto plan_i8 = [&](const Launch& l) {
+        operands = &l;
+        pass = static_cast<int>(std::clamp<long long>(f->digit_bytes / (l.units * 256LL), 1, f->batch));
+        if (pass == f->batch) split_i8(l, 0, f->batch);
+    };
     auto update_i8 = [&](const Launch& l) {
-        using C = std::conditional_t<sizeof(R) == 8, I8Fp64, I8Fp32>;
-        const long long tiles = static_cast<long long>(l.count) * (kTcN / C::Nc) * f->batch;
-        chained(k_update_i8<R, C>, dim3(static_cast<unsigned>(std::min<long long>(tiles, f->sms))), kI8Threads, C::smem,
-                st, S, l.first, l.count, f->batch, L, CB, ls, cs, l.kcap, sizeof(R) == 8 ? f->dws : f->tcws,
-                sizeof(R) == 8 ? f->dws_stride : f->tcws_stride, f->err);
+        for (int b0 = 0; b0 < f->batch; b0 += pass) {
+            const int nb = std::min(pass, f->batch - b0);
+            if (pass < f->batch) split_i8(*operands, b0, nb);
+            const long long tiles = static_cast<long long>(l.count) * (kTcN / Digits::Nc) * nb;
+            chained(k_update_i8<R, Digits>, dim3(static_cast<unsigned>(std::min<long long>(tiles, f->sms))), kI8Threads,
+                    Digits::smem, st, S, l.first, l.count, nb, L + ls * b0, CB + cs * b0, ls, cs, l.kcap, digits,
+                    operands->units * 256LL, f->err);
+        }
     };
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
     const size_t bwd_smem = (kTriSmem + (sa ? red_smem(sa->nr) : 0)) * sizeof(cx<R>);  // backward triangles
@@ -422,16 +440,14 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                 break;
             case K_DMMA_SCALE:
                 if constexpr (sizeof(R) == 8)
-                    chained(k_i8_split<double, I8Fp64>, dim3(grid.x, grid.y, kTcM / 32), 256, 0, st, S, l.first, L, ls,
-                            f->dws, f->dws_stride, l.kcap);
+                    plan_i8(l);
                 else
                     throw Error(APHI_ERR_INVALID, "operand scaling planned for an FP32 factor");
                 break;
             case K_TC_SPLIT:
                 if constexpr (sizeof(R) == 4) {
                     if (i8) {
-                        chained(k_i8_split<float, I8Fp32>, dim3(grid.x, grid.y, kTcM / 32), 256, 0, st, S, l.first, L,
-                                ls, f->tcws, f->tcws_stride, l.kcap);
+                        plan_i8(l);
                         break;
                     }
                     k_tc_split<<<dim3(grid.x, grid.y, (l.kcap + 8 * kTcK - 1) / (8 * kTcK)), kTcThreads, 0, st>>>(
@@ -650,6 +666,18 @@ void solve_numeric(aphi_factor* f, int nrhs, const double* b, double* x, cudaStr
 
 }  // namespace
 
+// Bytes of the digits' workspace for `stride` bytes an entry: all entries of a
+// batch while that is at most 1 GiB, above it as many as fit (one at least).
+// The launches that then take several passes fill the chip with each, since an
+// entry's share of them is over 1 GiB / batch: six entries of 32^3 in FP32 take
+// 195.6 ms (digits and tiles) so and 194.1 with room for all. Without the bound
+// the digits of FP64 batches (48 bytes a number) need three times what the
+// scaled rows of the DMMA form did, and the 32^3 sweep of 16 frequencies (FP32
+// batch of 16, FP64 batches of 8) no longer fits the device.
+static long long digit_workspace(long long stride, int batch) {
+    return std::max(stride, std::min(stride * batch, 1LL << 30));
+}
+
 aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
     if (!an) throw Error(APHI_ERR_INVALID, "factor: null analysis");
     if (precision != 64 && precision != 32) throw Error(APHI_ERR_BAD_SHAPE, "factor: precision must be 64 or 32");
@@ -693,8 +721,10 @@ aphi_factor* factor_create(aphi_analysis* an, int precision, int batch) {
         want(&f->kmax, sizeof(int) * batch);
         want(&f->err, 4 * sizeof(int));
         want(&f->counters, counters);
-        if (f->tcws_stride > 0) want(&f->tcws, static_cast<size_t>(f->tcws_stride) * batch);
-        if (f->dws_stride > 0) want(&f->dws, static_cast<size_t>(f->dws_stride) * batch);
+        f->digit_bytes = digit_workspace(precision == 64 ? f->dws_stride : f->tcws_stride, batch);
+        if (f->tcws_stride > 0)
+            want(&f->tcws, static_cast<size_t>(f->tc_i8 ? f->digit_bytes : f->tcws_stride * batch));
+        if (f->dws_stride > 0) want(&f->dws, static_cast<size_t>(f->digit_bytes));
         device_parts(&f->arena, parts);
         APHI_CUDA(cudaMemset(f->err, 0, 4 * sizeof(int)));
         APHI_CUDA(cudaMemset(f->counters, 0, counters));

@@ -43,10 +43,11 @@ struct aphi_factor {
     bool presplit = true;       // split 2: operands split once per panel group (k_tc_split; APHI_TC_PRESPLIT=0: in the tile)
     bool tc_i8 = true;          // split 2: INT8 digits (i8_update.cuh); APHI_TC_PRESPLIT set, to anything: two TF32 pieces
     int pre_stages = 3;         // plane buffers of the pre-split tile (APHI_TC_PRESTAGES=4: four; always four with tc_group 4)
-    unsigned char* dws = nullptr;  // FP64: the trailing updates' prepared operands (byte digits), dws_stride bytes per entry
-    long long dws_stride = 0;      // (APHI_DMMA_PRESCALE=0: none, the tiles run on DMMA from the panels)
+    unsigned char* dws = nullptr;  // FP64: the trailing updates' prepared operands (byte digits), up to dws_stride bytes per
+    long long dws_stride = 0;      // entry (APHI_DMMA_PRESCALE=0: none, the tiles run on DMMA from the panels)
+    long long digit_bytes = 0;     // of dws, or of tcws with INT8 digits (digit_workspace)
     int sms = 0;                   // multiprocessors of the device (persistent tiles' grid)
-    unsigned char* tcws = nullptr;  // the pre-split operand planes, tcws_stride bytes per entry (capacity entries)
+    unsigned char* tcws = nullptr;  // FP32: the digits, or the pre-split operand planes (tcws_stride bytes per entry)
     long long tcws_stride = 0;
     int* err = nullptr;         // device error word (bounded waits)
     int* kmax = nullptr;        // capacity: the column where each entry's factorization stopped

@@ -699,7 +699,7 @@ __global__ void __launch_bounds__(256) k_update_wide(Sched S, long long item0, c
 }
 
 // FP64 update on the FP64 tensor path (DMMA, mma.sync m8n8k4): the in-panel
-// updates (K = 32, too short for the INT8 tiles below), and the trailing ones
+// updates (K = 64, too short for the INT8 tiles below), and the trailing ones
 // too with APHI_DMMA_PRESCALE=0. Same items, tile and K (up to kcap =
 // kWidePair: a group of 128-column panels) as k_update_wide. 8 warps in a 4 x 2
 // grid, each a 32 x 32 complex block of the tile: 4 x 4 blocks of 8 x 8, each
@@ -1404,7 +1404,7 @@ __global__ void __launch_bounds__(kTcThreads) k_update_tc_presplit(Sched S, long
 // vectors into the front vector (y at the pivot rows, U_s below), then per
 // 64-column block: solve the block's unit triangle, update the rows below.
 // Backward (L^T x = D^-1 y), per level top-down, blocks last to first: partial
-// sums of L[rows below, block]^T x over 256-row chunks, then one CTA adds them
+// sums of L[rows below, block]^T x over row chunks, then one CTA adds them
 // in chunk order, scales by D^-1 and solves the block's triangle.
 
 
