@@ -334,6 +334,24 @@ def parity_vs_reference(args, rank, omegas, x):
             "frequencies": out}
 
 
+def update_kernel(precision, kind, tc_split, live):
+    """The kernel that serves a kind of update, the peak of its useful flops
+    [TFLOP/s] and what that is. The INT8 tiles form 36 (FP64: eight digits,
+    eight levels) or 10 (FP32: four and four) digit products per real product,
+    at a peak of four times the TF32 one (the nominal ratio)."""
+    digits = {"fp64": 36, "fp32": 10}[precision]
+    int8 = (4.0 * live["tf32_tc_n256"] / digits, f"4 x tf32_tc_n256 / {digits} digit products")
+    if kind == "update_tc":
+        if tc_split == 2 and "APHI_TC_PRESPLIT" not in os.environ:
+            return ("k_update_i8<float> (tcgen05 INT8-digit trailing update)", *int8)
+        return "k_update_tc (tcgen05 split-TF32 trailing update)", live["tf32_tc_n256"], "tf32_tc_n256"
+    if precision == "fp32":
+        return (f"k_update_wide<float> (SIMT {kind})" if kind == "update_wide" else kind), live["fp32_ffma"], "fp32_ffma"
+    if kind == "update_wide" and os.environ.get("APHI_DMMA_PRESCALE") != "0":
+        return ("k_update_i8<double> (tcgen05 INT8-digit trailing update)", *int8)
+    return f"k_update_wide_dmma (FP64 DMMA {kind})", live["fp64_dmma"], "fp64_dmma"
+
+
 def run_ours(args):
     import torch
     import aphi_b200 as ab
@@ -433,11 +451,7 @@ def run_ours(args):
                             "tflops": useful / (ms / 1000.0) / 1e12 if useful else None})
     kernels.sort(key=lambda k: -k["ms"])
     top = kernels[0]
-    name = {"update_wide": "k_update_wide_dmma (FP64 DMMA trailing update)" if top["precision"] == "fp64"
-            else "k_update_wide<float> (SIMT trailing update)",
-            "update_tc": "k_update_tc (tcgen05 split-TF32 trailing update)"}.get(top["kind"], top["kind"])
-    peak_key = {"fp64": "fp64_dmma", "fp32": "tf32_tc_n256" if top["kind"] == "update_tc" else "fp32_ffma"}[
-        top["precision"]]
+    name, peak, peak_source = update_kernel(top["precision"], top["kind"], args.tc_split, live_peaks)
 
     # The timed sweep's solutions against the reference's own solutions of
     # the same systems, where a fixture of this mesh exists (rank 0 solves the
@@ -560,10 +574,9 @@ def run_ours(args):
             "speedup_vs_fp64": value / fp64_value,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d), "d2h_bytes_per_step": int(d2h)},
             "roofline": {"bound": "tensor", "kernel": name, "achieved": top["tflops"],
-                         "peak": live_peaks[peak_key], "unit": "TFLOP/s",
-                         "frac": top["tflops"] / live_peaks[peak_key],
-                         "peak_source": (f"{peak_key}: measured live on this device by aphi_measure_peaks "
-                                         f"(MEASURED_PEAKS.json has only HBM and bf16: bf16 {bf16:.0f} TF/s, {src})"),
+                         "peak": peak, "unit": "TFLOP/s", "frac": top["tflops"] / peak,
+                         "peak_source": (f"{peak_source}, measured live on this device by aphi_measure_peaks "
+                                         f"(the file of measured peaks has only HBM and bf16: bf16 {bf16:.0f} TF/s, {src})"),
                          "traffic": traffic, "traffic_method": traffic_note,
                          "algorithmic": (f"useful Schur-update flops: {plan_flops[top['precision']][top['kind']][2]:.4e} "
                                          f"per factorization x {entries[top['precision']]} factorizations in the "
@@ -600,7 +613,7 @@ def main():
     ap.add_argument("--fp64-batch", type=int, default=8)
     ap.add_argument("--fp32-batch", type=int, default=0, help="FP32 entries per factorization (0: the whole sweep)")
     ap.add_argument("--tc-split", type=int, default=2, choices=[2, 3],
-                    help="TF32 pieces per FP32 operand in the tensor-core update (3: six products, 2: three)")
+                    help="the FP32 tensor-core update's form (2: INT8 digits; 3: three TF32 pieces per operand)")
     ap.add_argument("--fp64-steps", type=int, default=1)
     ap.add_argument("--sample-cells", type=int, default=16)
     ap.add_argument("--autotune", type=int, default=1, help="tune the schedule on this mesh first (untimed)")

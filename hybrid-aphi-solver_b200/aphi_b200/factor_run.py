@@ -33,7 +33,7 @@ def main() -> None:
     ap.add_argument("--f-hi", type=float, default=1.0e3)
     ap.add_argument("--simt", action="store_true", help="FP32 on the SIMT kernels instead of tcgen05")
     ap.add_argument("--tc-split", type=int, default=3, choices=[2, 3],
-                    help="TF32 pieces per operand in the tensor-core update")
+                    help="the tensor-core update's form (3: three TF32 pieces per operand; 2: INT8 digits)")
     ap.add_argument("--solves", type=int, default=0, help="also time this many solves of the batch")
     a = ap.parse_args()
     import torch

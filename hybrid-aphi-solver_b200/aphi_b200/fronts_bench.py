@@ -138,7 +138,8 @@ def run(count=512, seed=0, reps=3, check_every=16, lo=32, hi=2048, precisions=("
         if prec == ab.PREC_FP32:
             unit, raw = "tf32_tc_n64", upd_tf * 6        # 24 TF32 MMAs per complex multiply-add of 4
         else:
-            unit, raw = "fp64_dmma", upd_tf
+            # 36 digit products per real one, at four times the TF32 rate
+            unit, raw = "tf32_tc_n256", upd_tf * 36 / 4
         p, c = f.read_fronts(0)
         err = errors(fr, panels, p.cpu().numpy(), c.cpu().numpy(), sample)
         best = min(ms)
