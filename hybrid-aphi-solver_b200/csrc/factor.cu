@@ -425,7 +425,7 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
             case K_UPDATE_WIDE:
             case K_UPDATE_PANEL:
                 if (l.kind == K_UPDATE_PANEL && !l.wide) {
-                    chained(k_update_panel<R>, grid, 256, 2 * kStep * kTile * sizeof(cx<R>), st, S, l.first, L, CB, ls, cs);
+                    chained(k_update_panel<R>, grid, 256, 2 * kStep * kTile * sizeof(cx<R>), st, S, l.first, L, ls);
                     break;
                 }
                 if constexpr (sizeof(R) == 8) {

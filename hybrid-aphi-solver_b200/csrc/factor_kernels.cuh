@@ -505,79 +505,85 @@ __global__ void __launch_bounds__(kTrsmThreads) k_panel_trsm(Sched S, long long 
 // over the step's kb columns t, for i >= j >= k0 + kb and j inside the
 // current 128-column panel (the columns to its right get the whole panel's
 // update at once when the panel is complete).
+// Bound by latency and, where tiles are many, by FFMA issue: every load of a
+// thread is in flight at once, the destination's behind the operands', so a
+// block takes two round trips. Six entries of 32^3 in FP32 77 us a launch, eight
+// of 24^3 51 us; with the operands loaded a few at a time beside their pivots
+// and the destination read after the products 93 and 63. Two blocks a
+// multiprocessor keep the loads in registers (three spill: 90 and 62 us).
 template <class R>
-__global__ void __launch_bounds__(256) k_update_panel(Sched S, long long item0, cx<R>* Lb, cx<R>* CBb,
-                                                      long long lstride, long long cbstride) {
+__global__ void __launch_bounds__(256, sizeof(R) == 4 ? 2 : 1) k_update_panel(Sched S, long long item0, cx<R>* Lb, long long lstride) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cx<R>* As = reinterpret_cast<cx<R>*>(smem_raw);  // [kStep][kTile], scaled by D
     cx<R>* Bs = As + kStep * kTile;                  // [kStep][kTile]
+    __shared__ cx<R> D[kStep];
+    constexpr int kLoads = kStep * kTile / 256, kSkip = 256 / kTile;
     pdl_start_next();
     const Item it = S.items[item0 + blockIdx.x];
     const int s = it.s, k0 = it.a, i0 = it.b, j0 = it.c;
-    cx<R>* L = Lb + lstride * blockIdx.y;
-    cx<R>* CB = CBb + cbstride * blockIdx.y;
     const int w = S.first[s + 1] - S.first[s];
     const int m = S.rows[s];
-    const int cs = m - w;
     const int kb = min(kStep, w - k0);
-    const cx<R>* P = L + S.loff[s] + static_cast<long long>(k0) * m;
+    const int jend = min(w, (k0 / kTcPanel) * kTcPanel + kTcPanel);
+    cx<R>* Ls = Lb + lstride * blockIdx.y + S.loff[s];
+    const cx<R>* P = Ls + static_cast<long long>(k0) * m;
+    const int r = threadIdx.x % kTile, t0 = threadIdx.x / kTile;
+    const bool in_a = i0 + r < m, in_b = j0 + r < m;
     pdl_wait();
-    for (int e = threadIdx.x; e < kStep * kTile; e += blockDim.x) {
-        const int r = e % kTile, t = e / kTile;
-        cx<R> a{0, 0}, b{0, 0};
-        if (t < kb) {
-            const cx<R> d = P[k0 + t + static_cast<long long>(t) * m];
-            if (i0 + r < m) a = P[i0 + r + static_cast<long long>(t) * m] * d;
-            if (j0 + r < m) b = P[j0 + r + static_cast<long long>(t) * m];
-        }
-        As[t * kTile + r] = a;
-        Bs[t * kTile + r] = b;
+    cx<R> av[kLoads], bv[kLoads];
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+        const int t = t0 + kSkip * u;
+        const cx<R>* col = P + static_cast<long long>(t) * m + r;
+        av[u] = t < kb && in_a ? col[i0] : cx<R>{0, 0};
+        bv[u] = t < kb && in_b ? col[j0] : cx<R>{0, 0};
     }
+    if (threadIdx.x < kb) D[threadIdx.x] = P[k0 + threadIdx.x + static_cast<long long>(threadIdx.x) * m];
     __syncthreads();
+#pragma unroll
+    for (int u = 0; u < kLoads; ++u) {
+        const int t = t0 + kSkip * u;
+        As[t * kTile + r] = t < kb ? av[u] * D[t] : cx<R>{0, 0};
+        Bs[t * kTile + r] = bv[u];
+    }
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    cx<R>* const dst = Ls + i0 + tx + static_cast<long long>(j0 + ty) * m;
+    auto mine = [&](int a, int b) {
+        const int i = i0 + tx + 16 * a, j = j0 + ty + 16 * b;
+        return j < jend && i < m && i >= j;
+    };
+    cx<R> old[4][4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b)
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+            old[a][b] = mine(a, b) ? dst[16 * a + static_cast<long long>(16 * b) * m] : cx<R>{0, 0};
+    __syncthreads();
     cx<R> acc[4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
         for (int b = 0; b < 4; ++b) acc[a][b] = cx<R>{0, 0};
+#pragma unroll 2
     for (int t = 0; t < kb; ++t) {
-        cx<R> av[4], bv[4];
+        cx<R> x[4], y[4];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) av[a] = As[t * kTile + tx + 16 * a];
+        for (int a = 0; a < 4; ++a) x[a] = As[t * kTile + tx + 16 * a];
 #pragma unroll
-        for (int b = 0; b < 4; ++b) bv[b] = Bs[t * kTile + ty + 16 * b];
+        for (int b = 0; b < 4; ++b) y[b] = Bs[t * kTile + ty + 16 * b];
 #pragma unroll
         for (int a = 0; a < 4; ++a)
 #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                acc[a][b].re += av[a].re * bv[b].re - av[a].im * bv[b].im;
-                acc[a][b].im += av[a].re * bv[b].im + av[a].im * bv[b].re;
+                acc[a][b].re += x[a].re * y[b].re - x[a].im * y[b].im;
+                acc[a][b].im += x[a].re * y[b].im + x[a].im * y[b].re;
             }
-    }
-    cx<R>* Ls = L + S.loff[s];
-    cx<R>* CBs = CB + (cs > 0 ? S.cboff[s] : 0);
-    const int jend = min(w, (k0 / kTcPanel) * kTcPanel + kTcPanel);
-    // Read-modify-write: all 16 loads first, so their latencies overlap.
-    cx<R>* dst[4][4];
-    cx<R> old[4][4];
-#pragma unroll
-    for (int b = 0; b < 4; ++b) {
-        const int j = j0 + ty + 16 * b;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int i = i0 + tx + 16 * a;
-            dst[a][b] = nullptr;
-            if (j < jend && i < m && i >= j)
-                dst[a][b] = (j < w) ? Ls + i + static_cast<long long>(j) * m
-                                    : CBs + (i - w) + static_cast<long long>(j - w) * cs;
-            if (dst[a][b]) old[a][b] = *dst[a][b];
-        }
     }
 #pragma unroll
     for (int b = 0; b < 4; ++b)
 #pragma unroll
         for (int a = 0; a < 4; ++a)
-            if (dst[a][b]) *dst[a][b] = old[a][b] - acc[a][b];
+            if (mine(a, b)) dst[16 * a + static_cast<long long>(16 * b) * m] = old[a][b] - acc[a][b];
 }
 
 // SIMT trailing update of a complete panel (either precision). Item
