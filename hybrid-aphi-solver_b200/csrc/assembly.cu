@@ -35,6 +35,8 @@
 #include <complex>
 #include <cstring>
 #include <limits>
+#include <mutex>
+#include <set>
 #include <vector>
 
 #include "assembly.hpp"
@@ -932,6 +934,25 @@ std::unique_ptr<Assembly> assembly_create(const aphi_assembly_desc& d, bool devi
     return A;
 }
 
+// The fill's opt-in shared-memory limits, for the most frequencies of a launch.
+// A limit belongs to the kernel and the device, not to the call: set once per
+// device, and to one value, because assemblies are refilled from several host
+// threads at once (a limit that followed each call's need could be lowered by
+// another thread before the launch, which was then refused).
+static void set_fill_smem_limits() {
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    APHI_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.count(dev)) return;
+    APHI_CUDA(cudaFuncSetAttribute(k_tet_terms<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   TetBlock<kTetWarps>::bytes(kMaxBatchOmegas)));
+    APHI_CUDA(cudaFuncSetAttribute(k_tet_terms<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   TetBlock<4 * kTetWarps>::bytes(kMaxBatchOmegas)));
+    done.insert(dev);
+}
+
 void assembly_refill(Assembly& A, int nfreq, const double* omegas, int cond, double* values_dev,
                      double* rhs_dev, cudaStream_t stream) {
     if (nfreq < 1) throw Error(APHI_ERR_BAD_SHAPE, "refill: no frequency given");
@@ -945,6 +966,7 @@ void assembly_refill(Assembly& A, int nfreq, const double* omegas, int cond, dou
                         "it cannot be stored. Its (Phi,A) block is j*omega times its (A,Phi) block. "
                         "Use row_scaled or scaled_phi for symmetric storage.");
     }
+    set_fill_smem_limits();
     const int chunk = std::min(nfreq, kMaxBatchOmegas);
     if (A.terms_capacity < chunk) {
         if (A.d_terms) APHI_CUDA(cudaFree(A.d_terms));
@@ -965,7 +987,6 @@ void assembly_refill(Assembly& A, int nfreq, const double* omegas, int cond, dou
         // Few tets: one a warp, so that every multiprocessor has some; many:
         // four a warp, whose geometry then shares a warp's instructions.
         auto tet_terms = [&](auto kern, int rounds, int smem) {
-            APHI_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             kern<<<ceil_div(A.T, kTetWarps * rounds) + 1, 32 * kTetWarps, smem, stream>>>(ta, pa, om, cond, q, terms);
             APHI_CHECK_LAUNCH();
         };
