@@ -366,13 +366,31 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     const bool prof = f->profile;
     const bool presplit = sizeof(R) == 4 && f->tc_split == 2 && f->presplit && f->tcws;
     const bool i8 = presplit && f->tc_i8;  // FP32 trailing updates on INT8 digits
+    // Around every launch: counted, and timed under its kind when profiled.
+    auto begin = [&](int kind) {
+        if (!prof || !((f->prof_mask >> kind) & 1u)) return false;
+        cudaEvent_t e[2];
+        APHI_CUDA(cudaEventCreate(&e[0]));
+        APHI_CUDA(cudaEventCreate(&e[1]));
+        fm->prof_events.push_back(e[0]);
+        fm->prof_events.push_back(e[1]);
+        fm->prof_kinds.push_back(kind);
+        APHI_CUDA(cudaEventRecord(e[0], st));
+        return true;
+    };
+    auto end = [&](bool timed) {
+        APHI_CHECK_LAUNCH();
+        if (timed) APHI_CUDA(cudaEventRecord(fm->prof_events.back(), st));
+    };
     // The digits of a trailing update (split), and the update, which goes through
     // the batch in as many passes as the digits' workspace asks for.
     using Digits = std::conditional_t<sizeof(R) == 8, I8Fp64, I8Fp32>;
     unsigned char* const digits = sizeof(R) == 8 ? f->dws : f->tcws;
     auto split_i8 = [&](const Launch& l, int b0, int nb) {
+        const bool timed = begin(l.kind);
         chained(k_i8_split<R, Digits>, dim3(l.count, nb, kTcM / 32), 256, 0, st, S, l.first, L + ls * b0, ls, digits,
                 l.units * 256LL, l.kcap);
+        end(timed);
     };
     const Launch* operands = nullptr;  // of the next update
     int pass = f->batch;               // entries whose digits fit the workspace at once
@@ -386,9 +404,11 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
             const int nb = std::min(pass, f->batch - b0);
             if (pass < f->batch) split_i8(*operands, b0, nb);
             const long long tiles = static_cast<long long>(l.count) * (kTcN / Digits::Nc) * nb;
+            const bool timed = begin(l.kind);
             chained(k_update_i8<R, Digits>, dim3(static_cast<unsigned>(std::min<long long>(tiles, f->sms))), kI8Threads,
                     Digits::smem, st, S, l.first, l.count, nb, L + ls * b0, CB + cs * b0, ls, cs, l.kcap, digits,
                     operands->units * 256LL, f->err);
+            end(timed);
         }
     };
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
@@ -400,17 +420,17 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
         // no operand launch.
         if (l.kind == K_TC_SPLIT && !presplit) continue;
         if (l.kind == K_DMMA_SCALE && !prescaled) continue;
-        dim3 grid(l.count, sa && sa->ny > 0 ? sa->ny : f->batch);
-        const bool timed = prof && ((f->prof_mask >> l.kind) & 1u);
-        if (timed) {
-            cudaEvent_t e[2];
-            APHI_CUDA(cudaEventCreate(&e[0]));
-            APHI_CUDA(cudaEventCreate(&e[1]));
-            fm->prof_events.push_back(e[0]);
-            fm->prof_events.push_back(e[1]);
-            fm->prof_kinds.push_back(l.kind);
-            APHI_CUDA(cudaEventRecord(e[0], st));
+        // Digits: no launch of its own where the update's passes split for themselves.
+        if (l.kind == K_DMMA_SCALE || (l.kind == K_TC_SPLIT && i8)) {
+            plan_i8(l);
+            continue;
         }
+        if ((l.kind == K_UPDATE_WIDE && prescaled) || (l.kind == K_UPDATE_TC && i8)) {
+            update_i8(l);
+            continue;
+        }
+        dim3 grid(l.count, sa && sa->ny > 0 ? sa->ny : f->batch);
+        const bool timed = begin(l.kind);
         switch (l.kind) {
             case K_EXTEND_ADD: {
                 // Few items (they do not fill the chip): four blocks each, so that a
@@ -428,39 +448,22 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                     chained(k_update_panel<R>, grid, 256, 2 * kStep * kTile * sizeof(cx<R>), st, S, l.first, L, ls);
                     break;
                 }
-                if constexpr (sizeof(R) == 8) {
-                    if (l.kind == K_UPDATE_WIDE && prescaled)
-                        update_i8(l);
-                    else
-                        chained(k_update_wide_dmma, grid, 256, kDmmaSmem, st, S, l.first, L, CB, ls, cs, l.kcap,
-                                l.kind == K_UPDATE_PANEL ? 1 : 0);
-                } else
+                if constexpr (sizeof(R) == 8)
+                    chained(k_update_wide_dmma, grid, 256, kDmmaSmem, st, S, l.first, L, CB, ls, cs, l.kcap,
+                            l.kind == K_UPDATE_PANEL ? 1 : 0);
+                else
                     k_update_wide<R><<<grid, 256, wide_smem<R>(), st>>>(S, l.first, L, CB, ls, cs, l.kcap,
                                                                       l.kind == K_UPDATE_PANEL ? 1 : 0);
                 break;
-            case K_DMMA_SCALE:
-                if constexpr (sizeof(R) == 8)
-                    plan_i8(l);
-                else
-                    throw Error(APHI_ERR_INVALID, "operand scaling planned for an FP32 factor");
-                break;
             case K_TC_SPLIT:
-                if constexpr (sizeof(R) == 4) {
-                    if (i8) {
-                        plan_i8(l);
-                        break;
-                    }
+                if constexpr (sizeof(R) == 4)
                     k_tc_split<<<dim3(grid.x, grid.y, (l.kcap + 8 * kTcK - 1) / (8 * kTcK)), kTcThreads, 0, st>>>(
                         S, l.first, L, ls, f->tcws, f->tcws_stride, l.kcap);
-                } else
+                else
                     throw Error(APHI_ERR_INVALID, "operand split planned for an FP64 factor");
                 break;
             case K_UPDATE_TC:
                 if constexpr (sizeof(R) == 4) {
-                    if (i8) {
-                        update_i8(l);
-                        break;
-                    }
                     if (presplit) {
                         auto go = [&](auto kern, int smem) {
                             kern<<<grid, kTcThreads, smem, st>>>(S, l.first, L, CB, ls, cs, l.kcap, f->tcws,
@@ -510,8 +513,7 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
                 chained(k_bwd_diag<R>, grid, kBwdDiagThreads, bwd_smem, st, S, l.first, *sa, L, ls, y, part);
                 break;
         }
-        APHI_CHECK_LAUNCH();
-        if (timed) APHI_CUDA(cudaEventRecord(fm->prof_events.back(), st));
+        end(timed);
     }
 }
 
