@@ -169,6 +169,7 @@ _SIGS = {
     "aphi_csc_solve_host": (I, [I, PI, PI, PD, PD, I, PD]),
     "aphi_csr_residuals_host": (I, [I, PI, PI, PD, I, PD, PD, PD]),
     "aphi_factor_set_tc_split": (I, [P, I]),
+    "aphi_factor_set_fp64_digits": (I, [P, I]),
     "aphi_spmv": (I, [P, I, I, P, P, P, P]),
     "aphi_factor_profile_kinds": (I, [P, C.c_uint]),
     "aphi_selftest_tc_tile_split": (I, [I, I, I, I, I, P, P, P]),
@@ -758,6 +759,13 @@ class Factor:
         check(lib().aphi_factor_set_tc_split(self._h, split))
         self.tc_split = split
 
+    def set_fp64_digits(self, on: bool) -> None:
+        """FP64 factors: trailing updates on byte digits (the default: accurate
+        relative to each row's largest component) or, with False, in FP64
+        arithmetic (each number's own precision, for rows graded within
+        themselves; slower)."""
+        check(lib().aphi_factor_set_fp64_digits(self._h, int(on)))
+
     def set_batch(self, batch: int) -> None:
         """Process `batch` (1..capacity) entries from now on, without reallocating."""
         check(lib().aphi_factor_set_batch(self._h, batch))
@@ -927,12 +935,15 @@ class SweepSolver:
     by COCG preconditioned with its own FP64 factor, to the same rtol / tol:
     for systems whose plain FP64 direct solve stops short of the residual
     target (the torus with its cut port: ~4e-10 at 50 Hz).
+
+    fp64_digits: the form of the FP64 factors' trailing updates
+    (Factor.set_fp64_digits).
     """
 
     def __init__(self, analysis: Analysis, assembly: Assembly, batch: int, precision: str = "mixed",
                  fp64_batch: int = 8, rtol: float = 1e-14, tol: float = 1e-16, max_iters: int = 40,
                  fp32_batch: int | None = None, predict: bool = True, fp64_refine: bool = False,
-                 tc_split: int = 2, overlap: bool = True):
+                 tc_split: int = 2, overlap: bool = True, fp64_digits: bool = True):
         if precision not in ("mixed", "fp64"):
             raise InvalidArgument(ERR_BAD_SHAPE, f"SweepSolver: precision {precision!r} is not 'mixed' or 'fp64'")
         self.analysis, self.assembly = analysis, assembly
@@ -944,6 +955,7 @@ class SweepSolver:
         self.fp64_refine = fp64_refine
         self.tc_split = tc_split
         self.overlap = overlap
+        self.fp64_digits = fp64_digits
         self._side_stream = None
         self.stall_omega = None      # lowest frequency whose FP32 refinement stalled
         self._factors = {}
@@ -964,6 +976,8 @@ class SweepSolver:
             f = Factor(self.analysis, precision, size)
             if precision == PREC_FP32:
                 f.set_tc_split(self.tc_split)
+            elif not self.fp64_digits:
+                f.set_fp64_digits(False)
             if self._profile:
                 f.profile(True, self._profile_kinds)
             self._factors[precision] = f

@@ -79,6 +79,18 @@ int aphi_factor_set_tc_split(aphi_factor* f, int split) {
     });
 }
 
+int aphi_factor_set_fp64_digits(aphi_factor* f, int on) {
+    return guard([&] {
+        if (!f) throw Error(APHI_ERR_INVALID, "aphi_factor_set_fp64_digits: null factor");
+        if (f->precision != 64)
+            throw Error(APHI_ERR_BAD_SHAPE, "aphi_factor_set_fp64_digits: an FP32 factor (see aphi_factor_set_tc_split)");
+        if (on && f->an->dmma_ws_units > 0 && !f->dws)
+            throw Error(APHI_ERR_BAD_SHAPE, "aphi_factor_set_fp64_digits: the factor was made without room for digits "
+                                            "(APHI_DMMA_PRESCALE=0)");
+        f->fp64_digits = on != 0;
+    });
+}
+
 int aphi_factor_profile(aphi_factor* f, int enable) {
     return guard([&] {
         if (!f) throw Error(APHI_ERR_INVALID, "aphi_factor_profile: null factor");

@@ -414,7 +414,7 @@ void run_plan(const aphi_factor* f, const std::vector<Launch>& plan, cudaStream_
     const size_t tri_smem = kTriSmem * sizeof(cx<R>);               // forward triangles
     const size_t bwd_smem = (kTriSmem + (sa ? red_smem(sa->nr) : 0)) * sizeof(cx<R>);  // backward triangles
     // FP64 trailing updates on INT8 digits, prepared once per panel group.
-    const bool prescaled = sizeof(R) == 8 && f->dws;
+    const bool prescaled = sizeof(R) == 8 && f->dws && f->fp64_digits;
     for (const Launch& l : plan) {
         // Without prepared operands the tile splits (FP64: scales) them itself:
         // no operand launch.

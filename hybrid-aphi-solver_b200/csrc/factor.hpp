@@ -47,6 +47,7 @@ struct aphi_factor {
     long long dws_stride = 0;      // entry (APHI_DMMA_PRESCALE=0: none, the tiles run on DMMA from the panels)
     long long digit_bytes = 0;     // of dws, or of tcws with INT8 digits (digit_workspace)
     int sms = 0;                   // multiprocessors of the device (persistent tiles' grid)
+    bool fp64_digits = true;       // FP64: the trailing updates take the digits (aphi_factor_set_fp64_digits)
     unsigned char* tcws = nullptr;  // FP32: the digits, or the pre-split operand planes (tcws_stride bytes per entry)
     long long tcws_stride = 0;
     int* err = nullptr;         // device error word (bounded waits)

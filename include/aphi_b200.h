@@ -284,11 +284,34 @@ int aphi_factor_set_batch(aphi_factor* f, int batch);
 /* FP32 factors: the form of the tensor-core trailing update. 3 (the default):
  * each operand as three TF32 pieces, six cross products kept, every product
  * more accurate than an FP32 multiply. 2: the faster form, each operand as
- * four 8-bit digits relative to its row's largest component (2^-30 of it),
- * summed exactly; with the environment variable APHI_TC_PRESPLIT set when the
- * factor is made, two TF32 pieces instead (products hh + hl + lh, each to
- * about 2^-21 relative). APHI_TC_SPLIT=2 sets the default. */
+ * four 8-bit digits relative to its row's largest component: with A and B the
+ * powers of two next above the largest components of the two rows that an entry
+ * sums over (L D and L, the pivots' magnitudes shared out evenly between them),
+ * a sum of K complex products is off by at most K 2^-29 A B from the operands'
+ * rounding and K 2^-27.4 A B from the digit products that are left out, beside
+ * the roundings of an FP32 result; the products that are kept are summed
+ * exactly. A number below 2^-6 of its row's largest keeps fewer than its 24
+ * bits, one below 2^-31 none; rows that are not graded are more accurate than
+ * with two TF32 pieces. With the environment variable APHI_TC_PRESPLIT set when
+ * the factor is made, two TF32 pieces instead (products hh + hl + lh, each to
+ * about 2^-21 of itself). APHI_TC_SPLIT=2 sets the default. */
 int aphi_factor_set_tc_split(aphi_factor* f, int split);
+/* FP64 factors: whether the trailing updates run on byte digits (on = 1, the
+ * default) or in FP64 arithmetic (on = 0, half as fast: two factorizations of
+ * the 32^3 cylinder take 283 ms on digits and 572 ms so). Digits: each operand as eight 8-bit digits
+ * relative to its row's largest component. With A and B as above a sum of K
+ * complex products is off by at most K 2^-61 A B from the operands' rounding
+ * and K 2^-58 A B from the digit products that are left out, beside the
+ * roundings of an FP64 result; the products that are kept are summed exactly.
+ * FP64 arithmetic is off by up to K 2^-52 of the sum of the products'
+ * magnitudes instead. That sum is at least A B / 10 on the diagonal, and A B / 4
+ * where the two rows' largest components stand in one column, so there the
+ * digits are the more accurate form; an entry whose rows are graded against one another
+ * (products all far below A B) keeps its accuracy relative to A B, that is to
+ * the diagonal entries of its row and column, but not relative to itself. The
+ * change may be made between factorizations; it is refused for FP32 factors and
+ * (on = 1) where APHI_DMMA_PRESCALE=0 was set as the factor was made. */
+int aphi_factor_set_fp64_digits(aphi_factor* f, int on);
 
 typedef struct {
     int ok;                    /* FactorStats::ok */
