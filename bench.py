@@ -277,7 +277,7 @@ def device_ms(fn, stream, reps=3):
 
 
 def assembly_roofline(w, asm, an, nfreq, ms, hbm):
-    """k_tet_terms + k_slot_sum + k_port_terms over a whole sweep. Algorithmic
+    """k_tet_terms + k_slot_sum over a whole sweep. Algorithmic
     bytes per frequency: T (16 B tet -> node ids + 96 B coordinates + 24 B edge
     ids + 6 B signs + 64 B DOF indices + 4 B body id) + 4 B per live pair of
     each tet's DOFs (its slot map, sum n_t (n_t + 1) / 2) + 16 B per stored
@@ -290,7 +290,7 @@ def assembly_roofline(w, asm, an, nfreq, ms, hbm):
     # what this design moves: the term array written once and read once per
     # frequency, its slot lists read once per batch, values and rhs written
     design = nfreq * (32 * asm.num_terms + 16 * (an.nnz + an.n)) + 4 * asm.num_terms + 4 * (an.nnz + an.n)
-    return {"kernels": "k_tet_terms + k_port_terms + k_slot_sum", "bound": "hbm", "frequencies": nfreq,
+    return {"kernels": "k_tet_terms + k_slot_sum", "bound": "hbm", "frequencies": nfreq,
             "ms_per_sweep": ms, "ms_per_frequency": ms / nfreq, "algorithmic_bytes_per_frequency": per_freq,
             "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
             "design_bytes_per_sweep": design, "design_gbs": design / (ms / 1000.0) / 1e9}
@@ -529,22 +529,10 @@ def run_ours(args):
     del fp64
 
     hbm, bf16, bf16s, src = peaks()
-    # DRAM traffic of the dominant kernel per launch of the timed steps: the
-    # per-entry traffic of a one-pass ncu capture of the same kernel on this
-    # mesh (profiles/traffic.json), times the frequencies each of the timed
-    # launches carried (a launch's traffic grows with its entries: each
-    # entry's panels and blocks are separate memory).
-    traffic_path = ROOT / "profiles" / "traffic.json"
-    traffic, traffic_note = None, None
-    if traffic_path.exists():
-        t = json.loads(traffic_path.read_text()).get(f"{top['precision']}_{top['kind']}_{args.cells}")
-        st = plan_flops[top["precision"]].get(top["kind"])
-        if t and st and top["launches"]:
-            calls = top["launches"] / st[0]
-            per_call = entries[top["precision"]] / calls
-            traffic = t["bytes_per_launch"] / t["batch"] * per_call
-            traffic_note = (f"{t['bytes_per_launch'] / t['batch'] / 1e9:.3f} GB per entry per launch from a capture "
-                            f"at batch {t['batch']} (default schedule), x {per_call:.2f} entries per launch here")
+    # DRAM traffic of the dominant kernel: only three launches at 24^3 have been
+    # captured (a capture of the whole factorization at this size is too large).
+    traffic = None
+    traffic_note = "not captured at this size; three launches at 24^3 in profiles/k_update_i8_cylinder24.md"
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
         try:

@@ -179,7 +179,7 @@ class Server:
         self.factors = {(c, p): ab.Factor(m.analysis, p, self.max_batch[c]) for c, m in meshes.items() for p in precs}
         for (c, p), f in self.factors.items():
             if p == ab.PREC_FP32:
-                f.set_tc_split(2)     # hh + hl + lh: the refinement needs no more iterations than with 3
+                f.set_tc_split(2)     # INT8 digits: the refinement needs no more iterations than with 3
         self.queues = {c: collections.deque() for c in meshes}
         self.busy = set()
         self.cv = threading.Condition()

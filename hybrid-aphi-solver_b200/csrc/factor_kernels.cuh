@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(256) k_update_wide(Sched S, long long item0, c
 
 // FP64 update on the FP64 tensor path (DMMA, mma.sync m8n8k4): the in-panel
 // updates (K = 64, too short for the INT8 tiles below), and the trailing ones
-// too with APHI_DMMA_PRESCALE=0. Same items, tile and K (up to kcap =
+// too where the factor asks for FP64 arithmetic. Same items, tile and K (up to kcap =
 // kWidePair: a group of 128-column panels) as k_update_wide. 8 warps in a 4 x 2
 // grid, each a 32 x 32 complex block of the tile: 4 x 4 blocks of 8 x 8, each
 // four real products (Cr += Ar Br - Ai Bi, Ci += Ar Bi + Ai Br; the minus by
@@ -758,8 +758,8 @@ __device__ __forceinline__ void red_sub(double* p, double v) {
 // a contiguous run of a column; a warp takes 16 columns at a time, which is
 // one 16-byte row of a core matrix per digit. Two passes over the operands,
 // the second served by the caches: the rows' largest components, then the
-// digits. Bound by its writes (48 bytes per entry; 24^3, 8 entries: 15.2 ms
-// per factorization beside 117 ms of tiles) and, on small fronts, by the
+// digits. Bound by its writes (48 bytes per entry; 24^3, 8 entries: 15.6 ms
+// per factorization beside 115 ms of tiles) and, on small fronts, by the
 // passes' dependent round trips (11 us a launch).
 template <class R, class C>
 __global__ void __launch_bounds__(256, 2) k_i8_split(Sched S, long long item0, const cx<R>* Lb, long long lstride,
@@ -894,14 +894,15 @@ __global__ void __launch_bounds__(256, 2) k_i8_split(Sched S, long long item0, c
 // Every wait is bounded and gives up early once another role has failed.
 //
 // Measured, trailing updates of a factorization (the form that each replaced):
-//   FP64, 32^3, two entries    177 ms (486, DMMA)     76 useful FP64 TFLOP/s
-//   FP64, 24^3, eight entries  112 ms (292)
-//   FP64, 8^3, one entry       10.4 us a launch (26)
-//   FP32, 32^3, six entries    166 ms (311, two TF32 pieces)
-//   FP32, 24^3, six entries     31 ms (56)
-//   FP32, 12^3, six entries    1.0 ms (1.5)
+//   FP64, 32^3, two entries    178-188 ms (486, DMMA) 71-75 useful FP64 TFLOP/s
+//   FP64, 24^3, eight entries  115-118 ms (292)
+//   FP32, 32^3, six entries    170-176 ms (311, two TF32 pieces)
+//   FP32, 24^3, six entries    30.5 ms (56)
+//   FP32, 12^3, six entries    0.91 ms (1.5)
+// and on 8^3 (FP64, one entry) 17 launches in 0.26 ms.
 // It is the faster form from the smallest launches up, so every FP64 trailing
-// update takes it, and every FP32 one that asks for two pieces. In FP64 an
+// update takes it unless its factor asks for FP64 arithmetic
+// (aphi_factor_set_fp64_digits), and every FP32 one with tc_split 2. In FP64 an
 // SM's shared memory bounds a tile: per stage the MMAs read 240 KB of digits
 // and the copies write 96 KB, 2,700 cycles beside 2,304 of tensor work (K =
 // 256: 22,000 cycles, then 4,000 to read the accumulators); in FP32 the MMAs
