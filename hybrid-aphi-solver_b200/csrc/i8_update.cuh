@@ -30,7 +30,8 @@
 // systems of the cylinder (7^3 to 28^3, 50 Hz to 1 MHz, port and random
 // right-hand sides) the solutions' errors against extended-precision ones are
 // 0.96 times those of the DMMA form (geometric mean; 0.61 to 1.60), the
-// backward errors 0.99 times.
+// backward errors 0.99 times; over 1,024 systems of the torus with its cut port
+// (14^3 to 22^3, 50 Hz to 10 kHz, both formulations) 0.99 +- 0.01 and 0.99.
 // Seven digits (2^-54) are enough for the solutions' accuracy but not for the
 // smallest pivots, which are what is left of sums of much larger terms: on
 // the 32^3 cylinder at 1 MHz the smallest pivot came out 2e-8 off, and 1e-10
